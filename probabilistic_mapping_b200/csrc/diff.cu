@@ -14,9 +14,8 @@
 //           intensities by the bilinear weights and into the 6-DoF pose of every source through
 //           the spatial derivative of the bilinear sample and the projection, as the left se(3)
 //           perturbation P_s -> exp([omega]) P_s + upsilon (omega first).
-// One warp per scanline for the paths (lane l holds planes [l*PPL, (l+1)*PPL)), one thread per
-// voxel for the cost adjoint with atomics into the intensity gradient and per-warp reductions of
-// the pose gradient in double precision.
+// One warp per scanline for the paths (lane l holds planes [l*PPL, (l+1)*PPL)); tiles of positions for the
+// cost adjoint, with atomics into the intensity gradient and per-CTA reductions of the pose gradient.
 #include <cstring>
 #include <string>
 #include <vector>
@@ -211,7 +210,8 @@ __global__ void __launch_bounds__(128) path_bwd_kernel(const PathArgs a) {
     }
 }
 
-// Soft-argmin and the per-pixel loss terms; gS when grad is set (scale = 1 / |valid pixels|).
+// Soft-argmin and the per-pixel loss terms; gS when grad is set, without the 1 / |valid pixels| of the loss's
+// mean (cost_bwd_kernel applies it).
 template <int PPL>
 __global__ void __launch_bounds__(128) soft_kernel(const float* __restrict__ S, const float* __restrict__ rho_gt,
                                                    const uint8_t* __restrict__ invalid, int N, int D, float rho0,
@@ -248,9 +248,9 @@ __global__ void __launch_bounds__(128) soft_kernel(const float* __restrict__ S, 
         return;
     }
     float g = 0.0f;
-    if (in && count[0] > 0.0) {
+    if (in) {
         const float diff = rh - rho_gt[p];
-        g = (diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f)) / (float)count[0];
+        g = diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
     }
     float o[PPL];
 #pragma unroll
@@ -259,12 +259,15 @@ __global__ void __launch_bounds__(128) soft_kernel(const float* __restrict__ S, 
     store_planes<PPL>(gS + (size_t)p * D + lane * PPL, o);
 }
 
+constexpr int kMaxDiffSources = 4;
+
 struct CostBwdArgs {
     const float* ref;
-    const float* srcs;        // S x N
-    const float* gC;          // V
+    const float4* quads;      // S x N: the cost kernel's source quads
+    const float* gC;          // V, scaled below by 1 / count
+    const double* count;      // pixels in the loss
     const uint8_t* invalid;
-    float hom[kMaxSources][12];
+    float hom[kMaxDiffSources][12];
     float fx, fy, cx, cy;
     int W, H, D, S;
     float rho0, drho;
@@ -272,115 +275,242 @@ struct CostBwdArgs {
     double* gP;               // S x 6
 };
 
-struct Smp {
-    bool ok;
-    float u, v, w, nx, ny, val, dIdu, dIdv, a, b;
-    int i, j;
+// Adjoint of the corrected 3x3 cost.  The sample at position q, source s and plane d serves the nine
+// pixels p around q, each term compares it with the same reference value ref(q), so the sign of
+// ref(q) - val(q) is common to the nine and the adjoint of the sample is
+//   -sign(ref(q) - val(q)) * sum over the 3x3 pixels p around q, measured by s at d, of gC(p, d) / (9 n(p, d)),
+// n(p, d) the sources that measure p at d: ONE sample, one scatter into the image and one pose term per
+// (q, s, d) instead of nine (and instead of the 18 more samples per (p, s, d) that a voxel's own validity
+// takes).  A CTA owns 28 x R positions q and 16 planes; a warp owns a plane pair and walks the rows:
+//   * lane l stands on column x0 - 2 + l.  A first pass over the R + 4 rows turns the validity of the
+//     samples into one ballot per row and plane, from which "all nine samples valid" is a few
+//     bit operations, and n a bit count over the sources;
+//   * the tile's gC (with its ring of one pixel) sits in shared memory, read in 64-byte plane runs and
+//     already divided by 9 n; the 3x3 sums are two shuffles per row and a rolling sum of three rows;
+//   * a sample's lower two taps wait in registers for the next row, whose upper taps fall on the same
+//     texels when the warp hardly turns the image, so that a sample costs two reductions, not four;
+//   * the pose terms stay in registers over a tile's rows, then one double atomic per CTA and component.
+// The samples repeat the cost kernel's operations (homography FMAs, reciprocal, exact bilinear), so that
+// the signs are the forward's.  Bound by issue (about 100 instructions per sample and plane pair); with one
+// thread per voxel, 27 samples per source and nine scatters it was bound by its atomics: 29.5 -> 0.78 ms at
+// 640x480x128 with 3 sources, 5.14 -> 0.088 ms at 320x240x64 with 2.
+constexpr int BQX = 28;                  // positions per row of a tile
+constexpr int BWARPS = 8;                // plane pairs per CTA
+constexpr int BPL = 2 * BWARPS;          // planes per CTA
+constexpr int BSP = BPL + 2;             // pitch of a pixel's planes in shared memory
+
+// Pending lower taps of the previous row: texel idx and its right neighbour.
+struct Pending {
+    unsigned idx;
+    float l, r;
 };
 
-// One warped sample with the cost kernel's operations (homography FMAs, reciprocal, exact bilinear).
-__device__ inline Smp warp_sample(const CostBwdArgs& A, int s, int qu, int qv, float rho) {
-    const float* h = A.hom[s];
-    const float fu = (float)qu, fv = (float)qv;
-    const float x = __fmaf_rn(h[0], fu, __fmaf_rn(h[1], fv, h[2]));
-    const float y = __fmaf_rn(h[3], fu, __fmaf_rn(h[4], fv, h[5]));
-    const float z = __fmaf_rn(h[6], fu, __fmaf_rn(h[7], fv, h[8]));
-    Smp r;
-    r.w = __fmaf_rn(h[11], rho, z);
-    r.nx = __fmaf_rn(h[9], rho, x);
-    r.ny = __fmaf_rn(h[10], rho, y);
-    const float2 rc = rcp_warp2(make_float2(r.w, r.w));
-    r.u = __fmul_rn(r.nx, rc.x);
-    r.v = __fmul_rn(r.ny, rc.x);
-    r.ok = (r.w >= 0.0f) && (r.u >= 0.0f) && (r.u <= (float)(A.W - 1)) && (r.v >= 0.0f) && (r.v <= (float)(A.H - 1));
-    if (!r.ok) return r;
-    const float fu0 = floorf(r.u), fv0 = floorf(r.v);
-    r.i = (int)fu0;
-    r.j = (int)fv0;
-    r.a = __fsub_rn(r.u, fu0);
-    r.b = __fsub_rn(r.v, fv0);
-    const float* img = A.srcs + (size_t)s * A.W * A.H;
-    const bool i1 = r.i + 1 < A.W, j1 = r.j + 1 < A.H;
-    const float t00 = img[(size_t)r.j * A.W + r.i];
-    const float t10 = i1 ? img[(size_t)r.j * A.W + r.i + 1] : 0.0f;
-    const float t01 = j1 ? img[(size_t)(r.j + 1) * A.W + r.i] : 0.0f;
-    const float t11 = (i1 && j1) ? img[(size_t)(r.j + 1) * A.W + r.i + 1] : 0.0f;
-    const float top = __fmaf_rn(r.a, __fsub_rn(t10, t00), t00);
-    const float bot = __fmaf_rn(r.a, __fsub_rn(t11, t01), t01);
-    r.val = __fmaf_rn(r.b, __fsub_rn(bot, top), top);
-    r.dIdu = (1.0f - r.b) * (t10 - t00) + r.b * (t11 - t01);
-    r.dIdv = (1.0f - r.a) * (t01 - t00) + r.a * (t11 - t10);
-    return r;
+__device__ __forceinline__ void red_add(float* p, float v) {
+    if (v != 0.0f) atomicAdd(p, v);
 }
 
-__device__ inline float ref_px(const CostBwdArgs& A, int x, int y) {
-    return (x < 0 || y < 0 || x >= A.W || y >= A.H) ? 0.0f : A.ref[(size_t)y * A.W + x];
-}
+template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(const CostBwdArgs A) {
+    constexpr int PX = BQX + 2, PY = R + 2;   // pixels p of the tile
+    __shared__ __align__(16) float hs[PX * PY * BSP];
+    __shared__ float refs[R * 32];
+    __shared__ unsigned ok1[BWARPS][R + 4][2];                      // validity of the samples, one source
+    __shared__ unsigned ok9[BWARPS][kMaxDiffSources][PY][2];        // all nine samples of a pixel valid
+    __shared__ float ps[BWARPS][6 * kMaxDiffSources];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int W = A.W, H = A.H, D = A.D;
+    const int x0 = blockIdx.x * BQX - 1, y0 = blockIdx.y * R - 1, d0 = blockIdx.z * BPL;   // first position q
+    const int x = x0 - 2 + lane;
 
-__constant__ int kPatch[9][2] = {{0, 0}, {0, -1}, {0, 1}, {-1, 0}, {1, 0}, {-1, -1}, {1, 1}, {-1, 1}, {1, -1}};
-constexpr int kMaxDiffSources = 4;
+    for (int e = tid; e < PX * PY * (BPL / 4); e += 32 * BWARPS) {
+        const int p = e >> 2, k = (e & 3) * 4;
+        const int py = p / PX, px = p - py * PX;
+        const int gx = x0 - 1 + px, gy = y0 - 1 + py;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (gx >= 0 && gy >= 0 && gx < W && gy < H) {
+            const size_t pix = (size_t)gy * W + gx;
+            if (!A.invalid[pix] && PM_RANGE_IN_BOUNDS(pix * D + d0 + k, 4, (long long)W * H * D, kSiteDiffGrad))
+                v = *reinterpret_cast<const float4*>(A.gC + pix * D + d0 + k);
+        }
+        *reinterpret_cast<float2*>(hs + p * BSP + k) = make_float2(v.x, v.y);
+        *reinterpret_cast<float2*>(hs + p * BSP + k + 2) = make_float2(v.z, v.w);
+    }
+    for (int e = tid; e < R * 32; e += 32 * BWARPS) {
+        const int gx = x0 - 2 + (e & 31), gy = y0 + (e >> 5);
+        refs[e] = gx >= 0 && gy >= 0 && gx < W && gy < H ? A.ref[(size_t)gy * W + gx] : 0.0f;
+    }
 
-__global__ void __launch_bounds__(128) cost_bwd_kernel(const CostBwdArgs A) {
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long V = (long)A.W * A.H * A.D;
-    float gp[kMaxDiffSources][6];
+    const int da = d0 + 2 * warp;
+    const float2 rho = make_float2(__fmaf_rn((float)da, A.drho, A.rho0), __fmaf_rn((float)(da + 1), A.drho, A.rho0));
+    const float fxl = (float)x;
+    const unsigned Wb = __float_as_uint((float)(W - 1)), Hb = __float_as_uint((float)(H - 1));
+    // warp of (x, y) at the plane pair: denominator, its reciprocal and the coordinates
+    auto warp_pos = [&](const float* h, int y, float2& w, float2& r, float2& u, float2& v) {
+        const float fy = (float)y;
+        const float hx = __fmaf_rn(h[0], fxl, __fmaf_rn(h[1], fy, h[2]));
+        const float hy = __fmaf_rn(h[3], fxl, __fmaf_rn(h[4], fy, h[5]));
+        const float hz = __fmaf_rn(h[6], fxl, __fmaf_rn(h[7], fy, h[8]));
+        w = __ffma2_rn(make_float2(h[11], h[11]), rho, make_float2(hz, hz));
+        r = rcp_warp2(w);
+        u = __fmul2_rn(__ffma2_rn(make_float2(h[9], h[9]), rho, make_float2(hx, hx)), r);
+        v = __fmul2_rn(__ffma2_rn(make_float2(h[10], h[10]), rho, make_float2(hy, hy)), r);
+    };
+
+    for (int s = 0; s < A.S; ++s) {
+        for (int r = 0; r < R + 4; ++r) {
+            float2 w, rc, u, v;
+            warp_pos(A.hom[s], y0 - 2 + r, w, rc, u, v);
+            // + 0 turns -0 into +0; negative values and NaN have bit patterns above the bound's
+            const float2 z = make_float2(0.0f, 0.0f);
+            u = __fadd2_rn(u, z);
+            v = __fadd2_rn(v, z);
+            const unsigned b0 = __ballot_sync(kFull, w.x >= 0.0f && __float_as_uint(u.x) <= Wb && __float_as_uint(v.x) <= Hb);
+            const unsigned b1 = __ballot_sync(kFull, w.y >= 0.0f && __float_as_uint(u.y) <= Wb && __float_as_uint(v.y) <= Hb);
+            if (lane == 0) {
+                ok1[warp][r][0] = b0;
+                ok1[warp][r][1] = b1;
+            }
+        }
+        __syncwarp();
+        if (lane < PY)
+            for (int j = 0; j < 2; ++j) {
+                const unsigned m = ok1[warp][lane][j] & ok1[warp][lane + 1][j] & ok1[warp][lane + 2][j];
+                ok9[warp][s][lane][j] = m & (m << 1) & (m >> 1);
+            }
+        __syncwarp();
+    }
+    __syncthreads();   // the tile's gC is staged
+
+    // gC / (9 n) and the 1 / count of the loss's mean, in place (a warp's own planes)
+    const float scale = A.count[0] > 0.0 ? 1.0f / (float)A.count[0] : 0.0f;
+    float inv[kMaxDiffSources + 1];
+    inv[0] = 0.0f;
 #pragma unroll
-    for (int s = 0; s < kMaxDiffSources; ++s)
-#pragma unroll
-        for (int i = 0; i < 6; ++i) gp[s][i] = 0.0f;
-    if (e < V) {
-        const long pix = e / A.D;
-        const int d = (int)(e - pix * A.D);
-        const int v = (int)(pix / A.W), u = (int)(pix - (long)v * A.W);
-        const float g = A.gC[e];
-        if (!A.invalid[pix] && g != 0.0f) {
-            const float rho = __fmaf_rn((float)d, A.drho, A.rho0);
-            int n = 0;
+    for (int n = 1; n <= kMaxDiffSources; ++n) inv[n] = scale / (9.0f * (float)n);
+    const bool in_p = lane >= 1 && lane <= PX;
+    float2* const hp = reinterpret_cast<float2*>(hs + (in_p ? lane - 1 : 0) * BSP + 2 * warp);
+    constexpr int HROW = PX * BSP / 2;   // float2 per row of pixels
+    if (in_p)
+        for (int r = 0; r < PY; ++r) {
+            int n0 = 0, n1 = 0;
             for (int s = 0; s < A.S; ++s) {
-                bool ok = true;
-                for (int k = 0; k < 9 && ok; ++k) ok = warp_sample(A, s, u + kPatch[k][0], v + kPatch[k][1], rho).ok;
-                n += ok;
+                n0 += (ok9[warp][s][r][0] >> lane) & 1u;
+                n1 += (ok9[warp][s][r][1] >> lane) & 1u;
             }
-            if (n > 0) {
-                for (int s = 0; s < A.S; ++s) {
-                    bool ok = true;
-                    for (int k = 0; k < 9 && ok; ++k) ok = warp_sample(A, s, u + kPatch[k][0], v + kPatch[k][1], rho).ok;
-                    if (!ok) continue;
-                    float* gi = A.gI + (size_t)s * A.W * A.H;
-                    for (int k = 0; k < 9; ++k) {
-                        const int qu = u + kPatch[k][0], qv = v + kPatch[k][1];
-                        const Smp q = warp_sample(A, s, qu, qv, rho);
-                        const float diff = ref_px(A, qu, qv) - q.val;
-                        const float sg = diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
-                        const float c = -sg * g / (9.0f * (float)n);
-                        if (c == 0.0f) continue;
-                        atomicAdd(gi + (size_t)q.j * A.W + q.i, c * (1.0f - q.a) * (1.0f - q.b));
-                        if (q.i + 1 < A.W) atomicAdd(gi + (size_t)q.j * A.W + q.i + 1, c * q.a * (1.0f - q.b));
-                        if (q.j + 1 < A.H) atomicAdd(gi + (size_t)(q.j + 1) * A.W + q.i, c * (1.0f - q.a) * q.b);
-                        if (q.i + 1 < A.W && q.j + 1 < A.H)
-                            atomicAdd(gi + (size_t)(q.j + 1) * A.W + q.i + 1, c * q.a * q.b);
-                        // pose: P = K^-1 (nx, ny, w); dP = omega x P + rho upsilon
-                        const float Px = (q.nx - A.cx * q.w) / A.fx, Py = (q.ny - A.cy * q.w) / A.fy, Pz = q.w;
-                        const float dP[6][3] = {{0.0f, -Pz, Py}, {Pz, 0.0f, -Px}, {-Py, Px, 0.0f},
-                                                {rho, 0.0f, 0.0f}, {0.0f, rho, 0.0f}, {0.0f, 0.0f, rho}};
+            float i0 = 0.0f, i1 = 0.0f;
 #pragma unroll
-                        for (int i = 0; i < 6; ++i) {
-                            const float du = (A.fx * dP[i][0] + (A.cx - q.u) * dP[i][2]) / q.w;
-                            const float dv = (A.fy * dP[i][1] + (A.cy - q.v) * dP[i][2]) / q.w;
-                            gp[s][i] += c * (q.dIdu * du + q.dIdv * dv);
-                        }
-                    }
-                }
+            for (int n = 1; n <= kMaxDiffSources; ++n) {
+                i0 = n0 == n ? inv[n] : i0;
+                i1 = n1 == n ? inv[n] : i1;
             }
+            const float2 g = hp[r * HROW];
+            hp[r * HROW] = make_float2(__fmul_rn(g.x, i0), __fmul_rn(g.y, i1));
+        }
+    __syncwarp();
+
+    const bool in_q = lane >= 2 && lane < 2 + BQX;
+    const float rfx = 1.0f / A.fx, rfy = 1.0f / A.fy;
+    for (int s = 0; s < A.S; ++s) {
+        const float4* const quads = A.quads + (size_t)s * W * H;
+        float* const gi = A.gI + (size_t)s * W * H;
+        float gp[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        Pending pend[2] = {{0u, 0.0f, 0.0f}, {0u, 0.0f, 0.0f}};
+        auto flush = [&](Pending& q) {
+            red_add(gi + q.idx, q.l);
+            red_add(gi + q.idx + 1, q.r);
+        };
+        float2 ha = make_float2(0.0f, 0.0f), hb = ha;   // row sums of the two rows above
+        for (int r = 0; r < PY; ++r) {
+            float2 g = make_float2(0.0f, 0.0f);
+            if (in_p) {
+                const float2 t = hp[r * HROW];
+                g.x = (ok9[warp][s][r][0] >> lane) & 1u ? t.x : 0.0f;
+                g.y = (ok9[warp][s][r][1] >> lane) & 1u ? t.y : 0.0f;
+            }
+            const float2 gl = make_float2(__shfl_up_sync(kFull, g.x, 1), __shfl_up_sync(kFull, g.y, 1));
+            const float2 gr = make_float2(__shfl_down_sync(kFull, g.x, 1), __shfl_down_sync(kFull, g.y, 1));
+            const float2 hc = __fadd2_rn(__fadd2_rn(gl, g), gr);
+            float2 B = __fadd2_rn(__fadd2_rn(ha, hb), hc);
+            ha = hb;
+            hb = hc;
+            if (r < 2) continue;
+            if (!in_q) B = make_float2(0.0f, 0.0f);
+            if (!__any_sync(kFull, B.x != 0.0f || B.y != 0.0f)) continue;
+            float2 w, rc, u, v;
+            warp_pos(A.hom[s], y0 + r - 2, w, rc, u, v);
+            const float ref = refs[(r - 2) * 32 + lane];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float bj = j ? B.y : B.x;
+                if (bj == 0.0f) continue;   // then some pixel around q is measured, and q's sample is valid
+                const float uj = j ? u.y : u.x, vj = j ? v.y : v.x, rj = j ? rc.y : rc.x;
+                float fu, fv;
+                int iu, iv;
+                floor_split(uj, fu, iu);
+                floor_split(vj, fv, iv);
+                const float a = __fsub_rn(uj, fu), b = __fsub_rn(vj, fv);
+                const unsigned idx = (unsigned)iv * (unsigned)W + (unsigned)iu;
+                if (!PM_IN_BOUNDS(idx, (long long)W * H, kSiteDiffGrad)) continue;
+                const float4 t = __ldg(quads + idx);   // I(x,y), I(x,y+1), I(x+1,y), I(x+1,y+1)
+                const float dx0 = __fsub_rn(t.z, t.x), dx1 = __fsub_rn(t.w, t.y);
+                const float top = __fmaf_rn(a, dx0, t.x), bot = __fmaf_rn(a, dx1, t.y);
+                const float diff = __fsub_rn(ref, __fmaf_rn(b, __fsub_rn(bot, top), top));
+                const float c = diff > 0.0f ? -bj : diff < 0.0f ? bj : 0.0f;
+                if (c == 0.0f) continue;
+                const float a1 = 1.0f - a, b1 = 1.0f - b;
+                // taps; the right and lower ones are 0 on the image's last column and row, where a or b is 0
+                const float ct = c * b1, cb = c * b;
+                float tl = ct * a1, tr = ct * a;
+                Pending& q = pend[j];
+                if (q.idx == idx) {
+                    tl += q.l;
+                    tr += q.r;
+                } else {
+                    flush(q);
+                }
+                red_add(gi + idx, tl);
+                red_add(gi + idx + 1, tr);
+                q.idx = idx + (unsigned)W;
+                q.l = cb * a1;
+                q.r = cb * a;
+                // pose: P = w (U, V, 1); dP = omega x P + rho upsilon; g = dL/dP * w
+                const float dIdu = __fmaf_rn(b, dx1, b1 * dx0);
+                const float dIdv = __fmaf_rn(a, t.w - t.z, a1 * (t.y - t.x));
+                const float U = (uj - A.cx) * rfx, V = (vj - A.cy) * rfy;
+                const float gx = c * dIdu * A.fx, gy = c * dIdv * A.fy;
+                const float gz = -__fmaf_rn(gx, U, gy * V);
+                const float k = (j ? rho.y : rho.x) * rj;
+                gp[0] += __fmaf_rn(V, gz, -gy);
+                gp[1] += __fmaf_rn(-U, gz, gx);
+                gp[2] += __fmaf_rn(U, gy, -V * gx);
+                gp[3] = __fmaf_rn(k, gx, gp[3]);
+                gp[4] = __fmaf_rn(k, gy, gp[4]);
+                gp[5] = __fmaf_rn(k, gz, gp[5]);
+            }
+        }
+        flush(pend[0]);
+        flush(pend[1]);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const float t = warp_sum(gp[i]);
+            if (lane == 0) ps[warp][6 * s + i] = t;
         }
     }
-    // pose gradient: warp sums, one double atomic per warp and component
-    const int lane = threadIdx.x & 31;
-    for (int s = 0; s < A.S; ++s)
-        for (int i = 0; i < 6; ++i) {
-            const float t = warp_sum(gp[s][i]);
-            if (lane == 0 && t != 0.0f) atomicAdd(A.gP + 6 * s + i, (double)t);
-        }
+    __syncthreads();
+    if (tid < 6 * A.S) {
+        double t = 0.0;
+        for (int w = 0; w < BWARPS; ++w) t += (double)ps[w][tid];
+        if (t != 0.0) atomicAdd(A.gP + tid, t);
+    }
+}
+
+// 16 rows per tile halve the share of the two-row rings against 8; images whose grid of 16-row tiles does not
+// give every SM several CTAs take 8 rows.
+cudaError_t launch_cost_bwd(const CostBwdArgs& A, cudaStream_t s) {
+    const int gx = (A.W + 2 + BQX - 1) / BQX, gz = A.D / BPL;
+    const long tall = (long)gx * ((A.H + 2 + 15) / 16) * gz;
+    if (tall >= 148 * 6) cost_bwd_kernel<16><<<dim3(gx, (A.H + 2 + 15) / 16, gz), 32 * BWARPS, 0, s>>>(A);
+    else cost_bwd_kernel<8><<<dim3(gx, (A.H + 2 + 7) / 8, gz), 32 * BWARPS, 0, s>>>(A);
+    return cudaGetLastError();
 }
 
 __global__ void to_quad_f_kernel(int W, int H, const float* __restrict__ img, float4* __restrict__ q) {
@@ -675,8 +805,9 @@ pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void
     CostBwdArgs A;
     std::memset(&A, 0, sizeof A);
     A.ref = d->ref;
-    A.srcs = d->srcs;
+    A.quads = d->quads;
     A.gC = d->gC;
+    A.count = d->sums + 1;
     A.invalid = d->invalid;
     for (int s = 0; s < S; ++s)
         for (int i = 0; i < 12; ++i) A.hom[s][i] = d->hom[s][i];
@@ -692,8 +823,7 @@ pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void
     A.drho = c.rho_step;
     A.gI = grad_srcs;
     A.gP = d->gP;
-    cost_bwd_kernel<<<(unsigned)((d->V + 127) / 128), 128, 0, st>>>(A);
-    PD_CK(d, cudaGetLastError());
+    PD_CK(d, launch_cost_bwd(A, st));
     PD_CK(d, cudaMemcpyAsync(grad_pose, d->gP, 6 * sizeof(double) * S, cudaMemcpyDeviceToHost, st));
     PD_CK(d, cudaStreamSynchronize(st));
     return PM_OK;
