@@ -2,261 +2,317 @@
 // its hand-written adjoint.
 //
 // Forward:  C = corrected 3x3 absolute-difference cost averaged over the valid sources (the cost
-//           kernel of cost.cu, exact bilinear, FP32); 8 SGM paths (sgm.cu:57-108) whose internal
-//           states L_r are kept (or recomputed per path in the backward); S = sum_r L_r;
+//           kernel of cost.cu, exact bilinear, FP32); 8 SGM paths (sgm.cu:57-108), the opposite ones
+//           summed into one volume per pair; S = sum of the pairs;
 //           rho_hat = sum_d softmax(-S/T)_d rho_d; loss = mean over valid pixels with rho_gt > 0 of
-//           |rho_hat - rho_gt|.
-// Backward: the soft-argmin Jacobian gives dS; each path is walked in reverse along its scanlines
-//           and the adjoint is routed through the minima the forward took (same FP32 operations,
-//           so ties resolve identically): to the same plane, the nearer neighbour plane (+P1) or
-//           the path minimum (+P2), and minus the path minimum's plane for the subtracted minimum;
+//           |rho_hat - rho_gt|; and the adjoint dS of the sum by the soft-argmin Jacobian.
+// Backward: each path is walked in reverse along its scanlines and the adjoint is routed through the
+//           minima the forward took, which it left as 2-bit records: to the same plane, the nearer
+//           neighbour plane (+P1) or the path minimum (+P2), and minus the path minimum's plane for
+//           the subtracted minimum;
 //           dC then flows through the absolute differences (their sign), into the source
 //           intensities by the bilinear weights and into the 6-DoF pose of every source through
 //           the spatial derivative of the bilinear sample and the projection, as the left se(3)
 //           perturbation P_s -> exp([omega]) P_s + upsilon (omega first).
 // One warp per scanline for the paths (lane l holds planes [l*PPL, (l+1)*PPL)); tiles of positions for the
 // cost adjoint, with atomics into the intensity gradient and per-CTA reductions of the pose gradient.
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
 
-#include "pm_device.cuh"
 #include "pm_stereo.h"
+#include "sgm_device.cuh"
 
+namespace pm {
 namespace {
-
-using namespace pm;
-
-constexpr int kDirs8[8][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, 1}, {-1, -1}, {-1, 1}, {1, -1}};
-
-__host__ __device__ inline int nchains(int dx, int dy, int W, int H) {
-    return dy == 0 ? H : (dx == 0 ? W : W + H - 1);
-}
-
-// start pixel and length of chain c of direction (dx, dy)
-__device__ inline void chain_of(int c, int dx, int dy, int W, int H, int& x, int& y, int& n) {
-    if (dy == 0) { x = dx > 0 ? 0 : W - 1; y = c; }
-    else if (dx == 0) { x = c; y = dy > 0 ? 0 : H - 1; }
-    else if (c < W) { x = c; y = dy > 0 ? 0 : H - 1; }
-    else { x = dx > 0 ? 0 : W - 1; y = dy > 0 ? (c - W + 1) : (c - W); }
-    const int nx = dx > 0 ? W - x : (dx < 0 ? x + 1 : 1 << 30);
-    const int ny = dy > 0 ? H - y : (dy < 0 ? y + 1 : 1 << 30);
-    n = nx < ny ? nx : ny;
-}
 
 __device__ inline float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
     return v;
 }
 
-// lowest plane index holding the warp-wide minimum m of the lane vectors
-template <int PPL> __device__ inline int argmin_plane(const float (&L)[PPL], float m, int lane) {
-    int j = PPL;
-#pragma unroll
-    for (int t = PPL - 1; t >= 0; --t)
-        if (L[t] == m) j = t;
-    const unsigned b = __ballot_sync(kFull, j < PPL);
-    const int src = __ffs(b) - 1;
-    return src * PPL + __shfl_sync(kFull, j, src);
+// ---- forward paths ------------------------------------------------------------------------
+// The product's pair recurrences (sgm_pair_block), which also leave the records that the adjoint
+// routes by: 2 bits per voxel and path and one plane index per pixel and path, where the path states
+// themselves would take 32.  Bound by memory like the product's: two reads of the costs, a store and a
+// reduction per pair, 20 bytes per voxel and pair, and 0.5 for the records.  All eight paths at 640x480x128:
+// 0.94 ms (one path after the other, each adding to the sum and storing its states: 5.0 ms).
+constexpr int kPairWarps = 2;   // scanlines per block: small blocks spread an image's scanlines over the SMs
+
+template <int PPL>
+__global__ void __launch_bounds__(32 * kPairWarps) diff_fwd_kernel(const SgmLaunch a, const RouteOut ro, const PairSet ps) {
+    extern __shared__ __align__(16) unsigned char ring[];
+    int bx = blockIdx.x, dx, dy;
+    const int pair = pair_of_block(ps, bx);
+    pair_dir(pair, dx, dy);
+    sgm_pair_block<PPL, false, kPairWarps, true, false, true>(a, dx, dy, 2 * pair, bx, ring, &ro);
 }
 
-struct PathArgs {
-    const float* C;          // V cost volume
-    const uint8_t* invalid;  // N, 1 = pixel invalid (its cost counts as 0)
-    const float* ref;        // N reference image (adaptive penalties)
-    float* L;                // V path states (written by the forward, read by the backward)
-    float* S;                // V sum of the paths (forward, accumulated) or nullptr
-    const float* gS;         // V adjoint of S (backward)
-    float* gC;               // V adjoint of C (backward, accumulated)
-    int W, H, D, dx, dy;
-    float p1, p2, tau, q1, q2;
+// ---- adjoint of the paths -----------------------------------------------------------------
+struct AdjArgs {
+    const float* gS;             // V adjoint of the sum
+    const uint32_t* codes[8];    // records of the forward (RouteOut)
+    const uint8_t* arg[8];
+    float* out[4];               // V per pair: the adjoint of the costs through both its paths
+    int acc[4];                  // 1: added to what out holds
+    int W, H, D;
 };
 
-__device__ inline void penalty(const PathArgs& a, long p, long pp, float& P1, float& P2) {
-    P1 = a.p1;
-    P2 = a.p2;
-    if (fabsf(__fsub_rn(a.ref[p], a.ref[pp])) < a.tau) {
-        P1 = __fmul_rn(P1, a.q1);
-        P2 = __fmul_rn(P2, a.q2);
-    }
-}
-
-// Forward of one path: L(p, d) = C'(p, d) + min(L(p', d), min(L(p', d-1), L(p', d+1)) + P1, m + P2) - m.
+// One adjoint recurrence along a scanline: lambda = gS + mu; the planes' lambda go to the
+// predecessor's planes that the forward's minima took (the same, the lower or the upper one), and the
+// plane of the predecessor's minimum receives the lambda that took the minimum, less all of them for
+// the subtracted minimum: together the negative sum over the planes that did not take it.
 template <int PPL>
-__global__ void __launch_bounds__(128) path_fwd_kernel(const PathArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (c >= nchains(a.dx, a.dy, a.W, a.H)) return;
-    int x, y, n;
-    chain_of(c, a.dx, a.dy, a.W, a.H, x, y, n);
-    const long step = (long)a.dy * a.W + a.dx;
-    long p = (long)y * a.W + x;
-    float L[PPL];
-    float m = 0.0f;
-    for (int k = 0; k < n; ++k, p += step) {
-        const bool inv = a.invalid[p] != 0;
-        float cv[PPL];
-        load_planes<PPL>(cv, a.C + (size_t)p * a.D + lane * PPL);
-        float Ln[PPL];
-        if (k == 0) {
-#pragma unroll
-            for (int j = 0; j < PPL; ++j) Ln[j] = inv ? 0.0f : cv[j];
-        } else {
-            float P1, P2;
-            penalty(a, p, p - step, P1, P2);
-            const float mP2 = __fadd_rn(m, P2);
-            float lm = __shfl_up_sync(kFull, L[PPL - 1], 1);
-            float lp = __shfl_down_sync(kFull, L[0], 1);
-            if (lane == 0) lm = inf_f();
-            if (lane == 31) lp = inf_f();
-#pragma unroll
-            for (int j = 0; j < PPL; ++j) {
-                const float left = j == 0 ? lm : L[j - 1];
-                const float right = j == PPL - 1 ? lp : L[j + 1];
-                const float vv = fminf(fminf(L[j], mP2), __fadd_rn(fminf(left, right), P1));
-                Ln[j] = __fsub_rn(__fadd_rn(inv ? 0.0f : cv[j], vv), m);
-            }
-        }
-        float lmin = inf_f();
-#pragma unroll
-        for (int j = 0; j < PPL; ++j) {
-            L[j] = Ln[j];
-            lmin = fminf(lmin, Ln[j]);
-        }
-        m = warp_min_f32(lmin);
-        if (a.L) store_planes<PPL>(a.L + (size_t)p * a.D + lane * PPL, L);
-        if (a.S) {
-            float sv[PPL];
-            load_planes<PPL>(sv, a.S + (size_t)p * a.D + lane * PPL);
-#pragma unroll
-            for (int j = 0; j < PPL; ++j) sv[j] = __fadd_rn(sv[j], L[j]);
-            store_planes<PPL>(a.S + (size_t)p * a.D + lane * PPL, sv);
-        }
-    }
-}
-
-// Adjoint of one path, walking each scanline from its end: lambda = gS + routed adjoint;
-// gC += lambda at valid pixels; lambda is routed to the predecessor's planes along the forward's
-// minima.
-template <int PPL>
-__global__ void __launch_bounds__(128) path_bwd_kernel(const PathArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (c >= nchains(a.dx, a.dy, a.W, a.H)) return;
-    int x, y, n;
-    chain_of(c, a.dx, a.dy, a.W, a.H, x, y, n);
-    const long step = (long)a.dy * a.W + a.dx;
-    long p = (long)y * a.W + x + (long)(n - 1) * step;
-    float mu[PPL];
-#pragma unroll
-    for (int j = 0; j < PPL; ++j) mu[j] = 0.0f;
-    for (int k = n - 1; k >= 0; --k, p -= step) {
-        float lam[PPL], g[PPL];
-        load_planes<PPL>(g, a.gS + (size_t)p * a.D + lane * PPL);
-#pragma unroll
-        for (int j = 0; j < PPL; ++j) lam[j] = __fadd_rn(g[j], mu[j]);
-        if (!a.invalid[p]) {
-            float gc[PPL];
-            load_planes<PPL>(gc, a.gC + (size_t)p * a.D + lane * PPL);
-#pragma unroll
-            for (int j = 0; j < PPL; ++j) gc[j] = __fadd_rn(gc[j], lam[j]);
-            store_planes<PPL>(a.gC + (size_t)p * a.D + lane * PPL, gc);
-        }
-        if (k == 0) break;
-        const long pp = p - step;
-        float Lp[PPL];
-        load_planes<PPL>(Lp, a.L + (size_t)pp * a.D + lane * PPL);
-        float P1, P2;
-        penalty(a, p, pp, P1, P2);
-        float lmin = inf_f();
-#pragma unroll
-        for (int j = 0; j < PPL; ++j) lmin = fminf(lmin, Lp[j]);
-        const float m = warp_min_f32(lmin);
-        const int km = argmin_plane<PPL>(Lp, m, lane);
-        const float mP2 = __fadd_rn(m, P2);
-        float lm = __shfl_up_sync(kFull, Lp[PPL - 1], 1);
-        float lp = __shfl_down_sync(kFull, Lp[0], 1);
-        if (lane == 0) lm = inf_f();
-        if (lane == 31) lp = inf_f();
-        float same[PPL], toL[PPL], toR[PPL];
-        float p2 = 0.0f, tot = 0.0f;
-#pragma unroll
-        for (int j = 0; j < PPL; ++j) {
-            const float left = j == 0 ? lm : Lp[j - 1];
-            const float right = j == PPL - 1 ? lp : Lp[j + 1];
-            const float nb = __fadd_rn(fminf(left, right), P1);
-            const float vmin = fminf(fminf(Lp[j], mP2), nb);
-            same[j] = toL[j] = toR[j] = 0.0f;
-            if (Lp[j] == vmin) same[j] = lam[j];
-            else if (nb == vmin) { if (left <= right) toL[j] = lam[j]; else toR[j] = lam[j]; }
-            else p2 = __fadd_rn(p2, lam[j]);
-            tot = __fadd_rn(tot, lam[j]);
-        }
-        // contributions crossing lane boundaries: plane 0's "to d-1" goes to the previous lane's
-        // last plane, the last plane's "to d+1" to the next lane's first plane
-        const float fromR = __shfl_down_sync(kFull, toL[0], 1);        // lane+1's plane 0 -> my last
-        const float fromL = __shfl_up_sync(kFull, toR[PPL - 1], 1);    // lane-1's last -> my plane 0
-        const float kmadd = __fsub_rn(warp_sum(p2), warp_sum(tot));
-#pragma unroll
-        for (int j = 0; j < PPL; ++j) {
-            float v = same[j];
-            if (j + 1 < PPL) v = __fadd_rn(v, toL[j + 1]);
-            else if (lane < 31) v = __fadd_rn(v, fromR);
-            if (j > 0) v = __fadd_rn(v, toR[j - 1]);
-            else if (lane > 0) v = __fadd_rn(v, fromL);
-            if (lane * PPL + j == km) v = __fadd_rn(v, kmadd);
-            mu[j] = v;
-        }
-    }
-}
-
-// Soft-argmin and the per-pixel loss terms; gS when grad is set, without the 1 / |valid pixels| of the loss's
-// mean (cost_bwd_kernel applies it).
-template <int PPL>
-__global__ void __launch_bounds__(128) soft_kernel(const float* __restrict__ S, const float* __restrict__ rho_gt,
-                                                   const uint8_t* __restrict__ invalid, int N, int D, float rho0,
-                                                   float drho, float T, float* rho_hat, double* sums,
-                                                   const double* count, float* gS) {
-    const int lane = threadIdx.x & 31;
-    const long p = (long)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (p >= N) return;
-    float s[PPL];
-    load_planes<PPL>(s, S + (size_t)p * D + lane * PPL);
-    float lmin = inf_f();
-#pragma unroll
-    for (int j = 0; j < PPL; ++j) lmin = fminf(lmin, s[j]);
-    const float smin = warp_min_f32(lmin);
-    float w[PPL], z = 0.0f, r = 0.0f;
+__device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[PPL], const uint32_t (&w)[2 * PPL],
+                                             int arg, int lane, float (&lam)[PPL]) {
+    const unsigned bit = 1u << lane;
+    add_planes<PPL>(lam, g, mu);
+    float lo[PPL], hi[PPL], direct = 0.0f;   // to the lower and the upper plane
 #pragma unroll
     for (int j = 0; j < PPL; ++j) {
-        w[j] = expf(-(s[j] - smin) / T);
-        z += w[j];
-        r += w[j] * (rho0 + (float)(lane * PPL + j) * drho);
+        const unsigned b0 = w[2 * j], b1 = w[2 * j + 1];
+        mu[j] = ((b0 | b1) & bit) ? 0.0f : lam[j];
+        lo[j] = (b0 & ~b1 & bit) ? lam[j] : 0.0f;
+        hi[j] = (b1 & ~b0 & bit) ? lam[j] : 0.0f;
+        direct += (b0 & b1 & bit) ? 0.0f : lam[j];
     }
-    z = warp_sum(z);
-    r = warp_sum(r);
-    const float rh = r / z;
-    const bool in = !invalid[p] && rho_gt[p] > 0.0f;
-    if (!gS) {
-        if (lane == 0) {
-            if (rho_hat) rho_hat[p] = in ? rh : 0.0f;
-            if (in) {
-                atomicAdd(sums, (double)fabsf(rh - rho_gt[p]));
-                atomicAdd(sums + 1, 1.0);
+    float fromU = __shfl_down_sync(kFull, lo[0], 1);        // lane + 1's first plane -> my last
+    float fromL = __shfl_up_sync(kFull, hi[PPL - 1], 1);    // lane - 1's last plane -> my first
+    if (lane == 31) fromU = 0.0f;
+    if (lane == 0) fromL = 0.0f;
+    const float rest = warp_sum(direct);
+#pragma unroll
+    for (int j = 0; j < PPL; ++j) {
+        float v = mu[j] + (j + 1 < PPL ? lo[j + 1 < PPL ? j + 1 : j] : fromU);
+        v += j > 0 ? hi[j > 0 ? j - 1 : j] : fromL;
+        mu[j] = lane * PPL + j == arg ? v - rest : v;
+    }
+}
+
+// A pair's adjoints: path 2p's from the far end of the scanline, path 2p + 1's from its start, both
+// by one warp, as sgm_pair_block walks the forward: two independent recurrences in flight, gS and the
+// records streamed PF steps ahead, the first visit of a pixel stores and the second adds.  Bound by
+// memory: two reads of gS, a store and a reduction, 20 bytes per voxel and pair (0.55 ms for all eight paths at
+// 640x480x128, 5.8 TB/s; path by path from the stored states 6.4 ms).
+template <int PPL, int NW>
+__device__ __forceinline__ void adjoint_pair_block(const AdjArgs& a, int pair, int bx, unsigned char* ring) {
+    constexpr int SLICE_B = 128 * PPL, REC_B = PPL == 1 ? 16 : 8 * PPL;
+    constexpr int CHAIN_B = SLICE_B + REC_B, STAGE_B = 2 * CHAIN_B;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int W = a.W, H = a.H, D = a.D;
+    int dx, dy;
+    pair_dir(pair, dx, dy);
+    const int c = bx * NW + warp;
+    if (c >= num_chains(dx, dy, W, H)) return;   // warp-uniform; no block barriers below
+    const Chain ch = chain_start(c, dx, dy, W, H);
+    const int n = ch.n;
+    const long step = (long)dy * W + dx;
+    const long pf0 = (long)ch.y * W + ch.x, pb0 = pf0 + (long)(n - 1) * step;
+    const long npix = (long)W * H;
+    [[maybe_unused]] const long long nvox = (long long)npix * D;
+    float* const out = a.out[pair];
+    const bool acc = a.acc[pair] != 0;
+    unsigned char* const wbase = ring + (size_t)warp * PF * STAGE_B;
+
+    // walker 0: path 2p's adjoint, pixel pb0 - k * step; walker 1: path 2p + 1's, pixel pf0 + k * step
+    auto pixel = [&](int walker, int k) { return walker ? pf0 + (long)k * step : pb0 - (long)k * step; };
+    auto issue = [&](unsigned char* sb, int k) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const long pix = pixel(v, k);
+            if (!PM_IN_BOUNDS(pix, npix, kSiteDiffGrad)) continue;
+            unsigned char* const s = sb + v * CHAIN_B;
+            cp_async_bytes<4 * PPL>(s + lane * 4 * PPL, a.gS + (size_t)pix * D + lane * PPL);
+            const uint32_t* rec = a.codes[2 * pair + v] + (size_t)pix * (2 * PPL);
+            if constexpr (PPL == 1) {
+                if (lane == 0) cp_async_8(s + SLICE_B, rec);
+            } else {
+                if (lane < PPL / 2) cp_async_16(s + SLICE_B + 16 * lane, rec + 4 * lane);
             }
         }
-        return;
+    };
+#pragma unroll 1
+    for (int k = 0; k < PF; ++k) {
+        if (k < n) issue(wbase + k * STAGE_B, k);
+        cp_async_commit();
     }
-    float g = 0.0f;
-    if (in) {
-        const float diff = rh - rho_gt[p];
-        g = diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
-    }
-    float o[PPL];
+    // plane indices of steps k0 + lane, a batch of 32 ahead (the last step routes nothing)
+    auto arg_at = [&](int walker, int k) {
+        const long pix = pixel(walker, k);
+        return k + 1 < n && PM_IN_BOUNDS(pix, npix, kSiteDiffRoute) ? (int)__ldg(a.arg[2 * pair + walker] + pix) : 0;
+    };
+    int arg0 = 0, arg1 = 0, next0 = arg_at(0, lane), next1 = arg_at(1, lane);
+    float mu0[PPL], mu1[PPL];
 #pragma unroll
-    for (int j = 0; j < PPL; ++j)
-        o[j] = g * (-1.0f / T) * (w[j] / z) * ((rho0 + (float)(lane * PPL + j) * drho) - rh);
-    store_planes<PPL>(gS + (size_t)p * D + lane * PPL, o);
+    for (int j = 0; j < PPL; ++j) mu0[j] = mu1[j] = 0.0f;
+    int st = 0;
+
+    auto body = [&](int k, float (&l0)[PPL], float (&l1)[PPL]) {
+        const int b = k & 31;
+        if (b == 0) {
+            arg0 = next0;
+            arg1 = next1;
+            next0 = arg_at(0, k + 32 + lane);
+            next1 = arg_at(1, k + 32 + lane);
+        }
+        cp_async_wait<PF - 1>();
+        __syncwarp();   // the records are copied by a few lanes and read by all
+        unsigned char* const sb = wbase + st * STAGE_B;
+        float g[PPL];
+        uint32_t w[2 * PPL];
+        auto load = [&](const unsigned char* s) {
+            load_planes<PPL>(g, reinterpret_cast<const float*>(s + lane * 4 * PPL));
+            if constexpr (PPL == 1) {
+                const uint2 t = *reinterpret_cast<const uint2*>(s + SLICE_B);
+                w[0] = t.x; w[1] = t.y;
+            } else {
+#pragma unroll
+                for (int i = 0; i < PPL / 2; ++i) {
+                    const uint4 t = *reinterpret_cast<const uint4*>(s + SLICE_B + 16 * i);
+                    w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
+                }
+            }
+        };
+        load(sb);
+        adjoint_step<PPL>(g, mu0, w, __shfl_sync(kFull, arg0, b), lane, l0);
+        load(sb + CHAIN_B);
+        adjoint_step<PPL>(g, mu1, w, __shfl_sync(kFull, arg1, b), lane, l1);
+        __syncwarp();   // every lane has read the stage that is refilled
+        if (k + PF < n) issue(sb, k + PF);
+        cp_async_commit();
+        st = (st + 1 == PF) ? 0 : st + 1;
+    };
+    auto put = [&](long pix, const float (&v)[PPL], bool add) {
+        float* const q = out + (size_t)pix * D + lane * PPL;
+        if (!PM_RANGE_IN_BOUNDS(q - out, PPL, nvox, kSiteDiffGrad)) return;
+        if (add) red_planes<PPL>(q, v);
+        else store_planes<PPL>(q, v);
+    };
+    const int half = n >> 1;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        float l0[PPL], l1[PPL];
+        body(k, l0, l1);
+        const long p0 = pixel(0, k), p1 = pixel(1, k);
+        if (p0 == p1) {   // the middle of an odd scanline
+            add_planes<PPL>(l0, l0, l1);
+            put(p0, l0, acc);
+        } else {
+            put(p0, l0, acc || k >= half);
+            put(p1, l1, acc || k >= half);
+        }
+    }
+    cp_async_wait<0>();
+}
+
+template <int PPL>
+__global__ void __launch_bounds__(32 * kPairWarps) diff_adj_kernel(const AdjArgs a, const PairSet ps) {
+    extern __shared__ __align__(16) unsigned char ring[];
+    int bx = blockIdx.x;
+    const int pair = pair_of_block(ps, bx);
+    adjoint_pair_block<PPL, kPairWarps>(a, pair, bx, ring);
+}
+
+// a += b over n floats (n a multiple of 4)
+__global__ void __launch_bounds__(256) fold_kernel(float4* __restrict__ a, const float4* __restrict__ b, size_t n4) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
+        float4 x = a[i];
+        const float4 y = b[i];
+        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+        a[i] = x;
+    }
+}
+
+// ---- soft-argmin --------------------------------------------------------------------------
+struct SoftArgs {
+    const float* vol[4];      // the pair volumes; their sum is the SGM sum
+    const float* rho_gt;
+    const uint8_t* invalid;
+    float* rho_hat;           // optional
+    float* gS;                // adjoint of the sum, without the 1 / count of the loss's mean
+    double* sums;             // loss sum, count
+    int N, D;
+    float rho0, drho, T;
+};
+
+// The sum of the pair volumes (in the product's order, (v0 + v1) + (v2 + v3), or with v2 + v3 folded into v2
+// beforehand), the soft-argmin over it, the loss's terms and its adjoint, one warp per pixel with the next
+// pixel's volumes in flight.  Bound by memory: NV reads and a write per voxel (0.17 ms at 640x480x128).  The loss is summed in double
+// precision per warp, block and grid.
+template <int PPL, int NV>
+__global__ void __launch_bounds__(256) soft_kernel(const SoftArgs a) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long nw = (long)gridDim.x * 8;
+    long p = (long)blockIdx.x * 8 + warp;
+    float next[NV][PPL];
+    auto load = [&](long pix) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            if (PM_RANGE_IN_BOUNDS((long long)pix * a.D + lane * PPL, PPL, (long long)a.N * a.D, kSiteDiffGrad))
+                load_planes<PPL>(next[v], a.vol[v] + (size_t)pix * a.D + lane * PPL);
+    };
+    if (p < a.N) load(p);
+    double loss = 0.0;
+    int count = 0;
+    for (; p < a.N; p += nw) {
+        float s[PPL];
+        if constexpr (NV == 4) {
+            float t[PPL];
+            add_planes<PPL>(s, next[0], next[1]);
+            add_planes<PPL>(t, next[2], next[3]);
+            add_planes<PPL>(s, s, t);
+        } else {
+            add_planes<PPL>(s, next[0], next[1]);
+            add_planes<PPL>(s, s, next[2]);
+        }
+        if (p + nw < a.N) load(p + nw);
+        float lmin = s[0];
+#pragma unroll
+        for (int j = 1; j < PPL; ++j) lmin = fminf(lmin, s[j]);
+        const float smin = warp_min_f32(lmin);
+        float w[PPL], z = 0.0f, r = 0.0f;
+#pragma unroll
+        for (int j = 0; j < PPL; ++j) {
+            w[j] = expf(-(s[j] - smin) / a.T);
+            z += w[j];
+            r += w[j] * (a.rho0 + (float)(lane * PPL + j) * a.drho);
+        }
+        z = warp_sum(z);
+        r = warp_sum(r);
+        const float rh = r / z, gt = a.rho_gt[p];
+        const bool in = !a.invalid[p] && gt > 0.0f;
+        const float diff = rh - gt;
+        if (lane == 0 && a.rho_hat) a.rho_hat[p] = in ? rh : 0.0f;
+        if (in) {
+            loss += (double)fabsf(diff);
+            ++count;
+        }
+        const float g = !in ? 0.0f : diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
+        const float k = g * (-1.0f / a.T) / z;
+        float o[PPL];
+#pragma unroll
+        for (int j = 0; j < PPL; ++j) o[j] = k * w[j] * ((a.rho0 + (float)(lane * PPL + j) * a.drho) - rh);
+        if (PM_RANGE_IN_BOUNDS((long long)p * a.D + lane * PPL, PPL, (long long)a.N * a.D, kSiteDiffGrad))
+            store_planes<PPL>(a.gS + (size_t)p * a.D + lane * PPL, o);
+    }
+    __shared__ double sl[8];
+    __shared__ int sc[8];
+    if (lane == 0) {
+        sl[warp] = loss;
+        sc[warp] = count;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i) {
+            loss += sl[i];
+            count += sc[i];
+        }
+        if (count) {
+            atomicAdd(a.sums, loss);
+            atomicAdd(a.sums + 1, (double)count);
+        }
+    }
 }
 
 constexpr int kMaxDiffSources = 4;
@@ -264,7 +320,8 @@ constexpr int kMaxDiffSources = 4;
 struct CostBwdArgs {
     const float* ref;
     const float4* quads;      // S x N: the cost kernel's source quads
-    const float* gC;          // V, scaled below by 1 / count
+    const float* gC[4];       // nv volumes whose sum is the costs' adjoint but for the 1 / count
+    int nv;
     const double* count;      // pixels in the loss
     const uint8_t* invalid;
     float hom[kMaxDiffSources][12];
@@ -329,7 +386,12 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
         if (gx >= 0 && gy >= 0 && gx < W && gy < H) {
             const size_t pix = (size_t)gy * W + gx;
             if (!A.invalid[pix] && PM_RANGE_IN_BOUNDS(pix * D + d0 + k, 4, (long long)W * H * D, kSiteDiffGrad))
-                v = *reinterpret_cast<const float4*>(A.gC + pix * D + d0 + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (i >= A.nv) break;
+                    const float4 t = *reinterpret_cast<const float4*>(A.gC[i] + pix * D + d0 + k);
+                    v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+                }
         }
         *reinterpret_cast<float2*>(hs + p * BSP + k) = make_float2(v.x, v.y);
         *reinterpret_cast<float2*>(hs + p * BSP + k + 2) = make_float2(v.z, v.w);
@@ -523,61 +585,60 @@ __global__ void to_quad_f_kernel(int W, int H, const float* __restrict__ img, fl
     }
 }
 
-template <int PPL> cudaError_t launch_path(const PathArgs& a, bool fwd, cudaStream_t s) {
-    const int nch = nchains(a.dx, a.dy, a.W, a.H);
-    if (fwd) path_fwd_kernel<PPL><<<(nch + 3) / 4, 128, 0, s>>>(a);
-    else path_bwd_kernel<PPL><<<(nch + 3) / 4, 128, 0, s>>>(a);
+template <int PPL> cudaError_t launch_fwd_t(const SgmLaunch& a, const RouteOut& ro, unsigned mask, cudaStream_t s) {
+    const PairSet ps = make_pair_set(mask, a.W, a.H, kPairWarps);
+    const size_t smem = (size_t)kPairWarps * PF * Ring<PPL, false>::STAGE_B;
+    diff_fwd_kernel<PPL><<<ps.start[ps.n], 32 * kPairWarps, smem, s>>>(a, ro, ps);
     return cudaGetLastError();
 }
-
-cudaError_t launch_path_any(const PathArgs& a, bool fwd, cudaStream_t s) {
-    switch (a.D / 32) {
-        case 1: return launch_path<1>(a, fwd, s);
-        case 2: return launch_path<2>(a, fwd, s);
-        case 4: return launch_path<4>(a, fwd, s);
-        case 8: return launch_path<8>(a, fwd, s);
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-template <int PPL>
-cudaError_t launch_soft(const float* S, const float* rgt, const uint8_t* inv, int N, int D, float rho0, float drho,
-                        float T, float* rho_hat, double* sums, const double* count, float* gS, cudaStream_t s) {
-    soft_kernel<PPL><<<(N + 3) / 4, 128, 0, s>>>(S, rgt, inv, N, D, rho0, drho, T, rho_hat, sums, count, gS);
+template <int PPL> cudaError_t launch_adj_t(const AdjArgs& a, unsigned mask, cudaStream_t s) {
+    const PairSet ps = make_pair_set(mask, a.W, a.H, kPairWarps);
+    const size_t smem = (size_t)kPairWarps * PF * 2 * (128 * PPL + (PPL == 1 ? 16 : 8 * PPL));
+    diff_adj_kernel<PPL><<<ps.start[ps.n], 32 * kPairWarps, smem, s>>>(a, ps);
     return cudaGetLastError();
 }
-
-cudaError_t launch_soft_any(const float* S, const float* rgt, const uint8_t* inv, int N, int D, float rho0,
-                            float drho, float T, float* rho_hat, double* sums, const double* count, float* gS,
-                            cudaStream_t s) {
-    switch (D / 32) {
-        case 1: return launch_soft<1>(S, rgt, inv, N, D, rho0, drho, T, rho_hat, sums, count, gS, s);
-        case 2: return launch_soft<2>(S, rgt, inv, N, D, rho0, drho, T, rho_hat, sums, count, gS, s);
-        case 4: return launch_soft<4>(S, rgt, inv, N, D, rho0, drho, T, rho_hat, sums, count, gS, s);
-        case 8: return launch_soft<8>(S, rgt, inv, N, D, rho0, drho, T, rho_hat, sums, count, gS, s);
-        default: return cudaErrorInvalidValue;
+template <int PPL> cudaError_t launch_soft_t(const SoftArgs& a, int nv, cudaStream_t s) {
+    const int blocks = std::min((a.N + 7) / 8, 148 * 6);
+    if (nv == 4) soft_kernel<PPL, 4><<<blocks, 256, 0, s>>>(a);
+    else soft_kernel<PPL, 3><<<blocks, 256, 0, s>>>(a);
+    return cudaGetLastError();
+}
+#define PM_DIFF_BY_PLANES(D, CALL)                       \
+    switch ((D) / 32) {                                  \
+        case 1: { constexpr int P = 1; return CALL; }    \
+        case 2: { constexpr int P = 2; return CALL; }    \
+        case 4: { constexpr int P = 4; return CALL; }    \
+        case 8: { constexpr int P = 8; return CALL; }    \
+        default: return cudaErrorInvalidValue;           \
     }
+cudaError_t launch_fwd(const SgmLaunch& a, const RouteOut& ro, unsigned mask, cudaStream_t s) {
+    PM_DIFF_BY_PLANES(a.D, (launch_fwd_t<P>(a, ro, mask, s)))
+}
+cudaError_t launch_adj(const AdjArgs& a, unsigned mask, cudaStream_t s) {
+    PM_DIFF_BY_PLANES(a.D, (launch_adj_t<P>(a, mask, s)))
+}
+cudaError_t launch_soft(const SoftArgs& a, int nv, cudaStream_t s) {
+    PM_DIFF_BY_PLANES(a.D, (launch_soft_t<P>(a, nv, s)))
 }
 
 }  // namespace
+}  // namespace pm
+
+using namespace pm;
 
 struct pm_diff {
     pm_diff_config cfg{};
     size_t N = 0, V = 0;
     float4* quads = nullptr;
-    float* C = nullptr;
+    float* C = nullptr;       // costs; from the soft-argmin on, the adjoint of the SGM sum
     uint8_t* invalid = nullptr;
-    float* S = nullptr;
-    float* L = nullptr;       // 8 path volumes (store_paths) or 1
-    float* gS = nullptr;
-    float* gC = nullptr;
+    float* vol = nullptr;     // forward: pair volumes; backward: their adjoints (4 with store_paths, else 3)
+    uint32_t* codes = nullptr;   // 8 paths' records, N * D / 16 words each
+    uint8_t* arg = nullptr;   // 8 paths' plane indices, N each
     double* sums = nullptr;   // [loss sum, valid count]
     double* gP = nullptr;     // S x 6
-    float* rho_hat = nullptr;
     // inputs of the last forward
     const float* ref = nullptr;
-    const float* srcs = nullptr;
-    const float* rho_gt = nullptr;
     float hom[kMaxSources][12]{};
     float cam[4]{};
     bool have_forward = false;
@@ -585,6 +646,7 @@ struct pm_diff {
     std::string err;
 };
 
+namespace pm {
 namespace {
 
 pm_status dfail(pm_diff* d, pm_status s, const char* msg, cudaError_t e = cudaSuccess) {
@@ -614,31 +676,22 @@ void free_diff(pm_diff* d) {
     cudaFree(d->quads);
     cudaFree(d->C);
     cudaFree(d->invalid);
-    cudaFree(d->S);
-    cudaFree(d->L);
-    cudaFree(d->gS);
-    cudaFree(d->gC);
+    cudaFree(d->vol);
+    cudaFree(d->codes);
+    cudaFree(d->arg);
     cudaFree(d->sums);
     cudaFree(d->gP);
 }
 
-PathArgs path_args(const pm_diff* d, int r) {
-    PathArgs a;
-    std::memset(&a, 0, sizeof a);
-    const pm_diff_config& c = d->cfg;
-    a.C = d->C;
-    a.invalid = d->invalid;
-    a.ref = d->ref;
-    a.W = c.width;
-    a.H = c.height;
-    a.D = c.num_planes;
-    a.dx = kDirs8[r][0];
-    a.dy = kDirs8[r][1];
-    a.p1 = c.p1; a.p2 = c.p2; a.tau = c.tau_so; a.q1 = c.q1; a.q2 = c.q2;
-    return a;
+// Pair p's volume: one each with store_paths.  Else the two diagonal pairs' sum replaces the first one's volume,
+// and the vertical pair, which then runs by itself, takes the second one's; its adjoint is added to pair 0's.
+float* pair_volume(const pm_diff* d, int p) {
+    const int four[4] = {0, 1, 2, 3}, three[4] = {0, 2, 1, 2};
+    return d->vol + (size_t)(d->cfg.store_paths ? four : three)[p] * d->V;
 }
 
 }  // namespace
+}  // namespace pm
 
 extern "C" {
 
@@ -673,7 +726,6 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     d->N = (size_t)c->width * c->height;
     d->V = d->N * c->num_planes;
     DGuard g(c->device);
-    const size_t npaths = c->store_paths ? 8 : 1;
     bool ok = true;
     auto alloc = [&](void** p, size_t b) {
         if (!ok) return;
@@ -683,10 +735,9 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     alloc((void**)&d->quads, 16 * d->N * c->num_sources);
     alloc((void**)&d->C, 4 * d->V);
     alloc((void**)&d->invalid, d->N);
-    alloc((void**)&d->S, 4 * d->V);
-    alloc((void**)&d->L, 4 * d->V * npaths);
-    alloc((void**)&d->gS, 4 * d->V);
-    alloc((void**)&d->gC, 4 * d->V);
+    alloc((void**)&d->vol, 4 * d->V * (c->store_paths ? 4 : 3));
+    alloc((void**)&d->codes, 2 * d->V);
+    alloc((void**)&d->arg, 8 * d->N);
     alloc((void**)&d->sums, 2 * sizeof(double));
     alloc((void**)&d->gP, 6 * sizeof(double) * c->num_sources);
     if (!ok) {
@@ -725,9 +776,6 @@ pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const
     DGuard g(c.device);
     cudaStream_t st = (cudaStream_t)stream;
     d->ref = ref;
-    d->srcs = srcs;
-    d->rho_gt = rho_gt;
-    d->rho_hat = rho_hat;
     // H1 = K R K^-1, H2 = K t for each source-from-reference pose
     const double Ki[9] = {1.0 / K[0], 0.0, -K[2] / K[0], 0.0, 1.0 / K[4], -K[5] / K[4], 0.0, 0.0, 1.0};
     for (int s = 0; s < S; ++s) {
@@ -761,18 +809,52 @@ pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const
     for (int s = 0; s < S; ++s)
         for (int i = 0; i < 12; ++i) a.hom[s][i] = d->hom[s][i];
     a.cost = d->C;
-    a.invalid = d->invalid;
     PD_CK(d, launch_cost(a, st));
-    PD_CK(d, cudaMemsetAsync(d->S, 0, 4 * d->V, st));
+
+    SgmLaunch g0;
+    std::memset(&g0, 0, sizeof g0);
+    g0.cost = d->C;
+    g0.ref = ref;
+    g0.W = W;
+    g0.H = H;
+    g0.D = D;
+    g0.num_paths = 8;
+    g0.p1 = c.p1; g0.p2 = c.p2; g0.tau = c.tau_so; g0.q1 = c.q1; g0.q2 = c.q2;
+    for (int p = 0; p < 4; ++p) g0.part[p] = pair_volume(d, p);
+    RouteOut ro;
     for (int r = 0; r < 8; ++r) {
-        PathArgs pa = path_args(d, r);
-        pa.L = d->L + (c.store_paths ? (size_t)r * d->V : 0);
-        pa.S = d->S;
-        PD_CK(d, launch_path_any(pa, true, st));
+        ro.codes[r] = d->codes + (size_t)r * (d->V / 16);
+        ro.arg[r] = d->arg + (size_t)r * d->N;
+    }
+    ro.invalid = d->invalid;
+    SoftArgs sa;
+    std::memset(&sa, 0, sizeof sa);
+    if (c.store_paths) {
+        PD_CK(d, launch_fwd(g0, ro, 0xfu, st));
+        for (int p = 0; p < 4; ++p) sa.vol[p] = pair_volume(d, p);
+    } else {
+        PD_CK(d, launch_fwd(g0, ro, 0xdu, st));
+        float* const v2 = pair_volume(d, 2);
+        fold_kernel<<<148 * 8, 256, 0, st>>>(reinterpret_cast<float4*>(v2), reinterpret_cast<const float4*>(pair_volume(d, 3)),
+                                             d->V / 4);
+        PD_CK(d, cudaGetLastError());
+        PD_CK(d, launch_fwd(g0, ro, 0x2u, st));
+        sa.vol[0] = pair_volume(d, 0);
+        sa.vol[1] = pair_volume(d, 1);
+        sa.vol[2] = v2;
     }
     PD_CK(d, cudaMemsetAsync(d->sums, 0, 2 * sizeof(double), st));
-    PD_CK(d, launch_soft_any(d->S, rho_gt, d->invalid, (int)d->N, D, c.rho0, c.rho_step, c.temperature, rho_hat,
-                             d->sums, nullptr, nullptr, st));
+    sa.rho_gt = rho_gt;
+    sa.invalid = d->invalid;
+    sa.rho_hat = rho_hat;
+    sa.gS = d->C;
+    sa.sums = d->sums;
+    sa.N = (int)d->N;
+    sa.D = D;
+    sa.rho0 = c.rho0;
+    sa.drho = c.rho_step;
+    sa.T = c.temperature;
+    PD_CK(d, launch_soft(sa, c.store_paths ? 4 : 3, st));
     double h[2];
     PD_CK(d, cudaMemcpyAsync(h, d->sums, sizeof h, cudaMemcpyDeviceToHost, st));
     PD_CK(d, cudaStreamSynchronize(st));
@@ -788,17 +870,25 @@ pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void
     const int S = c.num_sources, D = c.num_planes;
     DGuard g(c.device);
     cudaStream_t st = (cudaStream_t)stream;
-    PD_CK(d, launch_soft_any(d->S, d->rho_gt, d->invalid, (int)d->N, D, c.rho0, c.rho_step, c.temperature, nullptr,
-                             nullptr, d->sums + 1, d->gS, st));
-    PD_CK(d, cudaMemsetAsync(d->gC, 0, 4 * d->V, st));
+    AdjArgs aa;
+    std::memset(&aa, 0, sizeof aa);
+    aa.gS = d->C;
     for (int r = 0; r < 8; ++r) {
-        PathArgs pa = path_args(d, r);
-        pa.L = d->L + (c.store_paths ? (size_t)r * d->V : 0);
-        if (!c.store_paths) PD_CK(d, launch_path_any(pa, true, st));   // recompute this path's states
-        pa.S = nullptr;
-        pa.gS = d->gS;
-        pa.gC = d->gC;
-        PD_CK(d, launch_path_any(pa, false, st));
+        aa.codes[r] = d->codes + (size_t)r * (d->V / 16);
+        aa.arg[r] = d->arg + (size_t)r * d->N;
+    }
+    aa.W = c.width;
+    aa.H = c.height;
+    aa.D = D;
+    const int nv = c.store_paths ? 4 : 3;
+    const int slot[4] = {0, c.store_paths ? 1 : 0, c.store_paths ? 2 : 1, c.store_paths ? 3 : 2};
+    for (int p = 0; p < 4; ++p) aa.out[p] = d->vol + (size_t)slot[p] * d->V;
+    if (c.store_paths) {
+        PD_CK(d, launch_adj(aa, 0xfu, st));
+    } else {
+        PD_CK(d, launch_adj(aa, 0xdu, st));
+        aa.acc[1] = 1;
+        PD_CK(d, launch_adj(aa, 0x2u, st));
     }
     PD_CK(d, cudaMemsetAsync(grad_srcs, 0, 4 * d->N * S, st));
     PD_CK(d, cudaMemsetAsync(d->gP, 0, 6 * sizeof(double) * S, st));
@@ -806,7 +896,8 @@ pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void
     std::memset(&A, 0, sizeof A);
     A.ref = d->ref;
     A.quads = d->quads;
-    A.gC = d->gC;
+    for (int v = 0; v < nv; ++v) A.gC[v] = d->vol + (size_t)v * d->V;
+    A.nv = nv;
     A.count = d->sums + 1;
     A.invalid = d->invalid;
     for (int s = 0; s < S; ++s)

@@ -39,6 +39,7 @@ enum BoundsSite {
     kSiteCpuList,          // CPU-variant fusion: a hitter list entry or the occupant of a cell
     kSiteCpuGather,        // CPU-variant fusion: a neighbour or predecessor cell
     kSiteClassCount,       // pm_stats class counting
+    kSiteDiffRoute,        // differentiation form: a step's record, plane index or invalid flag
     kSiteDiffGrad,         // differentiation form: a voxel of an adjoint volume or a source quad
 };
 

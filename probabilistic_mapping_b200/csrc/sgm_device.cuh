@@ -25,8 +25,41 @@ struct Chain {
     int x, y, n;
 };
 
+// Blocks of NW scanlines of several path pairs in one launch: entry i covers blocks [start[i], start[i + 1]).
+struct PairSet {
+    int n, pair[4], start[5];
+};
+
 __host__ __device__ inline int num_chains(int dx, int dy, int W, int H) {
     return dy == 0 ? H : (dx == 0 ? W : W + H - 1);
+}
+
+// The pairs of `mask` (bit p: pair p), those with the longest scanlines first.
+inline PairSet make_pair_set(unsigned mask, int W, int H, int nw) {
+    PairSet s{};
+    const int wide[4] = {0, 2, 3, 1}, tall[4] = {1, 2, 3, 0};
+    for (int i = 0; i < 4; ++i) {
+        const int p = W >= H ? wide[i] : tall[i];
+        if (!((mask >> p) & 1u)) continue;
+        int dx, dy;
+        pair_dir(p, dx, dy);
+        s.pair[s.n] = p;
+        s.start[s.n + 1] = s.start[s.n] + (num_chains(dx, dy, W, H) + nw - 1) / nw;
+        ++s.n;
+    }
+    return s;
+}
+// The pair of block bx; bx becomes the block's index within it.
+__device__ __forceinline__ int pair_of_block(const PairSet& s, int& bx) {
+    int pair = s.pair[0], first = 0;
+#pragma unroll
+    for (int i = 1; i < 4; ++i)
+        if (i < s.n && bx >= s.start[i]) {
+            pair = s.pair[i];
+            first = s.start[i];
+        }
+    bx -= first;
+    return pair;
 }
 
 // Start pixel of chain c: pixels whose predecessor (x-dx, y-dy) lies outside the image.
@@ -315,13 +348,41 @@ __device__ __forceinline__ void path_first(PathState<PPL>& s, const float (&cv)[
     s.mprev = warp_min_f32(lane_min<PPL, FULL>(s.L, incl));
 }
 
+// The differentiation form's record of one step: which term of the minimum each plane took, as two
+// ballots per plane of a lane (bit l of word 2j / 2j + 1: bit 0 / 1 of plane l * PPL + j's code, see
+// RouteCode), and the lowest plane that holds the predecessor's minimum.
+enum RouteCode { kRouteSame = 0, kRouteLower = 1, kRouteUpper = 2, kRouteMin = 3 };
+template <int PPL> struct Route {
+    uint32_t w[2 * PPL];
+    int arg;
+    bool inv;   // the pixel has a plane that was never measured
+};
+// Where a pass with records puts them, per path: N records of 2 * PPL words and N plane indices; and
+// the invalid flag of every pixel (written by pair 0).
+struct RouteOut {
+    uint32_t* codes[8];
+    uint8_t* arg[8];
+    uint8_t* invalid;
+};
+template <int PPL> __device__ __forceinline__ void store_route(uint32_t* p, const Route<PPL>& r) {
+    if constexpr (PPL == 1) *reinterpret_cast<uint2*>(p) = make_uint2(r.w[0], r.w[1]);
+    else {
+#pragma unroll
+        for (int i = 0; i < 2 * PPL; i += 4)
+            *reinterpret_cast<uint4*>(p + i) = make_uint4(r.w[i], r.w[i + 1], r.w[i + 2], r.w[i + 3]);
+    }
+}
+
 // One pixel step of a path (sgm.cu:57-108): L(p, d) = C(p, d) + min(L(p-r, d), L(p-r, d+-1) + P1,
 // min_k L(p-r, k) + P2) - min_k L(p-r, k), P1/P2 scaled by q1/q2 when the flag q says the
 // reference image's path gradient is below tau; a plane never measured makes the pixel invalid:
 // its cost counts as 0 and the path's output there is COST_INF = 0.  o receives the output.
-template <int PPL, bool FULL>
+// ROUTE: rt receives the step's record; equal terms resolve to the same plane, then to a neighbour (the
+// lower one first), then to the minimum.
+template <int PPL, bool FULL, bool ROUTE = false>
 __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s, const float (&cv)[PPL], bool q,
-                                          float p1q, float p2q, uint32_t incl, int lane, float (&o)[PPL]) {
+                                          float p1q, float p2q, uint32_t incl, int lane, float (&o)[PPL],
+                                          Route<PPL>* rt = nullptr) {
     const bool inv = pixel_invalid<PPL, FULL>(cv, incl);
     const float P1 = q ? p1q : a.p1, P2 = q ? p2q : a.p2;
     const float mP2 = __fadd_rn(s.mprev, P2);
@@ -340,6 +401,20 @@ __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s,
     add_planes<PPL>(nb, nb, P1);
 #pragma unroll
     for (int j = 0; j < PPL; ++j) vv[j] = min3f(s.L[j], mP2, nb[j]);
+    if constexpr (ROUTE) {
+        int at = PPL;
+#pragma unroll
+        for (int j = PPL - 1; j >= 0; --j) {
+            const bool lower = (j == 0 ? lm : s.L[j - 1]) <= (j == PPL - 1 ? lp : s.L[j + 1]);
+            const bool same = s.L[j] == vv[j], side = nb[j] == vv[j];
+            rt->w[2 * j] = __ballot_sync(kFull, !same && (!side || lower));
+            rt->w[2 * j + 1] = __ballot_sync(kFull, !same && (!side || !lower));
+            at = s.L[j] == s.mprev ? j : at;
+        }
+        const int src = __ffs(__ballot_sync(kFull, at < PPL)) - 1;
+        rt->arg = PPL == 1 ? src : src * PPL + __shfl_sync(kFull, at, src);
+        rt->inv = inv;
+    }
     add_planes<PPL>(vv, cz, vv);               // C + val
     add_planes<PPL>(s.L, vv, -s.mprev);        // - minL (:98); the negation is exact
 #pragma unroll
@@ -378,9 +453,10 @@ __device__ __forceinline__ unsigned penalty_flags(float& cur, float& nxt, const 
 // ahead) and turned into one ballot of penalty flags.  The loop is split at the meeting point,
 // so the store and the reduction phases run without a per-step branch.  HOUT: FP16 pair volume.
 // One block of NW warps: scanlines bx*NW .. bx*NW + NW-1; `ring` holds NW * PF * STAGE_B bytes.
-template <int PPL, bool HALF, int NW, bool FULL, bool HOUT>
+// ROUTE: the steps' records go to *ro (paths slot and slot + 1).
+template <int PPL, bool HALF, int NW, bool FULL, bool HOUT, bool ROUTE = false>
 __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int dy, int slot, int bx,
-                                               unsigned char* ring) {
+                                               unsigned char* ring, const RouteOut* ro = nullptr) {
     using CT = typename CostElem<HALF>::T;
     using OT = typename CostElem<HOUT>::T;
     using RG = Ring<PPL, HALF>;
@@ -447,14 +523,33 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
     fs.qmask = penalty_flags(If, Ifn, a.ref, pf0, step, 0, n, lane, a.tau, lastf, npix);
     bs.qmask = penalty_flags(Ib, Ibn, a.ref, pb0, -step, 0, n, lane, a.tau, lastb, npix);
 
+    // ROUTE: the plane indices and invalid flags of the current batch of 32 steps, stored together
+    [[maybe_unused]] int argf = 0, argb = 0;
+    [[maybe_unused]] unsigned rinv = 0;
+    [[maybe_unused]] auto flush_route = [&](int k) {
+        const int kk = (k & ~31) + lane;
+        if (kk > k) return;
+        const long pf = pf0 + (long)kk * step, pb = pb0 - (long)kk * step;
+        if (!PM_IN_BOUNDS(pf, npix, kSiteDiffRoute) || !PM_IN_BOUNDS(pb, npix, kSiteDiffRoute)) return;
+        if (kk > 0) {
+            ro->arg[slot][pf] = (uint8_t)argf;
+            ro->arg[slot + 1][pb] = (uint8_t)argb;
+        }
+        if (slot == 0) ro->invalid[pf] = (uint8_t)((rinv >> lane) & 1u);
+    };
+
     // step 0: the first pixel of both paths
     cp_async_wait<PF - 1>();
     {
         float cf[PPL], cb[PPL], of[PPL], ob[PPL];
         load_slice<PPL, HALF>(cf, wbase + lane * CB);
         load_slice<PPL, HALF>(cb, wbase + CHAIN_B + lane * CB);
+        if constexpr (ROUTE) rinv = pixel_invalid<PPL, FULL>(cf, incl) ? 1u : 0u;
         path_first<PPL, FULL>(fs, cf, incl, of);
         path_first<PPL, FULL>(bs, cb, incl, ob);
+        if constexpr (ROUTE) {
+            if (n == 1) flush_route(0);
+        }
         if (n == 1) {
             meet(of, ob);
             put(qf, of);
@@ -482,8 +577,21 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         load_slice<PPL, HALF>(cf, sb + lane * CB);
         load_slice<PPL, HALF>(cb, sb + CHAIN_B + lane * CB);
         const int bit = k & 31;
-        path_step<PPL, FULL>(a, fs, cf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of);
-        path_step<PPL, FULL>(a, bs, cb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob);
+        if constexpr (ROUTE) {
+            Route<PPL> r;
+            path_step<PPL, FULL, true>(a, fs, cf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of, &r);
+            const long pf = pf0 + (long)k * step, pb = pb0 - (long)k * step;
+            if (lane == 0 && PM_IN_BOUNDS(pf, npix, kSiteDiffRoute)) store_route<PPL>(ro->codes[slot] + pf * (2 * PPL), r);
+            argf = lane == bit ? r.arg : argf;
+            rinv = (bit == 0 ? 0u : rinv) | (r.inv ? 1u << bit : 0u);
+            path_step<PPL, FULL, true>(a, bs, cb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob, &r);
+            if (lane == 0 && PM_IN_BOUNDS(pb, npix, kSiteDiffRoute)) store_route<PPL>(ro->codes[slot + 1] + pb * (2 * PPL), r);
+            argb = lane == bit ? r.arg : argb;
+            if (bit == 31 || k == n - 1) flush_route(k);
+        } else {
+            path_step<PPL, FULL>(a, fs, cf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of);
+            path_step<PPL, FULL>(a, bs, cb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob);
+        }
         // refill this stage (consumed above) with step k + PF
         if (k + PF < n) issue(sb, k + PF);
         cp_async_commit();
