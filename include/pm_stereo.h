@@ -305,7 +305,7 @@ PM_API const char* pm_batch_last_error(const pm_batch* b);
 /* ---------------------------------------------------------------------------------------
  * Differentiation form (no counterpart in the reference): a differentiable depth loss over the
  * path and its hand-written adjoint.  Forward: corrected 3x3 cost averaged over the valid
- * sources, 8 SGM paths (the terms their minima took kept as 2-bit records), soft-argmin
+ * sources, 8 SGM paths (the terms that their minima took kept as records), soft-argmin
  * rho_hat = sum_d softmax(-S/T)_d rho_d, loss = mean |rho_hat - rho_gt| over valid pixels with
  * rho_gt > 0.  Backward: gradients with respect to the source intensities and to the left se(3)
  * perturbation of every source pose (P_s -> exp([omega]) P_s + upsilon; omega first).
@@ -318,8 +318,8 @@ typedef struct pm_diff_config {
     float rho0, rho_step;
     float temperature;   /* soft-argmin temperature in cost units */
     float p1, p2, tau_so, q1, q2;
-    int store_paths;     /* 1: a volume per path pair, all pairs at once; 0: less memory, three volumes
-                            and the last pair by itself (same results) */
+    int store_paths;     /* 1: seven path volumes, all paths at once; 0: less memory, three volumes and
+                            the path pairs in three launches (same results) */
     int device;
 } pm_diff_config;
 PM_API void pm_diff_config_default(pm_diff_config* c, int width, int height, int num_planes, int num_sources);

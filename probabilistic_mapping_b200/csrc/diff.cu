@@ -7,7 +7,7 @@
 //           rho_hat = sum_d softmax(-S/T)_d rho_d; loss = mean over valid pixels with rho_gt > 0 of
 //           |rho_hat - rho_gt|; and the adjoint dS of the sum by the soft-argmin Jacobian.
 // Backward: each path is walked in reverse along its scanlines and the adjoint is routed through the
-//           minima the forward took, which it left as 2-bit records: to the same plane, the nearer
+//           minima the forward took, which it left as records: to the same plane, the nearer
 //           neighbour plane (+P1) or the path minimum (+P2), and minus the path minimum's plane for
 //           the subtracted minimum;
 //           dC then flows through the absolute differences (their sign), into the source
@@ -34,14 +34,13 @@ __device__ inline float warp_sum(float v) {
 
 // ---- forward paths ------------------------------------------------------------------------
 // The product's pair recurrences (sgm_pair_block), which also leave the records that the adjoint
-// routes by: 2 bits per voxel and path and one plane index per pixel and path, where the path states
-// themselves would take 32.  Bound by memory like the product's: two reads of the costs, a store and a
+// routes by: 3 to 4 bits per voxel and path, where the path states themselves would take 32.  Bound by memory like the product's: two reads of the costs, a store and a
 // reduction per pair, 20 bytes per voxel and pair, and 0.5 for the records.  All eight paths at 640x480x128:
 // 0.94 ms (one path after the other, each adding to the sum and storing its states: 5.0 ms).
 constexpr int kPairWarps = 2;   // scanlines per block: small blocks spread an image's scanlines over the SMs
 
 template <int PPL>
-__global__ void __launch_bounds__(32 * kPairWarps) diff_fwd_kernel(const SgmLaunch a, const RouteOut ro, const PairSet ps) {
+__global__ void __launch_bounds__(32 * kPairWarps, PPL <= 4 ? 12 : 1) diff_fwd_kernel(const SgmLaunch a, const RouteOut ro, const PairSet ps) {
     extern __shared__ __align__(16) unsigned char ring[];
     int bx = blockIdx.x, dx, dy;
     const int pair = pair_of_block(ps, bx);
@@ -52,10 +51,10 @@ __global__ void __launch_bounds__(32 * kPairWarps) diff_fwd_kernel(const SgmLaun
 // ---- adjoint of the paths -----------------------------------------------------------------
 struct AdjArgs {
     const float* gS;             // V adjoint of the sum
-    const uint32_t* codes[8];    // records of the forward (RouteOut)
-    const uint8_t* arg[8];
-    float* out[4];               // V per pair: the adjoint of the costs through both its paths
-    int acc[4];                  // 1: added to what out holds
+    const uint32_t* codes;       // records of the forward (RouteOut)
+    float* vol;                  // volumes of V: the adjoint of the costs through a pair's two paths ...
+    unsigned slots;              // ... goes to volume (slots >> 2 * pair) & 3
+    unsigned acc;                // bit p: pair p's is added to what its volume holds
     int W, H, D;
 };
 
@@ -64,18 +63,18 @@ struct AdjArgs {
 // plane of the predecessor's minimum receives the lambda that took the minimum, less all of them for
 // the subtracted minimum: together the negative sum over the planes that did not take it.
 template <int PPL>
-__device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[PPL], const uint32_t (&w)[2 * PPL],
-                                             int arg, int lane, float (&lam)[PPL]) {
+__device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[PPL],
+                                             const uint32_t (&w)[Route<PPL>::WORDS], int lane, float (&lam)[PPL]) {
     const unsigned bit = 1u << lane;
     add_planes<PPL>(lam, g, mu);
     float lo[PPL], hi[PPL], direct = 0.0f;   // to the lower and the upper plane
 #pragma unroll
     for (int j = 0; j < PPL; ++j) {
-        const unsigned b0 = w[2 * j], b1 = w[2 * j + 1];
-        mu[j] = ((b0 | b1) & bit) ? 0.0f : lam[j];
-        lo[j] = (b0 & ~b1 & bit) ? lam[j] : 0.0f;
-        hi[j] = (b1 & ~b0 & bit) ? lam[j] : 0.0f;
-        direct += (b0 & b1 & bit) ? 0.0f : lam[j];
+        const unsigned same = w[3 * j], side = w[3 * j + 1], lower = w[3 * j + 2];
+        mu[j] = (same & bit) ? lam[j] : 0.0f;
+        lo[j] = (~same & side & lower & bit) ? lam[j] : 0.0f;
+        hi[j] = (~same & side & ~lower & bit) ? lam[j] : 0.0f;
+        direct += ((same | side) & bit) ? lam[j] : 0.0f;
     }
     float fromU = __shfl_down_sync(kFull, lo[0], 1);        // lane + 1's first plane -> my last
     float fromL = __shfl_up_sync(kFull, hi[PPL - 1], 1);    // lane - 1's last plane -> my first
@@ -86,7 +85,7 @@ __device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[
     for (int j = 0; j < PPL; ++j) {
         float v = mu[j] + (j + 1 < PPL ? lo[j + 1 < PPL ? j + 1 : j] : fromU);
         v += j > 0 ? hi[j > 0 ? j - 1 : j] : fromL;
-        mu[j] = lane * PPL + j == arg ? v - rest : v;
+        mu[j] = (unsigned)(lane * PPL + j) == w[3 * PPL] ? v - rest : v;
     }
 }
 
@@ -97,7 +96,7 @@ __device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[
 // 640x480x128, 5.8 TB/s; path by path from the stored states 6.4 ms).
 template <int PPL, int NW>
 __device__ __forceinline__ void adjoint_pair_block(const AdjArgs& a, int pair, int bx, unsigned char* ring) {
-    constexpr int SLICE_B = 128 * PPL, REC_B = PPL == 1 ? 16 : 8 * PPL;
+    constexpr int SLICE_B = 128 * PPL, REC_B = 4 * Route<PPL>::WORDS;
     constexpr int CHAIN_B = SLICE_B + REC_B, STAGE_B = 2 * CHAIN_B;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int W = a.W, H = a.H, D = a.D;
@@ -107,29 +106,26 @@ __device__ __forceinline__ void adjoint_pair_block(const AdjArgs& a, int pair, i
     if (c >= num_chains(dx, dy, W, H)) return;   // warp-uniform; no block barriers below
     const Chain ch = chain_start(c, dx, dy, W, H);
     const int n = ch.n;
-    const long step = (long)dy * W + dx;
-    const long pf0 = (long)ch.y * W + ch.x, pb0 = pf0 + (long)(n - 1) * step;
-    const long npix = (long)W * H;
-    [[maybe_unused]] const long long nvox = (long long)npix * D;
-    float* const out = a.out[pair];
-    const bool acc = a.acc[pair] != 0;
+    const int step = dy * W + dx;
+    const int pf0 = ch.y * W + ch.x, pb0 = pf0 + (n - 1) * step;
+    const int npix = W * H;
+    const long long nvox = (long long)npix * D;
+    float* const out = a.vol + ((a.slots >> (2 * pair)) & 3u) * (size_t)nvox + lane * PPL;
+    const bool acc = (a.acc >> pair) & 1u;
     unsigned char* const wbase = ring + (size_t)warp * PF * STAGE_B;
 
     // walker 0: path 2p's adjoint, pixel pb0 - k * step; walker 1: path 2p + 1's, pixel pf0 + k * step
-    auto pixel = [&](int walker, int k) { return walker ? pf0 + (long)k * step : pb0 - (long)k * step; };
+    auto pixel = [&](int walker, int k) { return walker ? pf0 + k * step : pb0 - k * step; };
+    auto record = [&](int walker, int pix) { return (unsigned)(2 * pair + walker) * (unsigned)npix + (unsigned)pix; };
     auto issue = [&](unsigned char* sb, int k) {
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
-            const long pix = pixel(v, k);
+            const int pix = pixel(v, k);
             if (!PM_IN_BOUNDS(pix, npix, kSiteDiffGrad)) continue;
             unsigned char* const s = sb + v * CHAIN_B;
-            cp_async_bytes<4 * PPL>(s + lane * 4 * PPL, a.gS + (size_t)pix * D + lane * PPL);
-            const uint32_t* rec = a.codes[2 * pair + v] + (size_t)pix * (2 * PPL);
-            if constexpr (PPL == 1) {
-                if (lane == 0) cp_async_8(s + SLICE_B, rec);
-            } else {
-                if (lane < PPL / 2) cp_async_16(s + SLICE_B + 16 * lane, rec + 4 * lane);
-            }
+            cp_async_bytes<4 * PPL>(s + lane * 4 * PPL, a.gS + lane * PPL + (size_t)(unsigned)pix * (unsigned)D);
+            if (lane < REC_B / 16)
+                cp_async_16(s + SLICE_B + 16 * lane, a.codes + (size_t)record(v, pix) * (REC_B / 4) + 4 * lane);
         }
     };
 #pragma unroll 1
@@ -137,55 +133,37 @@ __device__ __forceinline__ void adjoint_pair_block(const AdjArgs& a, int pair, i
         if (k < n) issue(wbase + k * STAGE_B, k);
         cp_async_commit();
     }
-    // plane indices of steps k0 + lane, a batch of 32 ahead (the last step routes nothing)
-    auto arg_at = [&](int walker, int k) {
-        const long pix = pixel(walker, k);
-        return k + 1 < n && PM_IN_BOUNDS(pix, npix, kSiteDiffRoute) ? (int)__ldg(a.arg[2 * pair + walker] + pix) : 0;
-    };
-    int arg0 = 0, arg1 = 0, next0 = arg_at(0, lane), next1 = arg_at(1, lane);
     float mu0[PPL], mu1[PPL];
 #pragma unroll
     for (int j = 0; j < PPL; ++j) mu0[j] = mu1[j] = 0.0f;
     int st = 0;
 
     auto body = [&](int k, float (&l0)[PPL], float (&l1)[PPL]) {
-        const int b = k & 31;
-        if (b == 0) {
-            arg0 = next0;
-            arg1 = next1;
-            next0 = arg_at(0, k + 32 + lane);
-            next1 = arg_at(1, k + 32 + lane);
-        }
         cp_async_wait<PF - 1>();
         __syncwarp();   // the records are copied by a few lanes and read by all
         unsigned char* const sb = wbase + st * STAGE_B;
         float g[PPL];
-        uint32_t w[2 * PPL];
+        uint32_t w[REC_B / 4];
         auto load = [&](const unsigned char* s) {
             load_planes<PPL>(g, reinterpret_cast<const float*>(s + lane * 4 * PPL));
-            if constexpr (PPL == 1) {
-                const uint2 t = *reinterpret_cast<const uint2*>(s + SLICE_B);
-                w[0] = t.x; w[1] = t.y;
-            } else {
 #pragma unroll
-                for (int i = 0; i < PPL / 2; ++i) {
-                    const uint4 t = *reinterpret_cast<const uint4*>(s + SLICE_B + 16 * i);
-                    w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
-                }
+            for (int i = 0; i < REC_B / 16; ++i) {
+                const uint4 t = *reinterpret_cast<const uint4*>(s + SLICE_B + 16 * i);
+                w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
             }
         };
         load(sb);
-        adjoint_step<PPL>(g, mu0, w, __shfl_sync(kFull, arg0, b), lane, l0);
+        adjoint_step<PPL>(g, mu0, w, lane, l0);
         load(sb + CHAIN_B);
-        adjoint_step<PPL>(g, mu1, w, __shfl_sync(kFull, arg1, b), lane, l1);
+        adjoint_step<PPL>(g, mu1, w, lane, l1);
         __syncwarp();   // every lane has read the stage that is refilled
         if (k + PF < n) issue(sb, k + PF);
         cp_async_commit();
         st = (st + 1 == PF) ? 0 : st + 1;
     };
-    auto put = [&](long pix, const float (&v)[PPL], bool add) {
-        float* const q = out + (size_t)pix * D + lane * PPL;
-        if (!PM_RANGE_IN_BOUNDS(q - out, PPL, nvox, kSiteDiffGrad)) return;
+    auto put = [&](int pix, const float (&v)[PPL], bool add) {
+        float* const q = out + (size_t)(unsigned)pix * (unsigned)D;
+        if (!PM_RANGE_IN_BOUNDS((long long)pix * D + lane * PPL, PPL, nvox, kSiteDiffGrad)) return;
         if (add) red_planes<PPL>(q, v);
         else store_planes<PPL>(q, v);
     };
@@ -194,7 +172,7 @@ __device__ __forceinline__ void adjoint_pair_block(const AdjArgs& a, int pair, i
     for (int k = 0; k < n; ++k) {
         float l0[PPL], l1[PPL];
         body(k, l0, l1);
-        const long p0 = pixel(0, k), p1 = pixel(1, k);
+        const int p0 = pixel(0, k), p1 = pixel(1, k);
         if (p0 == p1) {   // the middle of an odd scanline
             add_planes<PPL>(l0, l0, l1);
             put(p0, l0, acc);
@@ -214,19 +192,23 @@ __global__ void __launch_bounds__(32 * kPairWarps) diff_adj_kernel(const AdjArgs
     adjoint_pair_block<PPL, kPairWarps>(a, pair, bx, ring);
 }
 
-// a += b over n floats (n a multiple of 4)
-__global__ void __launch_bounds__(256) fold_kernel(float4* __restrict__ a, const float4* __restrict__ b, size_t n4) {
+// a = (a + b) + c over volumes of 4 * n4 floats
+__global__ void __launch_bounds__(256) fold_kernel(float4* __restrict__ a, const float4* __restrict__ b,
+                                                   const float4* __restrict__ c, size_t n4) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
         float4 x = a[i];
-        const float4 y = b[i];
-        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+        const float4 y = b[i], z = c[i];
+        x.x = (x.x + y.x) + z.x;
+        x.y = (x.y + y.y) + z.y;
+        x.z = (x.z + y.z) + z.z;
+        x.w = (x.w + y.w) + z.w;
         a[i] = x;
     }
 }
 
 // ---- soft-argmin --------------------------------------------------------------------------
 struct SoftArgs {
-    const float* vol[4];      // the pair volumes; their sum is the SGM sum
+    const float* vol;         // NV volumes, whose sum in their order is the SGM sum
     const float* rho_gt;
     const uint8_t* invalid;
     float* rho_hat;           // optional
@@ -236,37 +218,24 @@ struct SoftArgs {
     float rho0, drho, T;
 };
 
-// The sum of the pair volumes (in the product's order, (v0 + v1) + (v2 + v3), or with v2 + v3 folded into v2
-// beforehand), the soft-argmin over it, the loss's terms and its adjoint, one warp per pixel with the next
-// pixel's volumes in flight.  Bound by memory: NV reads and a write per voxel (0.17 ms at 640x480x128).  The loss is summed in double
+// The sum of the volumes, the soft-argmin over it, the loss's terms and its adjoint, one warp per pixel.  The
+// paths are added in their order, so that the loss's signs do not depend on the layout of the volumes.  Bound by
+// memory: NV reads and a write per voxel (0.17 ms at 640x480x128 with 4 volumes).  The loss is summed in double
 // precision per warp, block and grid.
 template <int PPL, int NV>
 __global__ void __launch_bounds__(256) soft_kernel(const SoftArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long nw = (long)gridDim.x * 8;
-    long p = (long)blockIdx.x * 8 + warp;
-    float next[NV][PPL];
-    auto load = [&](long pix) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-            if (PM_RANGE_IN_BOUNDS((long long)pix * a.D + lane * PPL, PPL, (long long)a.N * a.D, kSiteDiffGrad))
-                load_planes<PPL>(next[v], a.vol[v] + (size_t)pix * a.D + lane * PPL);
-    };
-    if (p < a.N) load(p);
     double loss = 0.0;
     int count = 0;
-    for (; p < a.N; p += nw) {
-        float s[PPL];
-        if constexpr (NV == 4) {
-            float t[PPL];
-            add_planes<PPL>(s, next[0], next[1]);
-            add_planes<PPL>(t, next[2], next[3]);
-            add_planes<PPL>(s, s, t);
-        } else {
-            add_planes<PPL>(s, next[0], next[1]);
-            add_planes<PPL>(s, s, next[2]);
-        }
-        if (p + nw < a.N) load(p + nw);
+    for (long p = (long)blockIdx.x * 8 + warp; p < a.N; p += nw) {
+        if (!PM_IN_BOUNDS(p, a.N, kSiteDiffGrad)) continue;
+        float v[NV][PPL], s[PPL];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) load_planes<PPL>(v[i], a.vol + ((size_t)i * a.N + p) * a.D + lane * PPL);
+        add_planes<PPL>(s, v[0], v[1]);
+#pragma unroll
+        for (int i = 2; i < NV; ++i) add_planes<PPL>(s, s, v[i]);
         float lmin = s[0];
 #pragma unroll
         for (int j = 1; j < PPL; ++j) lmin = fminf(lmin, s[j]);
@@ -293,8 +262,7 @@ __global__ void __launch_bounds__(256) soft_kernel(const SoftArgs a) {
         float o[PPL];
 #pragma unroll
         for (int j = 0; j < PPL; ++j) o[j] = k * w[j] * ((a.rho0 + (float)(lane * PPL + j) * a.drho) - rh);
-        if (PM_RANGE_IN_BOUNDS((long long)p * a.D + lane * PPL, PPL, (long long)a.N * a.D, kSiteDiffGrad))
-            store_planes<PPL>(a.gS + (size_t)p * a.D + lane * PPL, o);
+        store_planes<PPL>(a.gS + (size_t)p * a.D + lane * PPL, o);
     }
     __shared__ double sl[8];
     __shared__ int sc[8];
@@ -593,13 +561,13 @@ template <int PPL> cudaError_t launch_fwd_t(const SgmLaunch& a, const RouteOut& 
 }
 template <int PPL> cudaError_t launch_adj_t(const AdjArgs& a, unsigned mask, cudaStream_t s) {
     const PairSet ps = make_pair_set(mask, a.W, a.H, kPairWarps);
-    const size_t smem = (size_t)kPairWarps * PF * 2 * (128 * PPL + (PPL == 1 ? 16 : 8 * PPL));
+    const size_t smem = (size_t)kPairWarps * PF * 2 * (128 * PPL + 4 * Route<PPL>::WORDS);
     diff_adj_kernel<PPL><<<ps.start[ps.n], 32 * kPairWarps, smem, s>>>(a, ps);
     return cudaGetLastError();
 }
 template <int PPL> cudaError_t launch_soft_t(const SoftArgs& a, int nv, cudaStream_t s) {
     const int blocks = std::min((a.N + 7) / 8, 148 * 6);
-    if (nv == 4) soft_kernel<PPL, 4><<<blocks, 256, 0, s>>>(a);
+    if (nv == 7) soft_kernel<PPL, 7><<<blocks, 256, 0, s>>>(a);
     else soft_kernel<PPL, 3><<<blocks, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
@@ -632,9 +600,9 @@ struct pm_diff {
     float4* quads = nullptr;
     float* C = nullptr;       // costs; from the soft-argmin on, the adjoint of the SGM sum
     uint8_t* invalid = nullptr;
-    float* vol = nullptr;     // forward: pair volumes; backward: their adjoints (4 with store_paths, else 3)
-    uint32_t* codes = nullptr;   // 8 paths' records, N * D / 16 words each
-    uint8_t* arg = nullptr;   // 8 paths' plane indices, N each
+    bool wide = false;        // a volume for each term of the paths' sum (7) instead of 3
+    float* vol = nullptr;     // forward: the paths' values; backward: the pairs' adjoints
+    uint32_t* codes = nullptr;   // 8 paths' records, N each
     double* sums = nullptr;   // [loss sum, valid count]
     double* gP = nullptr;     // S x 6
     // inputs of the last forward
@@ -678,16 +646,8 @@ void free_diff(pm_diff* d) {
     cudaFree(d->invalid);
     cudaFree(d->vol);
     cudaFree(d->codes);
-    cudaFree(d->arg);
     cudaFree(d->sums);
     cudaFree(d->gP);
-}
-
-// Pair p's volume: one each with store_paths.  Else the two diagonal pairs' sum replaces the first one's volume,
-// and the vertical pair, which then runs by itself, takes the second one's; its adjoint is added to pair 0's.
-float* pair_volume(const pm_diff* d, int p) {
-    const int four[4] = {0, 1, 2, 3}, three[4] = {0, 2, 1, 2};
-    return d->vol + (size_t)(d->cfg.store_paths ? four : three)[p] * d->V;
 }
 
 }  // namespace
@@ -735,9 +695,13 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     alloc((void**)&d->quads, 16 * d->N * c->num_sources);
     alloc((void**)&d->C, 4 * d->V);
     alloc((void**)&d->invalid, d->N);
-    alloc((void**)&d->vol, 4 * d->V * (c->store_paths ? 4 : 3));
-    alloc((void**)&d->codes, 2 * d->V);
-    alloc((void**)&d->arg, 8 * d->N);
+    // store_paths, and volumes of up to 4 MB, whose steps are bound by the recurrences' latency: 7 volumes
+    // and all paths at once; else 3 and the pairs in three launches
+    d->wide = c->store_paths || d->V <= ((size_t)1 << 20);
+    alloc((void**)&d->vol, 4 * d->V * (d->wide ? 7 : 3));
+    const int ppl = c->num_planes / 32;
+    const size_t words = ppl == 1 ? Route<1>::WORDS : ppl == 2 ? Route<2>::WORDS : ppl == 4 ? Route<4>::WORDS : Route<8>::WORDS;
+    alloc((void**)&d->codes, 8 * d->N * 4 * words);
     alloc((void**)&d->sums, 2 * sizeof(double));
     alloc((void**)&d->gP, 6 * sizeof(double) * c->num_sources);
     if (!ok) {
@@ -820,29 +784,29 @@ pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const
     g0.D = D;
     g0.num_paths = 8;
     g0.p1 = c.p1; g0.p2 = c.p2; g0.tau = c.tau_so; g0.q1 = c.q1; g0.q2 = c.q2;
-    for (int p = 0; p < 4; ++p) g0.part[p] = pair_volume(d, p);
     RouteOut ro;
-    for (int r = 0; r < 8; ++r) {
-        ro.codes[r] = d->codes + (size_t)r * (d->V / 16);
-        ro.arg[r] = d->arg + (size_t)r * d->N;
-    }
+    ro.codes = d->codes;
     ro.invalid = d->invalid;
+    ro.vol = d->vol;
+    // S = ((((((L0 + L1) + L2) + L3) + L4) + L5) + L6) + L7: L0 and L1 meet in volume 0, the others have their own
+    if (d->wide) {
+        ro.slots = 0x65432100u;
+        PD_CK(d, launch_fwd(g0, ro, 0xfu, st));
+    } else {
+        ro.slots = 0x21212100u;
+        const unsigned pairs[3] = {0x3u, 0x4u, 0x8u};
+        for (int i = 0; i < 3; ++i) {
+            if (i) {
+                float4* const v = reinterpret_cast<float4*>(d->vol);
+                fold_kernel<<<148 * 8, 256, 0, st>>>(v, v + d->V / 4, v + d->V / 2, d->V / 4);
+                PD_CK(d, cudaGetLastError());
+            }
+            PD_CK(d, launch_fwd(g0, ro, pairs[i], st));
+        }
+    }
     SoftArgs sa;
     std::memset(&sa, 0, sizeof sa);
-    if (c.store_paths) {
-        PD_CK(d, launch_fwd(g0, ro, 0xfu, st));
-        for (int p = 0; p < 4; ++p) sa.vol[p] = pair_volume(d, p);
-    } else {
-        PD_CK(d, launch_fwd(g0, ro, 0xdu, st));
-        float* const v2 = pair_volume(d, 2);
-        fold_kernel<<<148 * 8, 256, 0, st>>>(reinterpret_cast<float4*>(v2), reinterpret_cast<const float4*>(pair_volume(d, 3)),
-                                             d->V / 4);
-        PD_CK(d, cudaGetLastError());
-        PD_CK(d, launch_fwd(g0, ro, 0x2u, st));
-        sa.vol[0] = pair_volume(d, 0);
-        sa.vol[1] = pair_volume(d, 1);
-        sa.vol[2] = v2;
-    }
+    sa.vol = d->vol;
     PD_CK(d, cudaMemsetAsync(d->sums, 0, 2 * sizeof(double), st));
     sa.rho_gt = rho_gt;
     sa.invalid = d->invalid;
@@ -854,7 +818,7 @@ pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const
     sa.rho0 = c.rho0;
     sa.drho = c.rho_step;
     sa.T = c.temperature;
-    PD_CK(d, launch_soft(sa, c.store_paths ? 4 : 3, st));
+    PD_CK(d, launch_soft(sa, d->wide ? 7 : 3, st));
     double h[2];
     PD_CK(d, cudaMemcpyAsync(h, d->sums, sizeof h, cudaMemcpyDeviceToHost, st));
     PD_CK(d, cudaStreamSynchronize(st));
@@ -873,21 +837,18 @@ pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void
     AdjArgs aa;
     std::memset(&aa, 0, sizeof aa);
     aa.gS = d->C;
-    for (int r = 0; r < 8; ++r) {
-        aa.codes[r] = d->codes + (size_t)r * (d->V / 16);
-        aa.arg[r] = d->arg + (size_t)r * d->N;
-    }
+    aa.codes = d->codes;
     aa.W = c.width;
     aa.H = c.height;
     aa.D = D;
-    const int nv = c.store_paths ? 4 : 3;
-    const int slot[4] = {0, c.store_paths ? 1 : 0, c.store_paths ? 2 : 1, c.store_paths ? 3 : 2};
-    for (int p = 0; p < 4; ++p) aa.out[p] = d->vol + (size_t)slot[p] * d->V;
-    if (c.store_paths) {
+    const int nv = d->wide ? 4 : 3;
+    aa.vol = d->vol;
+    aa.slots = d->wide ? 0u | 1u << 2 | 2u << 4 | 3u << 6 : 0u | 0u << 2 | 1u << 4 | 2u << 6;
+    if (d->wide) {
         PD_CK(d, launch_adj(aa, 0xfu, st));
     } else {
         PD_CK(d, launch_adj(aa, 0xdu, st));
-        aa.acc[1] = 1;
+        aa.acc = 0x2u;
         PD_CK(d, launch_adj(aa, 0x2u, st));
     }
     PD_CK(d, cudaMemsetAsync(grad_srcs, 0, 4 * d->N * S, st));

@@ -348,29 +348,30 @@ __device__ __forceinline__ void path_first(PathState<PPL>& s, const float (&cv)[
     s.mprev = warp_min_f32(lane_min<PPL, FULL>(s.L, incl));
 }
 
-// The differentiation form's record of one step: which term of the minimum each plane took, as two
-// ballots per plane of a lane (bit l of word 2j / 2j + 1: bit 0 / 1 of plane l * PPL + j's code, see
-// RouteCode), and the lowest plane that holds the predecessor's minimum.
-enum RouteCode { kRouteSame = 0, kRouteLower = 1, kRouteUpper = 2, kRouteMin = 3 };
+// The differentiation form's record of one step: which term of the minimum each plane took, as three
+// ballots per plane j of a lane (word 3j: the same plane's; 3j + 1: a neighbour's; 3j + 2: the lower
+// neighbour is not above the upper one; earlier words take precedence), and the lowest plane that
+// holds the predecessor's minimum (word 3 * PPL).  Plain comparisons: two bits per plane would hold
+// the choice, but their encoding takes more instructions than the third ballot.
 template <int PPL> struct Route {
-    uint32_t w[2 * PPL];
-    int arg;
+    static constexpr int WORDS = (3 * PPL + 1 + 3) / 4 * 4;   // whole 16-byte pieces
+    uint32_t w[WORDS];
     bool inv;   // the pixel has a plane that was never measured
 };
-// Where a pass with records puts them, per path: N records of 2 * PPL words and N plane indices; and
-// the invalid flag of every pixel (written by pair 0).
+// Where a pass with records puts them: path r's record of a pixel is record r * N + pixel; and the invalid
+// flag of every pixel (written by pair 0).  8 * N < 2^32.  Path r's values go to volume
+// (slots >> 4 * r) & 15 of vol: the two paths of a pair meet in one volume, as in the product, or have
+// one each.
 struct RouteOut {
-    uint32_t* codes[8];
-    uint8_t* arg[8];
+    uint32_t* codes;
     uint8_t* invalid;
+    float* vol;
+    unsigned slots;
 };
 template <int PPL> __device__ __forceinline__ void store_route(uint32_t* p, const Route<PPL>& r) {
-    if constexpr (PPL == 1) *reinterpret_cast<uint2*>(p) = make_uint2(r.w[0], r.w[1]);
-    else {
 #pragma unroll
-        for (int i = 0; i < 2 * PPL; i += 4)
-            *reinterpret_cast<uint4*>(p + i) = make_uint4(r.w[i], r.w[i + 1], r.w[i + 2], r.w[i + 3]);
-    }
+    for (int i = 0; i < Route<PPL>::WORDS; i += 4)
+        *reinterpret_cast<uint4*>(p + i) = make_uint4(r.w[i], r.w[i + 1], r.w[i + 2], r.w[i + 3]);
 }
 
 // One pixel step of a path (sgm.cu:57-108): L(p, d) = C(p, d) + min(L(p-r, d), L(p-r, d+-1) + P1,
@@ -402,17 +403,17 @@ __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s,
 #pragma unroll
     for (int j = 0; j < PPL; ++j) vv[j] = min3f(s.L[j], mP2, nb[j]);
     if constexpr (ROUTE) {
-        int at = PPL;
+        unsigned at = ~0u;
 #pragma unroll
         for (int j = PPL - 1; j >= 0; --j) {
-            const bool lower = (j == 0 ? lm : s.L[j - 1]) <= (j == PPL - 1 ? lp : s.L[j + 1]);
-            const bool same = s.L[j] == vv[j], side = nb[j] == vv[j];
-            rt->w[2 * j] = __ballot_sync(kFull, !same && (!side || lower));
-            rt->w[2 * j + 1] = __ballot_sync(kFull, !same && (!side || !lower));
-            at = s.L[j] == s.mprev ? j : at;
+            rt->w[3 * j] = __ballot_sync(kFull, s.L[j] == vv[j]);
+            rt->w[3 * j + 1] = __ballot_sync(kFull, nb[j] == vv[j]);
+            rt->w[3 * j + 2] = __ballot_sync(kFull, (j == 0 ? lm : s.L[j - 1]) <= (j == PPL - 1 ? lp : s.L[j + 1]));
+            at = s.L[j] == s.mprev ? (unsigned)(lane * PPL + j) : at;
         }
-        const int src = __ffs(__ballot_sync(kFull, at < PPL)) - 1;
-        rt->arg = PPL == 1 ? src : src * PPL + __shfl_sync(kFull, at, src);
+        rt->w[3 * PPL] = __reduce_min_sync(kFull, at);
+#pragma unroll
+        for (int i = 3 * PPL + 1; i < Route<PPL>::WORDS; ++i) rt->w[i] = 0u;
         rt->inv = inv;
     }
     add_planes<PPL>(vv, cz, vv);               // C + val
@@ -423,17 +424,15 @@ __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s,
 }
 
 // Reference intensity of step k of a chain starting at pixel p0 (0 past its end).
-__device__ __forceinline__ float chain_ref(const float* __restrict__ ref, long p0, long step, int k, int n,
-                                           long npix) {
-    return k < n && PM_IN_BOUNDS(p0 + (long)k * step, npix, kSitePairRef) ? __ldg(ref + p0 + (long)k * step) : 0.0f;
+__device__ __forceinline__ float chain_ref(const float* __restrict__ ref, int p0, int step, int k, int n, int npix) {
+    return k < n && PM_IN_BOUNDS(p0 + k * step, npix, kSitePairRef) ? __ldg(ref + (unsigned)(p0 + k * step)) : 0.0f;
 }
 
 // The flags |I(k) - I(k-1)| < tau of the 32 steps k0 .. k0+31 of one chain as a ballot (bit i:
 // step k0 + i).  Lane i holds I(k0 + i) in `cur` (read one batch ahead into `nxt`, which is
 // then refilled with I(k0 + 64 + i)); `last` carries I(k0 - 1).
-__device__ __forceinline__ unsigned penalty_flags(float& cur, float& nxt, const float* __restrict__ ref, long p0,
-                                                  long step, int k0, int n, int lane, float tau, float& last,
-                                                  long npix) {
+__device__ __forceinline__ unsigned penalty_flags(float& cur, float& nxt, const float* __restrict__ ref, int p0,
+                                                  int step, int k0, int n, int lane, float tau, float& last, int npix) {
     const float I = cur;
     cur = nxt;
     nxt = chain_ref(ref, p0, step, k0 + 64 + lane, n, npix);
@@ -467,26 +466,41 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
     if (c >= num_chains(dx, dy, W, H)) return;        // warp-uniform; no block barriers below
     const Chain ch = chain_start(c, dx, dy, W, H);
     const int n = ch.n;
-    const long step = (long)dy * W + dx;
-    const long pf0 = (long)ch.y * W + ch.x;             // forward start
-    const long pb0 = pf0 + (long)(n - 1) * step;        // backward start (the forward end)
-    const long gstep = step * D;                         // elements per step in the volumes
+    // pixel indices (W * H < 2^31), and running addresses of the slices read and written.  ROUTE: the
+    // addresses are formed from the pixels, which takes an instruction more per slice and leaves the
+    // registers that the records need.
+    const int step = dy * W + dx;
+    const int pf0 = ch.y * W + ch.x;                    // forward start
+    const int pb0 = pf0 + (n - 1) * step;               // backward start (the forward end)
+    int pf = pf0, pb = pb0;                             // the current step's pixels
 
     unsigned char* const wbase = ring + (size_t)warp * PF * STAGE_B;
-    const CT* const cf0 = reinterpret_cast<const CT*>(a.cost) + (size_t)pf0 * D + lane * PPL;
-    const CT* const cb0 = reinterpret_cast<const CT*>(a.cost) + (size_t)pb0 * D + lane * PPL;
-    OT* const out = static_cast<OT*>(a.part[slot >> 1]);
-    OT* qf = out + (size_t)pf0 * D + lane * PPL;        // the current step's output slices
-    OT* qb = out + (size_t)pb0 * D + lane * PPL;
-    const long npix = (long)W * H;
+    const CT* const cost = reinterpret_cast<const CT*>(a.cost) + lane * PPL;
+    OT* out = static_cast<OT*>(a.part[slot >> 1]) + lane * PPL;
+    [[maybe_unused]] OT* out2 = out;   // ROUTE: the second path's volume
+    if constexpr (ROUTE) {
+        const size_t nv = (size_t)W * H * D;
+        out = reinterpret_cast<OT*>(ro->vol) + ((ro->slots >> (4 * slot)) & 15u) * nv + lane * PPL;
+        out2 = reinterpret_cast<OT*>(ro->vol) + ((ro->slots >> (4 * slot + 4)) & 15u) * nv + lane * PPL;
+    }
+    const bool one = !ROUTE || out == out2;
+    auto at = [&](int pix) { return (size_t)(unsigned)pix * (unsigned)D; };
+    const long gstep = (long)step * D;
+    [[maybe_unused]] const CT* const cf0 = cost + at(pf0);
+    [[maybe_unused]] const CT* const cb0 = cost + at(pb0);
+    OT* qf = ROUTE ? out : out + at(pf0);
+    OT* qb = ROUTE ? out2 : out + at(pb0);
+    const int npix = W * H;
     [[maybe_unused]] const long long nvox = (long long)npix * D;
-    auto put = [&](OT* q, const float (&v)[PPL]) {
-        if (!PM_RANGE_IN_BOUNDS(q - out, PPL, nvox, kSitePairOut)) return;
+    auto put = [&](int pix, OT* run, const float (&v)[PPL]) {   // run: the address, or ROUTE: the volume
+        OT* const q = ROUTE ? run + at(pix) : run;
+        if (!PM_RANGE_IN_BOUNDS((long long)pix * D + lane * PPL, PPL, nvox, kSitePairOut)) return;
         if constexpr (HOUT) store_planes_h<PPL>(q, v);
         else store_planes<PPL>(q, v);
     };
-    auto add = [&](OT* q, const float (&v)[PPL]) {
-        if (!PM_RANGE_IN_BOUNDS(q - out, PPL, nvox, kSitePairOut)) return;
+    auto add = [&](int pix, OT* run, const float (&v)[PPL]) {
+        OT* const q = ROUTE ? run + at(pix) : run;
+        if (!PM_RANGE_IN_BOUNDS((long long)pix * D + lane * PPL, PPL, nvox, kSitePairOut)) return;
         if constexpr (HOUT) red_planes_h<PPL>(q, v);
         else red_planes<PPL>(q, v);
     };
@@ -499,12 +513,12 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         }
     };
 
-    auto issue = [&](unsigned char* sb, int k) {
-        [[maybe_unused]] const CT* const base = reinterpret_cast<const CT*>(a.cost);
-        if (PM_RANGE_IN_BOUNDS(cf0 + (long)k * gstep - base, PPL, nvox, kSitePairLoad))
-            cp_async_bytes<CB>(sb + lane * CB, cf0 + (long)k * gstep);
-        if (PM_RANGE_IN_BOUNDS(cb0 - (long)k * gstep - base, PPL, nvox, kSitePairLoad))
-            cp_async_bytes<CB>(sb + CHAIN_B + lane * CB, cb0 - (long)k * gstep);
+    auto issue = [&](unsigned char* sb, int k) {   // the slices of step k's two pixels
+        [[maybe_unused]] const int f = pf0 + k * step, b = pb0 - k * step;
+        if (PM_RANGE_IN_BOUNDS((long long)f * D + lane * PPL, PPL, nvox, kSitePairLoad))
+            cp_async_bytes<CB>(sb + lane * CB, ROUTE ? cost + at(f) : cf0 + (long)k * gstep);
+        if (PM_RANGE_IN_BOUNDS((long long)b * D + lane * PPL, PPL, nvox, kSitePairLoad))
+            cp_async_bytes<CB>(sb + CHAIN_B + lane * CB, ROUTE ? cost + at(b) : cb0 - (long)k * gstep);
     };
 #pragma unroll 1
     for (int k = 0; k < PF; ++k) {
@@ -523,19 +537,15 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
     fs.qmask = penalty_flags(If, Ifn, a.ref, pf0, step, 0, n, lane, a.tau, lastf, npix);
     bs.qmask = penalty_flags(Ib, Ibn, a.ref, pb0, -step, 0, n, lane, a.tau, lastb, npix);
 
-    // ROUTE: the plane indices and invalid flags of the current batch of 32 steps, stored together
-    [[maybe_unused]] int argf = 0, argb = 0;
+    // ROUTE: the invalid flags of the current batch of 32 steps, stored together
     [[maybe_unused]] unsigned rinv = 0;
-    [[maybe_unused]] auto flush_route = [&](int k) {
-        const int kk = (k & ~31) + lane;
-        if (kk > k) return;
-        const long pf = pf0 + (long)kk * step, pb = pb0 - (long)kk * step;
-        if (!PM_IN_BOUNDS(pf, npix, kSiteDiffRoute) || !PM_IN_BOUNDS(pb, npix, kSiteDiffRoute)) return;
-        if (kk > 0) {
-            ro->arg[slot][pf] = (uint8_t)argf;
-            ro->arg[slot + 1][pb] = (uint8_t)argb;
-        }
-        if (slot == 0) ro->invalid[pf] = (uint8_t)((rinv >> lane) & 1u);
+    [[maybe_unused]] auto flush_invalid = [&](int k) {
+        const int kk = (k & ~31) + lane, f = pf - (k - kk) * step;
+        if (kk <= k && PM_IN_BOUNDS(f, npix, kSiteDiffRoute)) ro->invalid[f] = (uint8_t)((rinv >> lane) & 1u);
+    };
+    [[maybe_unused]] auto put_route = [&](int path, int pix, const Route<PPL>& r) {
+        if (lane == 0 && PM_IN_BOUNDS(pix, npix, kSiteDiffRoute))
+            store_route<PPL>(ro->codes + (size_t)((unsigned)path * (unsigned)npix + (unsigned)pix) * Route<PPL>::WORDS, r);
     };
 
     // step 0: the first pixel of both paths
@@ -548,14 +558,14 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         path_first<PPL, FULL>(fs, cf, incl, of);
         path_first<PPL, FULL>(bs, cb, incl, ob);
         if constexpr (ROUTE) {
-            if (n == 1) flush_route(0);
+            if (n == 1 && slot == 0) flush_invalid(0);
         }
-        if (n == 1) {
+        if (n == 1 && one) {
             meet(of, ob);
-            put(qf, of);
+            put(pf, qf, of);
         } else {
-            put(qf, of);
-            put(qb, ob);
+            put(pf, qf, of);
+            put(pb, qb, ob);
         }
         if (PF < n) issue(wbase, PF);
         cp_async_commit();
@@ -565,8 +575,12 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
     // steps 1 .. n-1: the first visits (stores), the meeting pixel of an odd chain, then the
     // second visits (reductions)
     auto body = [&](int k, float (&of)[PPL], float (&ob)[PPL]) {
-        qf += gstep;
-        qb -= gstep;
+        pf += step;
+        pb -= step;
+        if constexpr (!ROUTE) {
+            qf += gstep;
+            qb -= gstep;
+        }
         if ((k & 31) == 0) {
             fs.qmask = penalty_flags(If, Ifn, a.ref, pf0, step, k, n, lane, a.tau, lastf, npix);
             bs.qmask = penalty_flags(Ib, Ibn, a.ref, pb0, -step, k, n, lane, a.tau, lastb, npix);
@@ -580,14 +594,13 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         if constexpr (ROUTE) {
             Route<PPL> r;
             path_step<PPL, FULL, true>(a, fs, cf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of, &r);
-            const long pf = pf0 + (long)k * step, pb = pb0 - (long)k * step;
-            if (lane == 0 && PM_IN_BOUNDS(pf, npix, kSiteDiffRoute)) store_route<PPL>(ro->codes[slot] + pf * (2 * PPL), r);
-            argf = lane == bit ? r.arg : argf;
-            rinv = (bit == 0 ? 0u : rinv) | (r.inv ? 1u << bit : 0u);
+            put_route(slot, pf, r);
+            if (slot == 0) {
+                rinv = (bit == 0 ? 0u : rinv) | (r.inv ? 1u << bit : 0u);
+                if (bit == 31 || k == n - 1) flush_invalid(k);
+            }
             path_step<PPL, FULL, true>(a, bs, cb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob, &r);
-            if (lane == 0 && PM_IN_BOUNDS(pb, npix, kSiteDiffRoute)) store_route<PPL>(ro->codes[slot + 1] + pb * (2 * PPL), r);
-            argb = lane == bit ? r.arg : argb;
-            if (bit == 31 || k == n - 1) flush_route(k);
+            put_route(slot + 1, pb, r);
         } else {
             path_step<PPL, FULL>(a, fs, cf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of);
             path_step<PPL, FULL>(a, bs, cb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob);
@@ -602,23 +615,28 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
     for (int k = 1; k < half; ++k) {
         float of[PPL], ob[PPL];
         body(k, of, ob);
-        put(qf, of);
-        put(qb, ob);
+        put(pf, qf, of);
+        put(pb, qb, ob);
     }
     int k = half > 1 ? half : 1;
-    if ((n & 1) && n > 1) {   // both ends on the middle pixel (k == half)
+    if ((n & 1) && n > 1 && one) {   // both ends on the middle pixel (k == half)
         float of[PPL], ob[PPL];
         body(k, of, ob);
         meet(of, ob);
-        put(qf, of);
+        put(pf, qf, of);
         ++k;
     }
 #pragma unroll 1
     for (; k < n; ++k) {   // second visits: the first ones were this warp's own stores
         float of[PPL], ob[PPL];
         body(k, of, ob);
-        add(qf, of);
-        add(qb, ob);
+        if (one) {
+            add(pf, qf, of);
+            add(pb, qb, ob);
+        } else {
+            put(pf, qf, of);
+            put(pb, qb, ob);
+        }
     }
     cp_async_wait<0>();
 }
