@@ -37,10 +37,10 @@ __device__ inline float warp_sum(float v) {
 // routes by: 3 to 4 bits per voxel and path, where the path states themselves would take 32.  Bound by memory like the product's: two reads of the costs, a store and a
 // reduction per pair, 20 bytes per voxel and pair, and 0.5 for the records.  All eight paths at 640x480x128:
 // 0.94 ms (one path after the other, each adding to the sum and storing its states: 5.0 ms).
-constexpr int kPairWarps = 2;   // scanlines per block: small blocks spread an image's scanlines over the SMs
+constexpr int kPairWarps = 1;   // scanlines per block: small blocks spread an image's scanlines over the SMs
 
 template <int PPL>
-__global__ void __launch_bounds__(32 * kPairWarps, PPL <= 4 ? 12 : 1) diff_fwd_kernel(const SgmLaunch a, const RouteOut ro, const PairSet ps) {
+__global__ void __launch_bounds__(32 * kPairWarps, PPL <= 4 ? 23 : 1) diff_fwd_kernel(const SgmLaunch a, const RouteOut ro, const PairSet ps) {
     extern __shared__ __align__(16) unsigned char ring[];
     int bx = blockIdx.x, dx, dy;
     const int pair = pair_of_block(ps, bx);

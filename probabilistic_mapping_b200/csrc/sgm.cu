@@ -20,7 +20,7 @@
 //     first stores its values there and the other adds its own with a vector reduction, so the
 //     volume ends up holding P_2p + P_2p+1 (float addition is commutative, so this is the same
 //     sum in either order);
-//   * a pixel-parallel combine kernel (one warp per pixel, full occupancy) adds the pair volumes,
+//   * a pixel-parallel combine kernel (four pixels per warp, full occupancy) adds the pair volumes,
 //     (P0 + P1) + (P2 + P3) [+ ((P4 + P5) + (P6 + P7))], in registers and runs the
 //     winner-take-all directly, so the complete sum need not be written.  The FP32 result
 //     therefore differs from the reference's sequential path order only by rounding; the CPU
@@ -30,6 +30,7 @@
 //     are rounded to FP16, the second end adds with packed FP16 reductions, and the combine adds
 //     the pairs in FP32.  That halves the bytes of the pair volumes, which with FP32 pairs were
 //     60 % of the stage's traffic; the FP16 form is held to its FP64 accuracy bound, not to bits.
+#include <cstring>
 #include <vector>
 
 #include "sgm_device.cuh"
@@ -73,18 +74,28 @@ __global__ void __launch_bounds__(NW * 32) sgm_pair_kernel(const SgmLaunch a, in
     sgm_pair_block<PPL, HALF, NW, FULL, HOUT>(a, dx, dy, slot, blockIdx.x, ring);
 }
 
-// Blocks per SM that the combine kernel is held to (0: no bound): D = 192 in FP32, D = 256 in FP16
-// with four paths and D = 128 in FP16 with eight, where the compiler's default register choice
-// leaves one block per SM fewer.
-constexpr int combine_min_blocks(int ppl, int np, bool hin) {
-    return ppl == 6 && !hin ? (np == 2 ? 4 : 3) : ppl == 8 && hin && np == 2 ? 3 : ppl == 4 && hin && np == 4 ? 4 : 0;
-}
+// Blocks per SM that the one-pixel combine kernel is held to (0: no bound): D = 192 in FP32, where the
+// compiler's default register choice leaves one block per SM fewer.
+constexpr int combine_min_blocks(int ppl, int np) { return ppl == 6 ? (np == 2 ? 4 : 3) : 0; }
 
 // grid-stride over the image's pixels, one warp per pixel
 template <int PPL, int MODE, int NP, bool HIN>
-__global__ void __launch_bounds__(256, combine_min_blocks(PPL, NP, HIN)) combine_kernel(const SgmLaunch a) {
+__global__ void __launch_bounds__(256, combine_min_blocks(PPL, NP)) combine_kernel(const SgmLaunch a) {
     combine_pixels<PPL, MODE, NP, HIN, false>(a, (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5),
                                               (long)gridDim.x * (blockDim.x >> 5), (long)a.W * a.H);
+}
+
+// grid-stride over groups of four pixels, one warp per group
+constexpr int kGroupWarps = 8;
+template <int NCH, int MODE, int NP, bool HIN, bool FULL>
+__global__ void __launch_bounds__(32 * kGroupWarps) combine_group_kernel(const SgmLaunch a) {
+    __shared__ GroupSmem<NCH, kGroupWarps> sm;
+    const void* vol[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) vol[p] = a.part[p];
+    const long ngroups = ((long)a.W * a.H + GP - 1) / GP;
+    combine_groups<NCH, MODE, NP, HIN, FULL, kGroupWarps>(a, vol, sm, (long)blockIdx.x * kGroupWarps + (threadIdx.x >> 5),
+                                                          (long)gridDim.x * kGroupWarps, ngroups);
 }
 
 // pm_stats: the histogram of a per-pixel class array (classes below n <= 8), one ballot per class
@@ -177,12 +188,17 @@ cudaError_t launch_with_priority(void (*kern)(Args...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// every plane takes part in the minima (D a power of two, or the exact minimum)
+bool all_planes(const PlaneOrder& o, int ppl) {
+    for (int l = 0; l < 32; ++l)
+        if (o.incl[l] != (1u << ppl) - 1u) return false;
+    return true;
+}
+
 template <int PPL, bool HALF, int NW>
 cudaError_t launch_pair_nw(const SgmLaunch& a, int pair, cudaStream_t s) {
     const size_t smem = (size_t)NW * PF * Ring<PPL, HALF>::STAGE_B;
-    // every plane takes part in the minima (D a power of two, or the exact minimum): no masks
-    bool full = true;
-    for (int l = 0; l < 32; ++l) full = full && a.order.incl[l] == (1u << PPL) - 1u;
+    const bool full = all_planes(a.order, PPL);
     void (*kern)(SgmLaunch, int, int, int);
     if constexpr (HALF && PPL % 2 == 0) {
         if (a.part_half) kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, true> : sgm_pair_kernel<PPL, HALF, NW, false, true>;
@@ -214,35 +230,58 @@ cudaError_t launch_pair(const SgmLaunch& a, int pair, cudaStream_t s) {
     }
 }
 
-template <int PPL>
-cudaError_t launch_combine(const SgmLaunch& a, int mode, cudaStream_t s) {
+int sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long npix = (long)a.W * a.H;
-    const long blocks_needed = (npix + 7) / 8;   // 8 warps per block
-    const int blocks = (int)(blocks_needed < (long)sms * 8 ? blocks_needed : (long)sms * 8);
+    return sms;
+}
+
+// The four-pixel kernel over np pair volumes a.part[0 .. np) (np = 1: one volume, the sum).
+template <int PPL, int NP, bool HIN>
+cudaError_t launch_groups_t(const SgmLaunch& a, int mode, cudaStream_t s) {
+    const long groups = ((long)a.W * a.H + GP - 1) / GP, need = (groups + kGroupWarps - 1) / kGroupWarps;
+    const long most = (long)sm_count() * 8;
+    void (*kern)(SgmLaunch);
+    if (mode == kCombineArgmin) kern = combine_group_kernel<PPL, kCombineArgmin, NP, HIN, true>;
+    else if (all_planes(a.order, PPL)) kern = combine_group_kernel<PPL, kCombineFilter, NP, HIN, true>;
+    else kern = combine_group_kernel<PPL, kCombineFilter, NP, HIN, false>;
+    return launch_with_priority(kern, dim3((unsigned)(need < most ? need : most)), dim3(32 * kGroupWarps), 0, s, a.priority, a);
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Filter and debug argmin take four pixels per warp (combine_group_kernel), at 640x480, FP32 / FP16 pairs, us:
+//   D = 64, 4 paths 64 -> 35 (8 paths FP16 50 -> 34), D = 128, 8 paths 109 -> 107 (FP16 73 -> 65), D = 192, 8 paths
+//   156 -> 154 (FP16 123 -> 93);
+// one pixel per warp remains where it is as fast or the only one that can: 256 planes and 8 paths in FP32, whose loads
+// fill a warp (193 against 210 us); volumes that are not 16-byte aligned (a caller's); FP32 pair volumes of an FP16
+// cost volume, with its offsets; and the store of the sum alone, which is bound by memory in either form.
+template <int PPL>
+cudaError_t launch_combine(const SgmLaunch& a, int mode, cudaStream_t s) {
     const bool eight = a.num_paths == 8;
-    void (*kern)(SgmLaunch) = nullptr;
-    if (a.part_half) {
+    if (a.part_half) {   // volumes of this library, 256-byte aligned
         if constexpr (PPL % 2 == 0) {
-            if (mode == kCombineFilter)
-                kern = eight ? combine_kernel<PPL, kCombineFilter, 4, true> : combine_kernel<PPL, kCombineFilter, 2, true>;
-            else if (mode == kCombineArgmin)
-                kern = eight ? combine_kernel<PPL, kCombineArgmin, 4, true> : combine_kernel<PPL, kCombineArgmin, 2, true>;
-            else
-                kern = eight ? combine_kernel<PPL, kCombineStore, 4, true> : combine_kernel<PPL, kCombineStore, 2, true>;
-        } else {
-            return cudaErrorInvalidValue;
+            if (mode != kCombineStore)
+                return eight ? launch_groups_t<PPL, 4, true>(a, mode, s) : launch_groups_t<PPL, 2, true>(a, mode, s);
         }
-    } else if (mode == kCombineFilter) {
-        kern = eight ? combine_kernel<PPL, kCombineFilter, 4, false> : combine_kernel<PPL, kCombineFilter, 2, false>;
-    } else if (mode == kCombineArgmin) {
-        kern = eight ? combine_kernel<PPL, kCombineArgmin, 4, false> : combine_kernel<PPL, kCombineArgmin, 2, false>;
-    } else {
-        kern = eight ? combine_kernel<PPL, kCombineStore, 4, false> : combine_kernel<PPL, kCombineStore, 2, false>;
+        return cudaErrorInvalidValue;
     }
-    return launch_with_priority(kern, dim3(blocks), dim3(256), 0, s, a.priority, a);
+    bool group = mode != kCombineStore && !a.offset && (!a.total || aligned16(a.total));
+    for (int p = 0; p < a.num_paths / 2; ++p) group = group && aligned16(a.part[p]);
+    if (group && !(PPL == 8 && eight && mode == kCombineFilter))
+        return eight ? launch_groups_t<PPL, 4, false>(a, mode, s) : launch_groups_t<PPL, 2, false>(a, mode, s);
+    const long npix = (long)a.W * a.H;
+    const long blocks_needed = (npix + 7) / 8, most = (long)sm_count() * 8;   // 8 warps per block
+    void (*kern)(SgmLaunch);
+    if (mode == kCombineFilter)
+        kern = eight ? combine_kernel<PPL, kCombineFilter, 4, false> : combine_kernel<PPL, kCombineFilter, 2, false>;
+    else if (mode == kCombineArgmin)
+        kern = eight ? combine_kernel<PPL, kCombineArgmin, 4, false> : combine_kernel<PPL, kCombineArgmin, 2, false>;
+    else
+        kern = eight ? combine_kernel<PPL, kCombineStore, 4, false> : combine_kernel<PPL, kCombineStore, 2, false>;
+    return launch_with_priority(kern, dim3((unsigned)(blocks_needed < most ? blocks_needed : most)), dim3(256), 0, s,
+                                a.priority, a);
 }
 
 // Path pairs p = 0 .. num_paths/2 - 1: pairs 0..np-2 run on their own side streams when `side`
@@ -275,6 +314,20 @@ cudaError_t launch_filter_t(const float* sum, int W, int H, int D, const FilterP
                             const PlaneOrder& order, float* depth, size_t pitch, int32_t* index,
                             cudaStream_t s) {
     const long n = (long)W * H;
+    if (aligned16(sum)) {   // 640x480x64: 190 -> 24 us, 128 planes 191 -> 33 (24 at the copy rate)
+        SgmLaunch a;
+        std::memset(&a, 0, sizeof a);
+        a.part[0] = const_cast<float*>(sum);
+        a.W = W;
+        a.H = H;
+        a.D = D;
+        a.fp = fp;
+        a.order = order;
+        a.depth = depth;
+        a.depth_pitch = pitch;
+        a.index = index;
+        return launch_groups_t<PPL, 1, false>(a, kCombineFilter, s);
+    }
     filter_kernel<PPL><<<(unsigned)((n + 3) / 4), 128, 0, s>>>(sum, W, H, D, fp, order, depth, pitch, index);
     return cudaGetLastError();
 }
@@ -322,6 +375,20 @@ template <int PPL, bool HALF>
 cudaError_t launch_case_t(const void* vol, const float* offset, int W, int H, int D, const FilterParams& fp,
                           float* depth, size_t pitch, int32_t* index, cudaStream_t s) {
     const long n = (long)W * H;
+    if (aligned16(vol)) {
+        SgmLaunch a;
+        std::memset(&a, 0, sizeof a);
+        a.part[0] = const_cast<void*>(vol);
+        a.W = W;
+        a.H = H;
+        a.D = D;
+        a.fp = fp;
+        a.offset = offset;
+        a.depth = depth;
+        a.depth_pitch = pitch;
+        a.index = index;
+        if constexpr (!HALF || PPL % 2 == 0) return launch_groups_t<PPL, 1, HALF>(a, kCombineArgmin, s);
+    }
     case_kernel<PPL, HALF><<<(unsigned)((n + 3) / 4), 128, 0, s>>>(vol, offset, W, H, D, fp, depth, pitch, index);
     return cudaGetLastError();
 }

@@ -779,5 +779,193 @@ __device__ __forceinline__ void combine_pixels(const SgmLaunch& a, long first, l
     }
 }
 
+// ---- four pixels per warp ----------------------------------------------------------------
+// The same sum and winner-take-all with eight lanes per pixel: lane g of a pixel's eight holds planes
+// 32 c + 4 g .. 4 g + 3 of every 32-plane chunk c (FP16 volumes: 64 c + 8 g .. 8 g + 7), so a chunk of
+// a pixel is one contiguous 128-byte run of 16-byte loads.  One warp per pixel spends about a hundred
+// instructions per pixel on the reductions, the tests and the parabola, whatever the number of planes;
+// here a warp spends them on four pixels.  The values of the planes beside the minimum go through
+// shared memory.  Needs 16-byte aligned volumes.
+constexpr int GP = 4;        // pixels per warp
+constexpr int GL = 32 / GP;  // lanes per pixel
+
+__device__ __forceinline__ float group_min(float v) {
+#pragma unroll
+    for (int o = 1; o < GL; o <<= 1) v = fminf(v, __shfl_xor_sync(kFull, v, o));
+    return v;
+}
+__device__ __forceinline__ unsigned group_min(unsigned v) {
+#pragma unroll
+    for (int o = 1; o < GL; o <<= 1) v = min(v, __shfl_xor_sync(kFull, v, o));
+    return v;
+}
+
+// Shared memory of a block of NWARP warps: the planes' tie-break ranks (0xffffffff for planes that take
+// no part), the plane of each rank, and the warps' sums.
+template <int NCH, int NWARP> struct GroupSmem {
+    static constexpr int D = 32 * NCH, PITCH = D + 4;   // 16-byte rows, the pixels' on different banks
+    __align__(16) unsigned rank[D];
+    uint16_t plane[D];
+    __align__(16) float sums[NWARP][GP][PITCH];
+};
+
+// NP pair volumes (NP = 1: vol is the sum itself, or HIN: the FP16 cost volume, whose offset counts once).
+// The calling warp takes pixel groups first, first + nw, ... below ngroups.  FULL: every plane takes part.
+template <int NCH, int MODE, int NP, bool HIN, bool FULL, int NWARP>
+__device__ __forceinline__ void combine_groups(const SgmLaunch& a, const void* const (&vol)[NP],
+                                               GroupSmem<NCH, NWARP>& sm, long first, long nw, long ngroups) {
+    constexpr int D = 32 * NCH, NV = 4 * NCH;   // planes, and planes per lane
+    constexpr int VEC = HIN ? 8 : 4;            // planes per 16-byte load
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane % GL, q = lane / GL;     // lane of the pixel, pixel of the group
+    for (int d = threadIdx.x; d < D; d += NWARP * 32) {
+        if constexpr (MODE == kCombineArgmin) {
+            sm.rank[d] = (unsigned)d;           // planes in order
+            sm.plane[d] = (uint16_t)d;
+        } else {
+            const int ppl = D / 32;
+            const bool in = (a.order.incl[d / ppl] >> (d % ppl)) & 1u;
+            const unsigned r = a.order.rank[d];
+            sm.rank[d] = in ? r : 0xffffffffu;
+            if (in) sm.plane[r] = (uint16_t)d;
+        }
+    }
+    __syncthreads();
+    const long npix = (long)a.W * a.H;
+    // plane of the lane's value j
+    auto plane = [&](int j) { return (j / VEC) * (GL * VEC) + g * VEC + j % VEC; };
+    float(&row)[GroupSmem<NCH, NWARP>::PITCH] = sm.sums[warp][q];
+    const bool contiguous = a.depth_pitch == (size_t)a.W * sizeof(float);
+    for (long grp = first; grp < ngroups; grp += nw) {
+        const long pix = grp * GP + q;
+        const bool live = pix < npix;
+        long lp = live ? pix : npix - 1;
+        if (!PM_RANGE_IN_BOUNDS(lp * D, D, (long long)npix * D, kSiteCombineLoad)) lp = 0;   // the warp stays together
+        float s[NV];
+        const float off = HIN ? __ldg(a.offset + lp) : 0.0f;
+#pragma unroll
+        for (int c = 0; c < NV; c += VEC) {
+            const size_t e = (size_t)lp * D + (c / VEC) * (GL * VEC) + g * VEC;
+            float v[NP][VEC];
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                if constexpr (HIN) {
+                    const uint4 t = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(vol[p]) + e));
+                    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                        v[p][2 * i] = f.x;
+                        v[p][2 * i + 1] = f.y;
+                    }
+                } else {
+                    const float4 t = *reinterpret_cast<const float4*>(static_cast<const float*>(vol[p]) + e);
+                    v[p][0] = t.x; v[p][1] = t.y; v[p][2] = t.z; v[p][3] = t.w;
+                }
+            }
+            float o[VEC];
+            if constexpr (NP == 4) {
+                float s01[VEC], s23[VEC];
+                add_planes<VEC>(s01, v[0], v[1]);
+                add_planes<VEC>(s23, v[2], v[3]);
+                add_planes<VEC>(o, s01, s23);
+            } else if constexpr (NP == 2) {
+                add_planes<VEC>(o, v[0], v[1]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) o[i] = v[0][i];
+            }
+            if constexpr (HIN) add_planes<VEC>(o, o, NP == 1 ? off : __fmul_rn((float)(2 * NP), off));
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) s[c + i] = o[i];
+        }
+        if (a.total && live)
+#pragma unroll
+            for (int c = 0; c < NV; c += 4)
+                *reinterpret_cast<float4*>(a.total + (size_t)pix * D + plane(c)) = make_float4(s[c], s[c + 1], s[c + 2], s[c + 3]);
+
+        float depth;
+        int idx, cls = kWtaDepth;
+        // minimum over the planes that take part, then the lowest rank among its holders
+        float m = inf_f();
+#pragma unroll
+        for (int c = 0; c < NV; c += 4) {
+            const uint4 r = FULL || MODE == kCombineArgmin ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(sm.rank + plane(c));
+            const unsigned rk[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) m = FULL || MODE == kCombineArgmin || rk[i] != 0xffffffffu ? fminf(m, s[c + i]) : m;
+        }
+        if constexpr (MODE == kCombineArgmin) m = fminf(m, 100000.0f);
+        const float mn = group_min(m);
+        unsigned best = 0xffffffffu;
+#pragma unroll
+        for (int c = 0; c < NV; c += 4) {
+            const uint4 r = *reinterpret_cast<const uint4*>(sm.rank + plane(c));
+            const unsigned rk[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) best = s[c + i] == mn && rk[i] < best ? rk[i] : best;
+        }
+        best = group_min(best);
+        if constexpr (MODE == kCombineArgmin) {
+            // no plane below 100000: plane 0 (a value equal to 100000 is not below it)
+            idx = mn < 100000.0f && best < (unsigned)D ? (int)best : 0;
+            if (below_eps(mn)) depth = kCaseInf;
+            else if (idx == 0 || idx == D - 1) depth = 0.0f;
+            else depth = rcp_rn(__fmaf_rn((float)idx, a.fp.drho, a.fp.rho0));
+        } else {
+            idx = best < (unsigned)D ? (int)sm.plane[best] : 0;
+#pragma unroll
+            for (int c = 0; c < NV; c += 4) *reinterpret_cast<float4*>(&row[plane(c)]) = make_float4(s[c], s[c + 1], s[c + 2], s[c + 3]);
+            __syncwarp();
+            const float pre = row[idx > 0 ? idx - 1 : 0], post = row[idx < D - 1 ? idx + 1 : D - 1];
+            float second = inf_f();
+            const bool uniq = a.fp.uniq > 0.0f && a.fp.uniq < 1.0f;
+            if (uniq) {   // kernel-uniform
+#pragma unroll
+                for (int c = 0; c < NV; c += 4) {
+                    const uint4 r = FULL ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(sm.rank + plane(c));
+                    const unsigned rk[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const bool far = (unsigned)(plane(c) + i - idx + 1) > 2u;   // d < idx - 1 or d > idx + 1
+                        second = far && (FULL || rk[i] != 0xffffffffu) ? fminf(second, s[c + i]) : second;
+                    }
+                }
+                second = group_min(second);
+            }
+            __syncwarp();   // the row is read before the next group's sums are written
+            if (within_eps(mn)) {
+                depth = kDepInf;                                   // non-overlap (filter_cost.cu:37-38)
+                cls = kWtaNoOverlap;
+            } else if (idx == 0 || idx == D - 1) {
+                depth = 0.0f;                                      // border plane (:39-40)
+                cls = kWtaBorder;
+            } else if (__fadd_rn(pre, post) < __fmul_rn(__fmul_rn(2.0f, mn), a.fp.var_scale)) {
+                depth = 0.0f;                                      // flat minimum (:41-42)
+                cls = kWtaFlat;
+            } else if (uniq && mn > __fmul_rn(a.fp.uniq, second)) {
+                depth = 0.0f;
+                cls = kWtaAmbiguous;
+            } else {                                               // parabola (:45-51)
+                const float a2 = __fadd_rn(__fsub_rn(pre, __fmul_rn(2.0f, mn)), post);
+                const float b = __fadd_rn(-pre, post);
+                const float sub = __fsub_rn((float)idx, __fdiv_rn(b, __fmul_rn(2.0f, a2)));
+                depth = rcp_rn(__fmaf_rn(sub, a.fp.drho, a.fp.rho0));
+            }
+        }
+        if (g == 0 && live && PM_IN_BOUNDS(pix, (long long)npix, kSiteCombineOut)) {
+            float* dp = a.depth + pix;
+            if (!contiguous) {   // W * H < 2^32: 32-bit division
+                const unsigned up = (unsigned)pix, uw = (unsigned)a.W;
+                const unsigned y = up / uw, x = up - y * uw;
+                dp = reinterpret_cast<float*>(reinterpret_cast<char*>(a.depth) + (size_t)y * a.depth_pitch) + x;
+            }
+            *dp = depth;
+            if (a.index) a.index[pix] = idx;
+            if (a.wta_class) a.wta_class[pix] = (uint8_t)cls;
+        }
+    }
+}
+
 }  // namespace
 }  // namespace pm
