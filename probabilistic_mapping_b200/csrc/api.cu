@@ -45,8 +45,6 @@ struct pm_mapper {
     float* d_boff = nullptr;    // FP16 form: block offsets before the rebase (W*H*D/16)
     float* d_cnt = nullptr;     // allocated on the first fold
     float* d_part[4] = {};      // SGM: one volume per opposite-path pair (num_paths / 2 of them)
-    SgmStreams side{};          // concurrent path groups
-    bool have_side = false;
     float* d_depth = nullptr;   // WTA depth, linear
     int32_t* d_idx = nullptr;   // WTA plane index
     bool store_sgm = false;
@@ -323,7 +321,7 @@ pm_status run_sgm_filter(pm_mapper* h) {
     a.depth_pitch = sizeof(float) * (size_t)c.width;
     a.index = h->d_idx;
     a.wta_class = h->stats ? h->d_wta_class : nullptr;
-    PM_CK(h, launch_sgm(a, kCombineFilter, h->stream, h->have_side ? &h->side : nullptr));
+    PM_CK(h, launch_sgm(a, kCombineFilter, h->stream));
     if (h->stats)
         PM_CK(h, launch_count_classes(h->d_wta_class, (long)c.width * c.height, kWtaClasses, h->d_stats + kStatWta,
                                       h->stream));
@@ -393,11 +391,6 @@ void release(pm_mapper* h) {
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
     if (h->ev_cost_kernel) cudaEventDestroy(h->ev_cost_kernel);
-    for (int g = 0; g < 3; ++g) {
-        if (h->side.stream[g]) cudaStreamDestroy(h->side.stream[g]);
-        if (h->side.join[g]) cudaEventDestroy(h->side.join[g]);
-    }
-    if (h->side.fork) cudaEventDestroy(h->side.fork);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -476,13 +469,6 @@ pm_status pm_create(const pm_config* cfg, pm_mapper** out) {
     }
     for (int s = 0; s < 2 && ok; ++s)
         for (int k = 0; k < 4 && ok; ++k) ok = alloc((void**)&h->d_state[s][k], 4 * N);
-    if (ok) {
-        ok = note(cudaEventCreateWithFlags(&h->side.fork, cudaEventDisableTiming));
-        for (int g3 = 0; g3 < 3 && ok; ++g3)
-            ok = note(cudaStreamCreateWithFlags(&h->side.stream[g3], cudaStreamNonBlocking)) &&
-                 note(cudaEventCreateWithFlags(&h->side.join[g3], cudaEventDisableTiming));
-        h->have_side = ok;
-    }
     if (ok) ok = cudaMemsetAsync(h->d_table, 0, 4 * N, h->stream) == cudaSuccess;
     for (int s = 0; s < 2 && ok; ++s)
         for (int k = 0; k < 4 && ok; ++k) ok = cudaMemsetAsync(h->d_state[s][k], 0, 4 * N, h->stream) == cudaSuccess;
@@ -618,7 +604,7 @@ pm_status pm_output_case(pm_mapper* h, int output_case, float* result, size_t pi
         a.depth = h->d_fused;
         a.depth_pitch = sizeof(float) * (size_t)c.width;
         a.index = h->d_idx;
-        PM_CK(h, launch_sgm(a, kCombineArgmin, h->stream, h->have_side ? &h->side : nullptr));
+        PM_CK(h, launch_sgm(a, kCombineArgmin, h->stream));
     }
     mark_done(h, 1);
     mark(h, 3);
@@ -927,7 +913,7 @@ pm_status pm_stage_sgm(const pm_config* cfg, const float* cost, const float* ref
     a.part[0] = out;   // the combine kernel reads part[0] of a pixel before it writes the total there
     for (int r = 1; r < cfg->num_paths / 2; ++r) a.part[r] = scratch + (r - 1) * V;
     a.total = out;
-    return launch_sgm(a, kCombineStore, (cudaStream_t)stream, nullptr) == cudaSuccess ? PM_OK : PM_ERR_CUDA;
+    return launch_sgm(a, kCombineStore, (cudaStream_t)stream) == cudaSuccess ? PM_OK : PM_ERR_CUDA;
 }
 
 pm_status pm_stage_filter(const pm_config* cfg, const float* sgm, float* depth, size_t pitch, int32_t* index,
@@ -962,7 +948,7 @@ pm_status pm_stage_sgm_filter(const pm_config* cfg, const float* cost, const flo
     a.depth = depth;
     a.depth_pitch = pitch;
     a.index = index;
-    return launch_sgm(a, kCombineFilter, (cudaStream_t)stream, nullptr) == cudaSuccess ? PM_OK : PM_ERR_CUDA;
+    return launch_sgm(a, kCombineFilter, (cudaStream_t)stream) == cudaSuccess ? PM_OK : PM_ERR_CUDA;
 }
 
 pm_status pm_stage_depth_fuse(int W, int H, const float pose[12], const float cam[4], float* depth,

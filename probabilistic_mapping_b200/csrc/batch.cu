@@ -91,9 +91,8 @@ struct Seq {
     int pair_warps = 4, serial_pairs = 0;
     float tuned_ms = 0.0f;
     // capture streams and events
-    cudaStream_t st[4] = {};
-    SgmStreams side{};
-    cudaEvent_t done = nullptr, lane_free = nullptr;
+    cudaStream_t st = nullptr;
+    cudaEvent_t done = nullptr, lane_free = nullptr, inputs = nullptr;
 };
 
 }  // namespace
@@ -196,11 +195,8 @@ void free_batch(pm_batch* b) {
         cudaFree(q.d_var);
         cudaFree(q.d_stats);
         cudaFree(q.d_cls);
-        for (auto& s : q.st)
-            if (s) cudaStreamDestroy(s);
-        if (q.side.fork) cudaEventDestroy(q.side.fork);
-        for (auto& e : q.side.join)
-            if (e) cudaEventDestroy(e);
+        if (q.st) cudaStreamDestroy(q.st);
+        if (q.inputs) cudaEventDestroy(q.inputs);
         if (q.done) cudaEventDestroy(q.done);
         if (q.lane_free) cudaEventDestroy(q.lane_free);
     }
@@ -341,7 +337,7 @@ cudaError_t count_wta_classes(const Seq& q, cudaStream_t m) {
 cudaError_t enqueue_seq(pm_batch* b, int i, int k) {
     Seq& q = b->seqs[i];
     LaneBufs& l = b->lanes[q.lane];
-    cudaStream_t m = q.st[0];
+    cudaStream_t m = q.st;
     cudaError_t e;
     if ((e = enqueue_inputs(b, i, k, m))) return e;
     if ((e = clear_stats(q, m))) return e;
@@ -350,7 +346,7 @@ cudaError_t enqueue_seq(pm_batch* b, int i, int k) {
     l.last_user = i;
     if ((e = launch_cost(cost_launch(q, l, k), m))) return e;
     const SgmLaunch g = sgm_launch(q, l, b->sgm_priority);
-    if ((e = launch_sgm(g, kCombineFilter, m, &q.side))) return e;
+    if ((e = launch_sgm(g, kCombineFilter, m))) return e;
     if ((e = cudaEventRecord(q.lane_free, m))) return e;
     if ((e = count_wta_classes(q, m))) return e;
     return enqueue_fusion(b, i, k, m);
@@ -474,11 +470,11 @@ cudaError_t enqueue_persist(pm_batch* b, int k) {
     cudaError_t e;
     for (int i = 0; i < (int)b->seqs.size(); ++i) {
         Seq& q = b->seqs[i];
-        if ((e = cudaStreamWaitEvent(q.st[0], b->root, 0))) return e;
-        if ((e = enqueue_inputs(b, i, k, q.st[0]))) return e;
-        if ((e = clear_stats(q, q.st[0]))) return e;
-        if ((e = cudaEventRecord(q.side.fork, q.st[0]))) return e;
-        if ((e = cudaStreamWaitEvent(b->run, q.side.fork, 0))) return e;
+        if ((e = cudaStreamWaitEvent(q.st, b->root, 0))) return e;
+        if ((e = enqueue_inputs(b, i, k, q.st))) return e;
+        if ((e = clear_stats(q, q.st))) return e;
+        if ((e = cudaEventRecord(q.inputs, q.st))) return e;
+        if ((e = cudaStreamWaitEvent(b->run, q.inputs, 0))) return e;
     }
     if ((e = cudaMemsetAsync(b->d_counters, 0, b->counter_bytes, b->run))) return e;
     PersistLaunch L = b->plaunch;
@@ -487,10 +483,10 @@ cudaError_t enqueue_persist(pm_batch* b, int k) {
     if ((e = cudaEventRecord(b->persist_done, b->run))) return e;
     for (int i = 0; i < (int)b->seqs.size(); ++i) {
         Seq& q = b->seqs[i];
-        if ((e = cudaStreamWaitEvent(q.st[0], b->persist_done, 0))) return e;
-        if ((e = count_wta_classes(q, q.st[0]))) return e;
-        if ((e = enqueue_fusion(b, i, k, q.st[0]))) return e;
-        if ((e = cudaEventRecord(q.done, q.st[0]))) return e;
+        if ((e = cudaStreamWaitEvent(q.st, b->persist_done, 0))) return e;
+        if ((e = count_wta_classes(q, q.st))) return e;
+        if ((e = enqueue_fusion(b, i, k, q.st))) return e;
+        if ((e = cudaEventRecord(q.done, q.st))) return e;
         if ((e = cudaStreamWaitEvent(b->run, q.done, 0))) return e;
     }
     return cudaSuccess;
@@ -508,9 +504,9 @@ pm_status build_graphs(pm_batch* b) {
         if (b->persistent && e == cudaSuccess) e = enqueue_persist(b, k);
         for (int i = 0; !b->persistent && i < (int)b->seqs.size() && e == cudaSuccess; ++i) {
             Seq& q = b->seqs[i];
-            e = cudaStreamWaitEvent(q.st[0], b->root, 0);
+            e = cudaStreamWaitEvent(q.st, b->root, 0);
             if (e == cudaSuccess) e = enqueue_seq(b, i, k);
-            if (e == cudaSuccess) e = cudaEventRecord(q.done, q.st[0]);
+            if (e == cudaSuccess) e = cudaEventRecord(q.done, q.st);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(b->run, q.done, 0);
         }
         cudaGraph_t g = nullptr;
@@ -559,9 +555,9 @@ pm_status autotune(pm_batch* b) {
                 q.pair_warps = w;
                 q.serial_pairs = serial;
                 const SgmLaunch g = sgm_launch(q, l, 0);
-                e = launch_sgm(g, kCombineFilter, b->run, &q.side);   // warm-up
+                e = launch_sgm(g, kCombineFilter, b->run);   // warm-up
                 if (e == cudaSuccess) e = cudaEventRecord(t0, b->run);
-                for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = launch_sgm(g, kCombineFilter, b->run, &q.side);
+                for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = launch_sgm(g, kCombineFilter, b->run);
                 if (e == cudaSuccess) e = cudaEventRecord(t1, b->run);
                 if (e == cudaSuccess) e = cudaEventSynchronize(t1);
                 float ms = 0.0f;
@@ -681,15 +677,10 @@ pm_status pm_batch_create(const pm_config* cfgs, int n, int num_sources, int lan
         for (int s = 0; q.cfg.sampler != PM_SAMPLER_EXACT && s < q.S && ok; ++s)
             ok = note(make_source_texture(q.cfg.width, q.cfg.height, q.cfg.sampler == PM_SAMPLER_TEXTURE_F32,
                                           &q.d_srch[s], &q.srch_pitch, &q.tex[s]));
-        for (int s = 0; s < 4 && ok; ++s) ok = note(cudaStreamCreateWithFlags(&q.st[s], cudaStreamNonBlocking));
-        if (ok) {
-            for (int s = 0; s < 3; ++s) q.side.stream[s] = q.st[1 + s];
-            ok = note(cudaEventCreateWithFlags(&q.side.fork, cudaEventDisableTiming)) &&
-                 note(cudaEventCreateWithFlags(&q.done, cudaEventDisableTiming)) &&
-                 note(cudaEventCreateWithFlags(&q.lane_free, cudaEventDisableTiming));
-            for (int s = 0; s < 3 && ok; ++s)
-                ok = note(cudaEventCreateWithFlags(&q.side.join[s], cudaEventDisableTiming));
-        }
+        ok = ok && note(cudaStreamCreateWithFlags(&q.st, cudaStreamNonBlocking)) &&
+             note(cudaEventCreateWithFlags(&q.inputs, cudaEventDisableTiming)) &&
+             note(cudaEventCreateWithFlags(&q.done, cudaEventDisableTiming)) &&
+             note(cudaEventCreateWithFlags(&q.lane_free, cudaEventDisableTiming));
     }
     pm_status tune = PM_OK;
     if (ok && (flags & PM_BATCH_AUTOTUNE) && !b->persistent) {

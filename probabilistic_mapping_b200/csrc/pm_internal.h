@@ -104,26 +104,19 @@ struct SgmLaunch {
     size_t depth_pitch;
     int32_t* index;        // W*H (optional)
     PlaneOrder order;
-    int pair_warps;        // scanlines per block of the path-pair kernel: 2, 4 or 8 (0: 2)
-    int serial_pairs;      // 1: run the path pairs one after another on the caller's stream
+    int pair_warps;        // scanlines per block of the path-pair kernel: 2, 4 or 8 (0: by the image)
+    int serial_pairs;      // 1: one launch per path pair, one after another, instead of one for all
     int priority;          // launch priority of the pair and combine kernels (0: the stream's)
     uint8_t* wta_class;    // W*H winner-take-all class of each pixel (WtaClass, fused filter only), or nullptr
 };
 // pm_stats: adds the per-pixel classes (values below n) of npix pixels to the n counters at g.
 cudaError_t launch_count_classes(const uint8_t* cls, long npix, int n, unsigned* g, cudaStream_t s);
-// Side streams for the concurrent path pairs: pairs 0..2 fork from the caller's stream and join
-// back before the combine kernel.
-struct SgmStreams {
-    cudaStream_t stream[3];
-    cudaEvent_t fork;
-    cudaEvent_t join[3];
-};
 // What the combine kernel does with the summed path volumes.
 enum CombineMode { kCombineStore = 0, kCombineFilter = 1, kCombineArgmin = 2 };
 // Runs the opposite-path pairs (pair p into part[p]), then adds the pair volumes in registers
 // and writes depth/index with the winner-take-all filter (kCombineFilter) or the debug argmin
-// (kCombineArgmin); kCombineStore only writes `total`.  side == nullptr runs everything on s.
-cudaError_t launch_sgm(const SgmLaunch& a, int mode, cudaStream_t s, const SgmStreams* side);
+// (kCombineArgmin); kCombineStore only writes `total`.
+cudaError_t launch_sgm(const SgmLaunch& a, int mode, cudaStream_t s);
 // The debug argmin over a float (half = 0) or __half (half = 1, shifted by offset) W*H*D volume.
 cudaError_t launch_case_argmin(const void* vol, int half, const float* offset, int W, int H, int D,
                                const FilterParams& fp, float* depth, size_t pitch, int32_t* index, cudaStream_t s);

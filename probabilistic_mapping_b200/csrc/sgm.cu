@@ -16,7 +16,7 @@
 //     the minima (D a power of two, or the exact minimum);
 //   * opposite paths run as pairs: one warp walks a scanline from both ends at once, so it keeps
 //     two independent recurrences in flight; the pairs (L/R, T/B and the two diagonals) run
-//     concurrently on separate streams.  Each pair owns one volume: the path that reaches a pixel
+//     side by side in one launch.  Each pair owns one volume: the path that reaches a pixel
 //     first stores its values there and the other adds its own with a vector reduction, so the
 //     volume ends up holding P_2p + P_2p+1 (float addition is commutative, so this is the same
 //     sum in either order);
@@ -68,10 +68,15 @@ void plane_order(int D, int compat, PlaneOrder& out) {
 
 namespace {
 
+// The path pairs of ps, side by side in one launch: their scanlines are independent, and one pair's
+// alone leave an SM three or four warps of a latency-bound recurrence.
 template <int PPL, bool HALF, int NW, bool FULL, bool HOUT>
-__global__ void __launch_bounds__(NW * 32) sgm_pair_kernel(const SgmLaunch a, int dx, int dy, int slot) {
+__global__ void __launch_bounds__(NW * 32) sgm_pair_kernel(const SgmLaunch a, const PairSet ps) {
     extern __shared__ __align__(16) unsigned char ring[];
-    sgm_pair_block<PPL, HALF, NW, FULL, HOUT>(a, dx, dy, slot, blockIdx.x, ring);
+    int bx = blockIdx.x, dx, dy;
+    const int pair = pair_of_block(ps, bx);
+    pair_dir(pair, dx, dy);
+    sgm_pair_block<PPL, HALF, NW, FULL, HOUT>(a, dx, dy, 2 * pair, bx, ring);
 }
 
 // Blocks per SM that the one-pixel combine kernel is held to (0: no bound): D = 192 in FP32, where the
@@ -196,10 +201,10 @@ bool all_planes(const PlaneOrder& o, int ppl) {
 }
 
 template <int PPL, bool HALF, int NW>
-cudaError_t launch_pair_nw(const SgmLaunch& a, int pair, cudaStream_t s) {
+cudaError_t launch_pairs_nw(const SgmLaunch& a, unsigned mask, cudaStream_t s) {
     const size_t smem = (size_t)NW * PF * Ring<PPL, HALF>::STAGE_B;
     const bool full = all_planes(a.order, PPL);
-    void (*kern)(SgmLaunch, int, int, int);
+    void (*kern)(SgmLaunch, PairSet);
     if constexpr (HALF && PPL % 2 == 0) {
         if (a.part_half) kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, true> : sgm_pair_kernel<PPL, HALF, NW, false, true>;
         else kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, false> : sgm_pair_kernel<PPL, HALF, NW, false, false>;
@@ -211,23 +216,24 @@ cudaError_t launch_pair_nw(const SgmLaunch& a, int pair, cudaStream_t s) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    int dx, dy;
-    pair_dir(pair, dx, dy);
-    const int nch = num_chains(dx, dy, a.W, a.H);
-    return launch_with_priority(kern, dim3((nch + NW - 1) / NW), dim3(NW * 32), smem, s, a.priority, a, dx, dy,
-                                2 * pair);
+    const PairSet ps = make_pair_set(mask, a.W, a.H, NW);
+    return launch_with_priority(kern, dim3(ps.start[ps.n]), dim3(NW * 32), smem, s, a.priority, a, ps);
 }
 
-// scanlines (warps) per block: a.pair_warps in {2, 4, 8}, 2 when unset (the batched form's
-// autotuner picks 2 for the 640x480x128 map too: smaller blocks spread one map's few scanlines
-// over more SMs)
+// Scanlines (warps) per block: a.pair_warps in {2, 4, 8}, or by the image when unset.  Four neighbouring
+// scanlines read and write neighbouring pixels, which keeps DRAM pages and L2 sectors together: 2 -> 4 warps per
+// block takes the stage at 752x480x128 FP16 from 470 to 388 us, 640x480x128 FP16 394 -> 362, 1280x720x192 FP32
+// 3420 -> 3250 (8: 439, 368, 3256).  Where an SM gets fewer than twelve scanlines they are spread over
+// the SMs instead: 333x251x96 154 -> 148 us with one per block, 96x64x32, 4 paths 26.9 -> 25.3.
 template <int PPL, bool HALF>
-cudaError_t launch_pair(const SgmLaunch& a, int pair, cudaStream_t s) {
+cudaError_t launch_pairs(const SgmLaunch& a, unsigned mask, cudaStream_t s) {
     switch (a.pair_warps) {
-        case 4: return launch_pair_nw<PPL, HALF, 4>(a, pair, s);
-        case 8: return launch_pair_nw<PPL, HALF, 8>(a, pair, s);
-        default: return launch_pair_nw<PPL, HALF, 2>(a, pair, s);
+        case 2: return launch_pairs_nw<PPL, HALF, 2>(a, mask, s);
+        case 4: return launch_pairs_nw<PPL, HALF, 4>(a, mask, s);
+        case 8: return launch_pairs_nw<PPL, HALF, 8>(a, mask, s);
+        default: break;
     }
+    return few_chains(mask, a.W, a.H) ? launch_pairs_nw<PPL, HALF, 1>(a, mask, s) : launch_pairs_nw<PPL, HALF, 4>(a, mask, s);
 }
 
 int sm_count() {
@@ -284,29 +290,16 @@ cudaError_t launch_combine(const SgmLaunch& a, int mode, cudaStream_t s) {
                                 a.priority, a);
 }
 
-// Path pairs p = 0 .. num_paths/2 - 1: pairs 0..np-2 run on their own side streams when `side`
-// is given, the last on `s`, which then joins the others and runs the combine kernel.
+// Path pairs p = 0 .. num_paths/2 - 1 in one launch (serial_pairs: one launch each), then the combine kernel.
 template <int PPL, bool HALF>
-cudaError_t launch_sgm_t(const SgmLaunch& a, int mode, cudaStream_t s, const SgmStreams* side) {
+cudaError_t launch_sgm_t(const SgmLaunch& a, int mode, cudaStream_t s) {
     const int np = a.num_paths / 2;
     cudaError_t e = cudaSuccess;
-    if (a.serial_pairs) side = nullptr;
-    if (side) {
-        if ((e = cudaEventRecord(side->fork, s)) != cudaSuccess) return e;
-        for (int p = 0; p < np - 1; ++p) {
-            if ((e = cudaStreamWaitEvent(side->stream[p], side->fork, 0)) != cudaSuccess) return e;
-            if ((e = launch_pair<PPL, HALF>(a, p, side->stream[p])) != cudaSuccess) return e;
-            if ((e = cudaEventRecord(side->join[p], side->stream[p])) != cudaSuccess) return e;
-        }
-    } else {
-        for (int p = 0; p < np - 1 && e == cudaSuccess; ++p) e = launch_pair<PPL, HALF>(a, p, s);
-        if (e != cudaSuccess) return e;
-    }
-    if ((e = launch_pair<PPL, HALF>(a, np - 1, s)) != cudaSuccess) return e;
-    if (side)
-        for (int p = 0; p < np - 1; ++p)
-            if ((e = cudaStreamWaitEvent(s, side->join[p], 0)) != cudaSuccess) return e;
-    return launch_combine<PPL>(a, mode, s);
+    if (a.serial_pairs)
+        for (int p = 0; p < np && e == cudaSuccess; ++p) e = launch_pairs<PPL, HALF>(a, 1u << p, s);
+    else
+        e = launch_pairs<PPL, HALF>(a, (1u << np) - 1u, s);
+    return e != cudaSuccess ? e : launch_combine<PPL>(a, mode, s);
 }
 
 template <int PPL>
@@ -334,23 +327,23 @@ cudaError_t launch_filter_t(const float* sum, int W, int H, int D, const FilterP
 
 }  // namespace
 
-cudaError_t launch_sgm(const SgmLaunch& a, int mode, cudaStream_t s, const SgmStreams* side) {
+cudaError_t launch_sgm(const SgmLaunch& a, int mode, cudaStream_t s) {
     const int ppl = a.D / 32;
     // FP16 volumes need an even number of planes per lane (4-byte cp.async pieces)
     if (a.cost_half && (ppl % 2)) return cudaErrorInvalidValue;
     switch (ppl) {
-        case 1: return launch_sgm_t<1, false>(a, mode, s, side);
-        case 2: return a.cost_half ? launch_sgm_t<2, true>(a, mode, s, side)
-                                   : launch_sgm_t<2, false>(a, mode, s, side);
-        case 3: return launch_sgm_t<3, false>(a, mode, s, side);
-        case 4: return a.cost_half ? launch_sgm_t<4, true>(a, mode, s, side)
-                                   : launch_sgm_t<4, false>(a, mode, s, side);
-        case 5: return launch_sgm_t<5, false>(a, mode, s, side);
-        case 6: return a.cost_half ? launch_sgm_t<6, true>(a, mode, s, side)
-                                   : launch_sgm_t<6, false>(a, mode, s, side);
-        case 7: return launch_sgm_t<7, false>(a, mode, s, side);
-        case 8: return a.cost_half ? launch_sgm_t<8, true>(a, mode, s, side)
-                                   : launch_sgm_t<8, false>(a, mode, s, side);
+        case 1: return launch_sgm_t<1, false>(a, mode, s);
+        case 2: return a.cost_half ? launch_sgm_t<2, true>(a, mode, s)
+                                   : launch_sgm_t<2, false>(a, mode, s);
+        case 3: return launch_sgm_t<3, false>(a, mode, s);
+        case 4: return a.cost_half ? launch_sgm_t<4, true>(a, mode, s)
+                                   : launch_sgm_t<4, false>(a, mode, s);
+        case 5: return launch_sgm_t<5, false>(a, mode, s);
+        case 6: return a.cost_half ? launch_sgm_t<6, true>(a, mode, s)
+                                   : launch_sgm_t<6, false>(a, mode, s);
+        case 7: return launch_sgm_t<7, false>(a, mode, s);
+        case 8: return a.cost_half ? launch_sgm_t<8, true>(a, mode, s)
+                                   : launch_sgm_t<8, false>(a, mode, s);
         default: return cudaErrorInvalidValue;
     }
 }

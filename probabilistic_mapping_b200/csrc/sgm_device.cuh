@@ -34,7 +34,8 @@ __host__ __device__ inline int num_chains(int dx, int dy, int W, int H) {
     return dy == 0 ? H : (dx == 0 ? W : W + H - 1);
 }
 
-// The pairs of `mask` (bit p: pair p), those with the longest scanlines first.
+// The pairs of `mask` (bit p: pair p), those with the longest scanlines first, the vertical one of a wide image
+// last (at 752x480x128 FP16 this order takes 388 us, the pairs' own 407 and their reverse 440).
 inline PairSet make_pair_set(unsigned mask, int W, int H, int nw) {
     PairSet s{};
     const int wide[4] = {0, 2, 3, 1}, tall[4] = {1, 2, 3, 0};
@@ -48,6 +49,11 @@ inline PairSet make_pair_set(unsigned mask, int W, int H, int nw) {
         ++s.n;
     }
     return s;
+}
+// Fewer than twelve scanlines per SM: one per block, else four neighbouring ones.
+inline bool few_chains(unsigned mask, int W, int H) {
+    const PairSet s = make_pair_set(mask, W, H, 1);
+    return s.start[s.n] < 148 * 12;
 }
 // The pair of block bx; bx becomes the block's index within it.
 __device__ __forceinline__ int pair_of_block(const PairSet& s, int& bx) {
