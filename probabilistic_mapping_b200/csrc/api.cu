@@ -218,6 +218,7 @@ void fill_cost_launch(const pm_config& c, CostLaunch& a) {
     a.drho = c.rho_step;
     a.mode = c.cost_mode;
     a.cost_half = c.precision == PM_PREC_FP16;
+    set_floor_bias(a);
 }
 
 void fill_sgm_launch(const pm_config& c, const PlaneOrder& order, SgmLaunch& a) {
@@ -259,9 +260,9 @@ pm_status upload_image(pm_mapper* h, const uint8_t* img, size_t pitch, float* ds
     else if (slot >= 0 && half && h->cfg.sampler == PM_SAMPLER_TEXTURE_F32)
         PM_CK(h, launch_to_float_h_pitched(W, H, dev, pitch, (float*)h->d_srch[slot], h->srch_pitch, sc, h->stream));
     else if (slot >= 0 && half)
-        PM_CK(h, launch_to_quad_half(W, H, dev, pitch, h->d_srcq + (size_t)slot * W * H, sc, h->stream));
+        PM_CK(h, launch_to_quad_half(W, H, dev, pitch, h->d_srcq + slot * quad_stride((size_t)W * H), sc, h->stream));
     else if (slot >= 0)
-        PM_CK(h, launch_to_quad(W, H, dev, pitch, h->d_srcq + (size_t)slot * W * H, sc, h->stream));
+        PM_CK(h, launch_to_quad(W, H, dev, pitch, h->d_srcq + slot * quad_stride((size_t)W * H), sc, h->stream));
     else if (half)
         PM_CK(h, launch_to_float_h(W, H, dev, pitch, dst, sc, h->stream));
     else
@@ -448,7 +449,8 @@ pm_status pm_create(const pm_config* cfg, pm_mapper** out) {
     h->own_stream = ok;
     const bool half = cfg->precision == PM_PREC_FP16;
     ok = ok && alloc((void**)&h->d_u8, N) && alloc((void**)&h->d_ref, 4 * N) &&
-         (cfg->sampler != PM_SAMPLER_EXACT || alloc((void**)&h->d_srcq, 16 * N * cfg->max_sources)) &&
+         (cfg->sampler != PM_SAMPLER_EXACT || (alloc((void**)&h->d_srcq, 16 * quad_stride(N) * cfg->max_sources) &&
+                                                  note(init_quad_slots(h->d_srcq, N, cfg->max_sources, h->stream)))) &&
          alloc(&h->d_cost, esz * V) && (!half || (alloc((void**)&h->d_off, 4 * N) && alloc((void**)&h->d_boff, 4 * N * (cfg->num_planes / 16)))) &&
          alloc((void**)&h->d_depth, 4 * N) &&
          alloc((void**)&h->d_idx, 4 * N) && alloc((void**)&h->d_ztable, 8 * N) &&

@@ -263,8 +263,8 @@ cudaError_t enqueue_inputs(pm_batch* b, int i, int k, cudaStream_t m) {
             e = half ? launch_to_float_h_pitched(W, H, f, W, (float*)q.d_srch[s], q.srch_pitch, sc, m)
                      : launch_to_float_pitched(W, H, f, W, (float*)q.d_srch[s], q.srch_pitch, sc, m);
         else
-            e = half ? launch_to_quad_half(W, H, f, W, q.d_srcq + (size_t)s * N, sc, m)
-                     : launch_to_quad(W, H, f, W, q.d_srcq + (size_t)s * N, sc, m);
+            e = half ? launch_to_quad_half(W, H, f, W, q.d_srcq + s * quad_stride(N), sc, m)
+                     : launch_to_quad(W, H, f, W, q.d_srcq + s * quad_stride(N), sc, m);
         if (e) return e;
     }
     return cudaSuccess;
@@ -293,6 +293,7 @@ CostLaunch cost_launch(const Seq& q, const LaneBufs& l, int k) {
     a.hom_dev = q.d_par[k];
     a.cost = l.cost;
     a.cost_half = c.precision == PM_PREC_FP16;
+    set_floor_bias(a);
     return a;
 }
 
@@ -665,7 +666,8 @@ pm_status pm_batch_create(const pm_config* cfgs, int n, int num_sources, int lan
             if (ok) std::memset(q.h_par[k], 0, sizeof(float) * q.par_floats);
         }
         ok = ok && alloc((void**)&q.d_ref, 4 * N) &&
-             (q.cfg.sampler != PM_SAMPLER_EXACT || alloc((void**)&q.d_srcq, 16 * N * q.S)) &&
+             (q.cfg.sampler != PM_SAMPLER_EXACT || (alloc((void**)&q.d_srcq, 16 * quad_stride(N) * q.S) &&
+                                                     note(init_quad_slots(q.d_srcq, N, q.S, b->run)))) &&
              alloc((void**)&q.d_depth, 4 * N) && alloc((void**)&q.d_idx, 4 * N) &&
              alloc((void**)&q.d_ztable, 8 * N) && alloc((void**)&q.d_table, 4 * N) &&
              alloc((void**)&q.d_fused, 4 * N) && alloc((void**)&q.d_var, 4 * N) &&

@@ -16,13 +16,16 @@
 //     the plane-innermost layout (cuda_utils.h:34).
 // Source frames are "quads": pixel (x, y) holds I(x,y), I(x,y+1), I(x+1,y), I(x+1,y+1) with the
 // texture border (zero) applied, so a bilinear sample is one aligned 16-byte load whose halves
-// are the packed operands of the horizontal interpolation.  floor() adds 1.5 * 2^23 with
-// round-toward-minus-infinity, leaving the integer part in the mantissa; the reciprocal is
+// are the packed operands of the horizontal interpolation; rejected samples read a quad of NaN.  floor()
+// adds an integer of at least 2^23 with round-toward-minus-infinity, leaving the integer part in the mantissa;
+// the reciprocal is
 // rcp.approx plus one Newton step without a range branch (rcp_warp2: RN(1/w) wherever an
 // image-sized scene puts w, a stated value elsewhere); the divisions of the running mean are a
 // reciprocal-multiply with one FMA correction.  Each is checked over every float against its
 // definition (pm_debug_check_arith), and every packed instruction rounds each element like its
 // scalar counterpart, so the FP32 oracle's scalar algorithm reproduces the volume bit for bit.
+#include <cstring>
+
 #include "cost_device.cuh"
 
 namespace pm {
@@ -82,6 +85,21 @@ cudaError_t launch_q(const CostLaunch& a, dim3 grid, cudaStream_t s) {
 }
 
 }  // namespace
+
+void set_floor_bias(CostLaunch& a) {
+    const uint32_t npix = (uint32_t)a.W * (uint32_t)a.H;
+    uint32_t bits = 0x4B400000u;   // 1.5 * 2^23; each step down moves the product by W + 1, past W*H in H steps
+    while (bits > 0x4B000000u && bits * (uint32_t)(a.W + 1) > 0xffffffffu - npix) --bits;
+    std::memcpy(&a.floor_bias, &bits, sizeof bits);
+}
+
+cudaError_t init_quad_slots(float4* q, size_t npix, int slots, cudaStream_t s) {
+    for (int i = 0; i < slots; ++i) {
+        const cudaError_t e = cudaMemsetAsync(q + i * quad_stride(npix) + npix, 0xff, sizeof(float4), s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
 
 cudaError_t launch_cost(const CostLaunch& a, cudaStream_t s) {
     if (a.nsrc > kMaxSources || a.D % PCB || a.W < 1 || a.H < 1) return cudaErrorInvalidValue;

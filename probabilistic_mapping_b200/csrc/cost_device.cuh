@@ -62,15 +62,18 @@ __device__ __forceinline__ float2 shfl_down2(float2 v) {
 // hardware reciprocal estimate in the warp) or FP32 form (kTexF, FP32 texels of the images, the
 // warp's Newton reciprocal: the reference's own sampler, calc_cost.cu:226-237).
 enum { kPlain = 0, kQuad = 1, kTex = 2, kQuadH = 3, kTexF = 4 };
-template <int SAMP> struct Src;
-template <> struct Src<kPlain> {
-    const float* __restrict__ p;
+// What the warps take negated numerators with (rcp_neg2): the FP32 form's samplers.
+template <int SAMP> constexpr bool kExact = SAMP == kPlain || SAMP == kQuad || SAMP == kTexF;
+// Float and quad images: floor(u) + M and floor(v) + M sit in the low mantissa bits of u + M and v + M rounded
+// down (M the launch's integer in [2^23, 1.5 * 2^23]), so the bits' combination bits(v) * W + bits(u) is the pixel
+// index plus off = bits(M) * (W + 1), modulo 2^32.  The base address is that of pixel -off: M is chosen so that no
+// index a sample can take wraps (CostLaunch::floor_bias).
+template <int SAMP> struct Src {
+    const char* __restrict__ base;
     int W, H;
-};
-template <> struct Src<kQuad> {
-    const float4* __restrict__ q;
-    int W, H;
-    unsigned off;   // (1.5 * 2^23 bit pattern) * (W + 1), folded out of the quad index
+    unsigned off;
+    unsigned rej;    // quads: the index (with off) of the slot's quad of NaN, which rejected samples read
+    float M;
 };
 template <> struct Src<kTex> {
     cudaTextureObject_t t;
@@ -80,11 +83,6 @@ template <> struct Src<kTexF> {
     cudaTextureObject_t t;
     int W, H;
 };
-template <> struct Src<kQuadH> {   // FP16 form: quads of FP16-rounded values in FP32 lanes
-    const float4* __restrict__ q;
-    int W, H;
-    unsigned off;
-};
 
 // Per-source constants of the warps, as packed pairs.
 struct WarpConst {
@@ -92,37 +90,26 @@ struct WarpConst {
     float W1, H1;
 };
 
-// The warped sample of one position (x, y, z) at two planes (calc_cost.cu:85-93):
-// w = z + t3*rho, u = (x + t1*rho) * r, v = (y + t2*rho) * r with r = rcp_warp2(w) (FP16 form:
-// the hardware reciprocal estimate); rejected (NaN) when w < 0 or (u, v) lies outside
-// [0, W-1] x [0, H-1] (NaN coordinates included).
-template <int SAMP>
-__device__ __forceinline__ float2 sample2_core(const Src<SAMP>& src, const WarpConst& c, float2 w, float2 nx,
-                                               float2 ny);
-template <int SAMP>
-__device__ __forceinline__ float2 sample2(const Src<SAMP>& src, const WarpConst& c, float x, float y, float z,
-                                          float2 rho) {
-    return sample2_core<SAMP>(src, c, __ffma2_rn(c.t3, rho, f2(z, z)), __ffma2_rn(c.t1, rho, f2(x, x)),
-                              __ffma2_rn(c.t2, rho, f2(y, y)));
-}
-// The same from the denominator w and the numerators (nx, ny) of the plane pair.
+// The warped sample at two planes (calc_cost.cu:85-93) from the denominators w = z + t3*rho and the
+// numerators (x + t1*rho, y + t2*rho), which the FP32 form's samplers take negated: u = nx * r, v = ny * r with
+// r = 1 / w by rcp_neg2 (FP16 form: the hardware reciprocal estimate); rejected (NaN) when w < 0 or (u, v) lies
+// outside [0, W-1] x [0, H-1] (NaN coordinates included).
 template <int SAMP>
 __device__ __forceinline__ float2 sample2_core(const Src<SAMP>& src, const WarpConst& c, float2 w, float2 nx,
                                                float2 ny) {
     float2 r;
-    if constexpr (SAMP == kTex || SAMP == kQuadH) {
+    if constexpr (!kExact<SAMP>) {
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(w.x));
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(w.y));
     } else {
-        r = rcp_warp2(w);
+        r = rcp_neg2(w);
     }
     const float2 u = __fmul2_rn(nx, r), v = __fmul2_rn(ny, r);
     // u + 0 turns -0 into +0 (which the reference's u < 0 accepts); then 0 <= u <= W-1 is one
     // unsigned compare of the bit patterns: negative values and NaN have patterns above W-1's.
     // The FP16 form's warps already use the reciprocal estimate, so it leaves out the +0: a
     // coordinate of exactly -0 (a numerator of -0, which needs rho = 0) is then rejected.
-    constexpr bool EXACT = !(SAMP == kTex || SAMP == kQuadH);
-    const float2 uz = EXACT ? __fadd2_rn(u, f2(0.0f, 0.0f)) : u, vz = EXACT ? __fadd2_rn(v, f2(0.0f, 0.0f)) : v;
+    const float2 uz = kExact<SAMP> ? __fadd2_rn(u, f2(0.0f, 0.0f)) : u, vz = kExact<SAMP> ? __fadd2_rn(v, f2(0.0f, 0.0f)) : v;
     const unsigned Wb = __float_as_uint(c.W1), Hb = __float_as_uint(c.H1);
     const bool ok0 = (w.x >= 0.0f) && (__float_as_uint(uz.x) <= Wb) && (__float_as_uint(vz.x) <= Hb);
     const bool ok1 = (w.y >= 0.0f) && (__float_as_uint(uz.y) <= Wb) && (__float_as_uint(vz.y) <= Hb);
@@ -133,24 +120,31 @@ __device__ __forceinline__ float2 sample2_core(const Src<SAMP>& src, const WarpC
         const float s0 = tex2D<float>(src.t, uh.x, vh.x);
         const float s1 = tex2D<float>(src.t, uh.y, vh.y);
         return f2(ok0 ? s0 : nan_f(), ok1 ? s1 : nan_f());
-    } else if constexpr (SAMP == kQuad || SAMP == kQuadH) {
-        // 0 <= u, v < 2^22: u + 1.5*2^23 rounded down is 1.5*2^23 + floor(u), exactly, and the
-        // integer part sits in the low mantissa bits
-        const float2 M = f2(12582912.0f, 12582912.0f);
+    } else {
+        const float2 M = f2(src.M, src.M), mM = f2(-src.M, -src.M);
         const float2 tu = __fadd2_rd(u, M), tv = __fadd2_rd(v, M);
-        const float2 a = sub2(u, __fadd2_rn(tu, f2(-12582912.0f, -12582912.0f)));
-        const float2 b = sub2(v, __fadd2_rn(tv, f2(-12582912.0f, -12582912.0f)));
-        // floor(v) * W + floor(u) in 32-bit arithmetic (exact modulo 2^32, the true value is
-        // below W * H); a rejected element reads quad 0 and is replaced by NaN below
-        const unsigned i0 = __float_as_uint(tv.x) * (unsigned)src.W + __float_as_uint(tu.x) - src.off;
-        const unsigned i1 = __float_as_uint(tv.y) * (unsigned)src.W + __float_as_uint(tu.y) - src.off;
-        float2 lo0, hi0, lo1, hi1;
-        {
-            [[maybe_unused]] const long long nq = (long long)src.W * src.H;
-            const bool in0 = !ok0 || PM_IN_BOUNDS(i0, nq, kSiteCostSource);
-            const bool in1 = !ok1 || PM_IN_BOUNDS(i1, nq, kSiteCostSource);
-            const float4 t0 = __ldg(src.q + (ok0 && in0 ? i0 : 0u));
-            const float4 t1 = __ldg(src.q + (ok1 && in1 ? i1 : 0u));
+        const float2 a = sub2(u, __fadd2_rn(tu, mM));
+        const float2 b = sub2(v, __fadd2_rn(tv, mM));
+        unsigned i0 = __float_as_uint(tv.x) * (unsigned)src.W + __float_as_uint(tu.x);
+        unsigned i1 = __float_as_uint(tv.y) * (unsigned)src.W + __float_as_uint(tu.y);
+        [[maybe_unused]] const long long nq = (long long)src.W * src.H;
+        const bool in0 = ok0 && PM_IN_BOUNDS(i0 - src.off, nq, kSiteCostSource);
+        const bool in1 = ok1 && PM_IN_BOUNDS(i1 - src.off, nq, kSiteCostSource);
+        float2 lo0, hi0, lo1, hi1;   // (I(x, y), I(x, y+1)) and (I(x+1, y), I(x+1, y+1)) of the two planes
+        if constexpr (SAMP == kPlain) {
+            // the neighbours of the last column and row, whose weights are 0 there, are read from the pixel itself
+            i0 = in0 ? i0 : src.off;
+            i1 = in1 ? i1 : src.off;
+            const unsigned lastx = __float_as_uint(src.M) + (unsigned)(src.W - 1), lasty = __float_as_uint(src.M) + (unsigned)(src.H - 1);
+            const unsigned dx0 = in0 && __float_as_uint(tu.x) < lastx ? 1u : 0u, dx1 = in1 && __float_as_uint(tu.y) < lastx ? 1u : 0u;
+            const unsigned dy0 = in0 && __float_as_uint(tv.x) < lasty ? (unsigned)src.W : 0u;
+            const unsigned dy1 = in1 && __float_as_uint(tv.y) < lasty ? (unsigned)src.W : 0u;
+            auto at = [&](unsigned i) { return __ldg(reinterpret_cast<const float*>(src.base + (size_t)i * 4)); };
+            lo0 = f2(at(i0), at(i0 + dy0)); hi0 = f2(at(i0 + dx0), at(i0 + dy0 + dx0));
+            lo1 = f2(at(i1), at(i1 + dy1)); hi1 = f2(at(i1 + dx1), at(i1 + dy1 + dx1));
+        } else {
+            const float4 t0 = __ldg(reinterpret_cast<const float4*>(src.base + (size_t)(in0 ? i0 : src.rej) * 16));
+            const float4 t1 = __ldg(reinterpret_cast<const float4*>(src.base + (size_t)(in1 ? i1 : src.rej) * 16));
             lo0 = f2(t0.x, t0.y); hi0 = f2(t0.z, t0.w);
             lo1 = f2(t1.x, t1.y); hi1 = f2(t1.z, t1.w);
         }
@@ -159,11 +153,16 @@ __device__ __forceinline__ float2 sample2_core(const Src<SAMP>& src, const WarpC
         const float2 p1 = __ffma2_rn(f2(a.y, a.y), sub2(hi1, lo1), lo1);
         const float s0 = __fmaf_rn(b.x, __fsub_rn(p0.y, p0.x), p0.x);
         const float s1 = __fmaf_rn(b.y, __fsub_rn(p1.y, p1.x), p1.x);
-        return f2(ok0 ? s0 : nan_f(), ok1 ? s1 : nan_f());
-    } else {
-        return f2(ok0 ? bilinear(src.p, src.W, src.H, u.x, v.x) : nan_f(),
-                  ok1 ? bilinear(src.p, src.W, src.H, u.y, v.y) : nan_f());
+        if constexpr (SAMP == kPlain) return f2(ok0 ? s0 : nan_f(), ok1 ? s1 : nan_f());
+        return f2(s0, s1);
     }
+}
+// The same from the (negated, see above) numerators' terms of one position at the plane pair.
+template <int SAMP>
+__device__ __forceinline__ float2 sample2(const Src<SAMP>& src, const WarpConst& c, float x, float y, float z,
+                                          float2 rho) {
+    return sample2_core<SAMP>(src, c, __ffma2_rn(c.t3, rho, f2(z, z)), __ffma2_rn(c.t1, rho, f2(x, x)),
+                              __ffma2_rn(c.t2, rho, f2(y, y)));
 }
 
 __device__ __forceinline__ Hom load_hom(const CostLaunch& a, int s) {
@@ -194,40 +193,46 @@ __device__ __forceinline__ Hom load_hom(const CostLaunch& a, int s) {
 // that starts from initReference (INC false) folds at most kMaxSources sources, so its divisors
 // never exceed 33 and only the dividends are tested.
 //
+// The state is held negated (-mean, -count): then the products and quotients below come out of pair operations
+// without negated operands, and rcp_neg2 of -(cnt + 1) is 1 / (cnt + 1).
+//
 // The FP16 form (APPROX) stores the result in FP16, so it folds with one multiply by RN(1/9)
 // and the hardware reciprocal estimate of cnt+1 (relative error ~1e-7, far below FP16's
 // 4.9e-4) instead of the correctly rounded divisions.
 template <bool INC, bool APPROX>
 __device__ __forceinline__ void fold2(float2& acc, float2& cn, float2 tmp, float r9) {
     const float2 r9p = f2(r9, r9);
+    const float2 n1 = __fadd2_rn(cn, f2(-1.0f, -1.0f));   // -(cnt + 1)
+    float2 q;
     if constexpr (APPROX) {
-        const float2 n1 = __fadd2_rn(cn, f2(1.0f, 1.0f));
         float2 r;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(n1.x));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(n1.y));
-        const float2 q = __fmul2_rn(__ffma2_rn(cn, acc, __fmul2_rn(tmp, r9p)), r);
-        const bool v0 = tmp.x == tmp.x, v1 = tmp.y == tmp.y;
-        acc = f2(v0 ? q.x : acc.x, v1 ? q.y : acc.y);
-        cn = f2(v0 ? n1.x : cn.x, v1 ? n1.y : cn.y);
-        return;
-    }
-    const float2 n1 = __fadd2_rn(cn, f2(1.0f, 1.0f));
-    const float2 nn1 = __ffma2_rn(cn, f2(-1.0f, -1.0f), f2(-1.0f, -1.0f));   // -(cnt + 1), exact
-    const float2 q0 = __fmul2_rn(tmp, r9p);
-    const float2 m = __ffma2_rn(__ffma2_rn(q0, f2(-9.0f, -9.0f), tmp), r9p, q0);
-    const float2 num = __ffma2_rn(cn, acc, m);
-    const float2 r = rcp_warp2(n1);
-    const float2 p0 = __fmul2_rn(num, r);
-    float2 q = __ffma2_rn(__ffma2_rn(p0, nn1, num), r, p0);
-    const bool fast = (!INC || (n1.x <= 33.0f && n1.y <= 33.0f)) && !(tmp.x != 0.0f && tmp.x < 1e-30f) &&
-                      !(tmp.y != 0.0f && tmp.y < 1e-30f) && !(num.x != 0.0f && num.x < 1e-30f) &&
-                      !(num.y != 0.0f && num.y < 1e-30f);
-    if (!fast) {
-        q.x = __fdiv_rn(__fmaf_rn(cn.x, acc.x, __fdiv_rn(tmp.x, 9.0f)), n1.x);
-        q.y = __fdiv_rn(__fmaf_rn(cn.y, acc.y, __fdiv_rn(tmp.y, 9.0f)), n1.y);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(-n1.x));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(-n1.y));
+        q = __fmul2_rn(__ffma2_rn(cn, acc, __fmul2_rn(tmp, r9p)), r);
+    } else {
+        const float2 q0 = __fmul2_rn(tmp, r9p);
+        const float2 m = __ffma2_rn(__ffma2_rn(q0, f2(-9.0f, -9.0f), tmp), r9p, q0);
+        const float2 num = __ffma2_rn(cn, acc, m);   // cnt * mean + tmp / 9
+        const float2 r = rcp_neg2(n1);
+        const float2 p0 = __fmul2_rn(num, r);
+        q = __ffma2_rn(__ffma2_rn(p0, n1, num), r, p0);
+        // A pass from initReference holds means of measured (>= 0) sums, so a sum of 1e-29 or more makes num at
+        // least a ninth of it; smaller sums (0 among them) are looked at one by one.
+        bool slow;
+        if constexpr (INC) slow = true;
+        else slow = tmp.x < 1e-29f || tmp.y < 1e-29f;
+        if (slow) {
+            const bool fast = (!INC || (n1.x >= -33.0f && n1.y >= -33.0f)) && !(tmp.x != 0.0f && tmp.x < 1e-30f) &&
+                              !(tmp.y != 0.0f && tmp.y < 1e-30f) && !(num.x != 0.0f && num.x < 1e-30f) &&
+                              !(num.y != 0.0f && num.y < 1e-30f);
+            if (!fast) {
+                q.x = __fdiv_rn(__fmaf_rn(cn.x, acc.x, __fdiv_rn(tmp.x, 9.0f)), -n1.x);
+                q.y = __fdiv_rn(__fmaf_rn(cn.y, acc.y, __fdiv_rn(tmp.y, 9.0f)), -n1.y);
+            }
+        }
     }
     const bool v0 = tmp.x == tmp.x, v1 = tmp.y == tmp.y;
-    acc = f2(v0 ? q.x : acc.x, v1 ? q.y : acc.y);
+    acc = f2(v0 ? -q.x : acc.x, v1 ? -q.y : acc.y);
     cn = f2(v0 ? n1.x : cn.x, v1 ? n1.y : cn.y);
 }
 
@@ -290,15 +295,15 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
                 if constexpr (HALF) c0 = __fadd_rn(c0, a.offset[(size_t)gy * W + gx]);
                 n0 = a.cnt[g];
             }
-            accs[p * SP + k] = c0;
-            cnts[p * SP + k] = (CntT)n0;
+            accs[p * SP + k] = -c0;   // the state is held negated (fold2)
+            cnts[p * SP + k] = (CntT)-n0;
         }
     } else {
-        // the whole arrays, pitch padding included, in 16-byte stores: -1 (FP16 form: a sum of
-        // 0) and a count of 0, whose FP32 and FP16 bit patterns are both zero
+        // the whole arrays, pitch padding included, in 16-byte stores: -1, negated (FP16 form: a sum of
+        // 0), and a count of 0, whose FP32 and FP16 bit patterns are both zero
         static_assert((NPIX * SP * sizeof(float)) % 16 == 0 && (NPIX * SP * sizeof(CntT)) % 16 == 0 &&
                           SM::ACC % 16 == 0 && SM::CNT % 16 == 0, "16-byte state stores");
-        const float c0 = HC ? 0.0f : -1.0f;
+        const float c0 = HC ? 0.0f : 1.0f;
         float4* const av = reinterpret_cast<float4*>(accs);
         for (int i = tid; i < NPIX * SP / 4; i += NT) av[i] = make_float4(c0, c0, c0, c0);
         float4* const cv = reinterpret_cast<float4*>(cnts);
@@ -317,20 +322,24 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
 
     for (int s = 0; s < a.nsrc; ++s) {
         Src<SAMP> src;
-        if constexpr (SAMP == kQuad || SAMP == kQuadH) {
-            src.q = a.srcq + (size_t)s * W * H;
-            src.off = 0x4B400000u * (unsigned)(W + 1);
-        } else if constexpr (SAMP == kTex || SAMP == kTexF) {
+        if constexpr (SAMP == kTex || SAMP == kTexF) {
             src.t = a.tex[s];
         } else {
-            src.p = a.srcs + (size_t)s * W * H;
+            src.M = a.floor_bias;
+            src.off = __float_as_uint(src.M) * (unsigned)(W + 1);
+            if constexpr (SAMP == kPlain) {
+                src.base = reinterpret_cast<const char*>(a.srcs + (size_t)s * W * H) - (size_t)src.off * 4;
+            } else {
+                src.base = reinterpret_cast<const char*>(a.srcq + s * quad_stride((size_t)W * H)) - (size_t)src.off * 16;
+                src.rej = src.off + (unsigned)W * (unsigned)H;
+            }
         }
         src.W = W;
         src.H = H;
         const Hom h = load_hom(a, s);
         WarpConst c;
-        c.t1 = f2(h.t1, h.t1);
-        c.t2 = f2(h.t2, h.t2);
+        c.t1 = kExact<SAMP> ? f2(-h.t1, -h.t1) : f2(h.t1, h.t1);
+        c.t2 = kExact<SAMP> ? f2(-h.t2, -h.t2) : f2(h.t2, h.t2);
         c.t3 = f2(h.t3, h.t3);
         c.W1 = (float)(W - 1);
         c.H1 = (float)(H - 1);
@@ -368,19 +377,23 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
         // columns (L / R); row r (down) is computed in the iteration
         float2 Su = f2(0.0f, 0.0f), Sc = Su, Lu = Su, Lc = Su, Ru = Su, Rc = Su;
         float hxc = 0.0f;
+        const float fx = (float)x, fy0 = (float)(y0 - 1);
 #pragma unroll   // unrolled, the rolling row registers are renamed instead of copied
         for (int r = 0; r < TY + 2; ++r) {
             float hx = 0.0f;   // the row's homogeneous x: MODE 0's neighbours of the next output row
             float2 Sd;
             if constexpr (PM) {
-                const float fy = (float)(y0 - 1 + r);
+                const float fy = __fadd_rn(fy0, (float)r);
                 const float2 yy = f2(fy, fy);
                 Sd = sample2_core<SAMP>(src, c, __ffma2_rn(R32, yy, A3), __ffma2_rn(R12, yy, A1),
                                         __ffma2_rn(R22, yy, A2));
                 if constexpr (MODE == 0) hx = __fmaf_rn(h.r12, fy, Xc);
             } else {
-                float hy, hz;
-                homog(h, x, y0 - 1 + r, hx, hy, hz);
+                // r11*x + r12*y + r13 and the y and z rows; x and y negated
+                const float fy = __fadd_rn(fy0, (float)r);
+                hx = __fmaf_rn(-h.r11, fx, -__fmaf_rn(h.r12, fy, h.r13));
+                const float hy = __fmaf_rn(-h.r21, fx, -__fmaf_rn(h.r22, fy, h.r23));
+                const float hz = __fmaf_rn(h.r31, fx, __fmaf_rn(h.r32, fy, h.r33));
                 Sd = sample2<SAMP>(src, c, hx, hy, hz, rho);
             }
             const float2 Ld = shfl_up2(Sd), Rd_ = shfl_down2(Sd);
@@ -399,8 +412,9 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
                         B4 = sample2_core<SAMP>(src, c, __fadd2_rn(xc, B3), __fadd2_rn(xc, B1), __fadd2_rn(xc, B2));
                         B8 = sample2_core<SAMP>(src, c, __fadd2_rn(xc, C3), __fadd2_rn(xc, C1), __fadd2_rn(xc, C2));
                     } else {
-                        const float xr = __fadd_rn(hxc, h.r11), yr = __fadd_rn(hxc, h.r21), zr = __fadd_rn(hxc, h.r31);
-                        const float xru = __fsub_rn(xr, h.r12), yru = __fsub_rn(xr, h.r22), zru = __fsub_rn(xr, h.r32);
+                        // hxc = -x: x + r11, x + r21 negated, x + r31; then those minus r12, r22 and r32
+                        const float xr = __fsub_rn(hxc, h.r11), yr = __fsub_rn(hxc, h.r21), zr = __fsub_rn(h.r31, hxc);
+                        const float xru = __fadd_rn(xr, h.r12), yru = __fadd_rn(xr, h.r22), zru = __fsub_rn(-h.r32, xr);
                         B4 = sample2<SAMP>(src, c, xr, yr, zr, rho);
                         B8 = sample2<SAMP>(src, c, xru, yru, zru, rho);
                     }
@@ -471,9 +485,14 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
             n[0] = n01.x; n[1] = n01.y; n[2] = n23.x; n[3] = n23.y;
         }
         float v[4] = {s01.x, s01.y, s23.x, s23.y};
-        if constexpr (HC) {   // sums and counts to means
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = sum_to_mean(v[j], n[j]);
+        for (int j = 0; j < 4; ++j) {
+            if constexpr (HC) {   // sums and counts to means
+                v[j] = sum_to_mean(v[j], n[j]);
+            } else {              // held negated
+                v[j] = -v[j];
+                n[j] = __fsub_rn(0.0f, n[j]);
+            }
         }
         const bool in = gx < W && gy < H && PM_RANGE_IN_BOUNDS(g, 4, (long long)W * H * D, kSiteCostState);
         if constexpr (HALF) {

@@ -287,7 +287,7 @@ constexpr int kMaxDiffSources = 4;
 
 struct CostBwdArgs {
     const float* ref;
-    const float4* quads;      // S x N: the cost kernel's source quads
+    const float4* quads;      // S slots: the cost kernel's source quads
     const float* gC[4];       // nv volumes whose sum is the costs' adjoint but for the 1 / count
     int nv;
     const double* count;      // pixels in the loss
@@ -440,7 +440,7 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
     const bool in_q = lane >= 2 && lane < 2 + BQX;
     const float rfx = 1.0f / A.fx, rfy = 1.0f / A.fy;
     for (int s = 0; s < A.S; ++s) {
-        const float4* const quads = A.quads + (size_t)s * W * H;
+        const float4* const quads = A.quads + s * quad_stride((size_t)W * H);
         float* const gi = A.gI + (size_t)s * W * H;
         float gp[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         Pending pend[2] = {{0u, 0.0f, 0.0f}, {0u, 0.0f, 0.0f}};
@@ -692,7 +692,7 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
         ok = cudaMalloc(p, b) == cudaSuccess;
         d->bytes += b;
     };
-    alloc((void**)&d->quads, 16 * d->N * c->num_sources);
+    alloc((void**)&d->quads, 16 * quad_stride(d->N) * c->num_sources);
     alloc((void**)&d->C, 4 * d->V);
     alloc((void**)&d->invalid, d->N);
     // store_paths, and volumes of up to 4 MB, whose steps are bound by the recurrences' latency: 7 volumes
@@ -704,6 +704,7 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     alloc((void**)&d->codes, 8 * d->N * 4 * words);
     alloc((void**)&d->sums, 2 * sizeof(double));
     alloc((void**)&d->gP, 6 * sizeof(double) * c->num_sources);
+    ok = ok && init_quad_slots(d->quads, d->N, c->num_sources, 0) == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         free_diff(d);
@@ -757,7 +758,7 @@ pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const
     d->cam[3] = (float)K[5];
     const dim3 qg((W + 255) / 256, H);
     for (int s = 0; s < S; ++s)
-        to_quad_f_kernel<<<qg, 256, 0, st>>>(W, H, srcs + (size_t)s * d->N, d->quads + (size_t)s * d->N);
+        to_quad_f_kernel<<<qg, 256, 0, st>>>(W, H, srcs + (size_t)s * d->N, d->quads + s * quad_stride(d->N));
     PD_CK(d, cudaGetLastError());
     CostLaunch a;
     std::memset(&a, 0, sizeof a);
@@ -770,6 +771,7 @@ pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const
     a.rho0 = c.rho0;
     a.drho = c.rho_step;
     a.mode = PM_COST_CORRECTED;
+    set_floor_bias(a);
     for (int s = 0; s < S; ++s)
         for (int i = 0; i < 12; ++i) a.hom[s][i] = d->hom[s][i];
     a.cost = d->C;

@@ -76,11 +76,17 @@ __device__ __forceinline__ float rcp_rn(float w) {
 // to RN(1/w) for 2^-126 <= |w| <= 2^126 (as rcp_rn); NaN for w = +-0, subnormal, infinite or NaN
 // w (a warped sample from such a w is rejected); +-0 for larger finite |w|.  The FP32 oracle
 // implements exactly this rule; pm_debug_check_arith checks it for every float.
-__device__ __forceinline__ float2 rcp_warp2(float2 w) {
+// rcp_neg2 gives the negated reciprocals -1/w: with r0 = rcp(-w), the step r0 + r0 (1 + w r0) needs no
+// negated pair operand (the estimate is odd in w, and every operation rounds symmetrically).
+__device__ __forceinline__ float2 rcp_neg2(float2 w) {
     float2 r0;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0.x) : "f"(w.x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0.y) : "f"(w.y));
-    return __ffma2_rn(r0, __ffma2_rn(make_float2(-w.x, -w.y), r0, make_float2(1.0f, 1.0f)), r0);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0.x) : "f"(-w.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0.y) : "f"(-w.y));
+    return __ffma2_rn(r0, __ffma2_rn(w, r0, make_float2(1.0f, 1.0f)), r0);
+}
+__device__ __forceinline__ float2 rcp_warp2(float2 w) {
+    const float2 r = rcp_neg2(w);
+    return make_float2(-r.x, -r.y);
 }
 
 // floor(u) for 0 <= u < 2^22 as (float, int) without a conversion instruction: adding
@@ -98,47 +104,6 @@ __device__ __forceinline__ float div_small(float x, float d, float r) {
     if (x != 0.0f && x < 1e-30f) return __fdiv_rn(x, d);
     const float q0 = __fmul_rn(x, r);
     return __fmaf_rn(__fmaf_rn(-q0, d, x), r, q0);
-}
-
-__device__ __forceinline__ void homog(const Hom& h, int qu, int qv, float& x, float& y, float& z) {
-    const float fu = (float)qu, fv = (float)qv;
-    x = __fmaf_rn(h.r11, fu, __fmaf_rn(h.r12, fv, h.r13));
-    y = __fmaf_rn(h.r21, fu, __fmaf_rn(h.r22, fv, h.r23));
-    z = __fmaf_rn(h.r31, fu, __fmaf_rn(h.r32, fv, h.r33));
-}
-
-// Bilinear fetch with texel centres at integer coordinates and zero border, the filtering of
-// tex2D(t, u + 0.5f, v + 0.5f) with cudaFilterModeLinear / cudaAddressModeBorder
-// (calc_cost.cu:93,230-237), evaluated with exact weights.  Caller guarantees
-// 0 <= u <= W-1 and 0 <= v <= H-1, so only the +1 texels can fall outside.
-__device__ __forceinline__ float bilinear(const float* __restrict__ img, int W, int H, float u, float v) {
-    const float fu = floorf(u), fv = floorf(v);
-    const int i = (int)fu, j = (int)fv;
-    const float a = __fsub_rn(u, fu), b = __fsub_rn(v, fv);
-    const float* row0 = img + (size_t)j * W;
-    const bool in_i1 = (i + 1) < W, in_j1 = (j + 1) < H;
-    const float t00 = __ldg(row0 + i);
-    const float t10 = in_i1 ? __ldg(row0 + i + 1) : 0.0f;
-    const float t01 = in_j1 ? __ldg(row0 + W + i) : 0.0f;
-    const float t11 = (in_i1 && in_j1) ? __ldg(row0 + W + i + 1) : 0.0f;
-    const float top = __fmaf_rn(a, __fsub_rn(t10, t00), t00);
-    const float bot = __fmaf_rn(a, __fsub_rn(t11, t01), t01);
-    return __fmaf_rn(b, __fsub_rn(bot, top), top);
-}
-
-// One warped sample (calc_cost.cu:85-93): w = z + t3*rho, u = (x + t1*rho)/w, v = (y + t2*rho)/w,
-// computed as one correctly rounded reciprocal and two products.  Rejected samples (w < 0 or
-// (u, v) outside [0, W-1] x [0, H-1], NaN included) return NaN, which then poisons the 9-term sum.
-__device__ __forceinline__ float warp_fetch(const float* __restrict__ img, int W, int H, float x, float y,
-                                            float z, const Hom& h, float rho) {
-    const float w = __fmaf_rn(h.t3, rho, z);
-    const float nx = __fmaf_rn(h.t1, rho, x);
-    const float ny = __fmaf_rn(h.t2, rho, y);
-    const float r = rcp_rn(w);
-    const float u = __fmul_rn(nx, r), v = __fmul_rn(ny, r);
-    const bool ok = (w >= 0.0f) && (u >= 0.0f) && (u <= (float)(W - 1)) && (v >= 0.0f) &&
-                    (v <= (float)(H - 1));
-    return ok ? bilinear(img, W, H, u, v) : nan_f();
 }
 
 // ---- warp reductions --------------------------------------------------------------------

@@ -47,9 +47,10 @@ enum BoundsSite {
 struct CostLaunch {
     const float* ref;      // W*H scaled reference image
     const float* srcs;     // nsrc consecutive W*H scaled source images (used when srcq is null)
-    // nsrc consecutive W*H quad images (2x2 bilinear footprints); in the FP16 form (cost_half)
+    // nsrc slots of quad_stride(W*H) quads (2x2 bilinear footprints); in the FP16 form (cost_half)
     // their values are rounded to FP16
     const float4* srcq;
+    float floor_bias;      // see Src in cost_device.cuh; set_floor_bias
     // use_tex: the sources through these texture objects (pitched images, linear filtering, zero
     // border; FP16 form: FP16 or FP16-rounded FP32 texels, FP32 form: FP32 texels)
     unsigned long long tex[kMaxSources];
@@ -74,6 +75,12 @@ struct CostLaunch {
     int incremental;       // start from (cost, cnt) in memory instead of (-1, 0)
     cudaEvent_t kernel_done = nullptr;   // recorded right after the cost kernel (before the rebase)
 };
+// An integer M in [2^23, 1.5 * 2^23] whose bits(M) * (W + 1), modulo 2^32, plus W*H stays below 2^32.
+void set_floor_bias(CostLaunch& a);
+// A source's quads are followed by one quad of NaN, which rejected samples read: quads per source slot, and the
+// fill of the NaN quads of `slots` slots.
+constexpr size_t quad_stride(size_t npix) { return npix + 1; }
+cudaError_t init_quad_slots(float4* q, size_t npix, int slots, cudaStream_t s);
 cudaError_t launch_cost(const CostLaunch& a, cudaStream_t s);
 
 // ---- SGM aggregation + winner-take-all (sgm.cu, filter_cost.cu) ---------------------------
