@@ -16,14 +16,23 @@
 //     the plane-innermost layout (cuda_utils.h:34).
 // Source frames are "quads": pixel (x, y) holds I(x,y), I(x,y+1), I(x+1,y), I(x+1,y+1) with the
 // texture border (zero) applied, so a bilinear sample is one aligned 16-byte load whose halves
-// are the packed operands of the horizontal interpolation; rejected samples read a quad of NaN.  floor()
-// adds an integer of at least 2^23 with round-toward-minus-infinity, leaving the integer part in the mantissa;
-// the reciprocal is
-// rcp.approx plus one Newton step without a range branch (rcp_warp2: RN(1/w) wherever an
-// image-sized scene puts w, a stated value elsewhere); the divisions of the running mean are a
-// reciprocal-multiply with one FMA correction.  Each is checked over every float against its
-// definition (pm_debug_check_arith), and every packed instruction rounds each element like its
-// scalar counterpart, so the FP32 oracle's scalar algorithm reproduces the volume bit for bit.
+// are the packed operands of the horizontal interpolation; rejected samples read a quad of NaN.
+// floor() adds an integer of at least 2^23 with round-toward-minus-infinity, leaving the integer
+// part in the mantissa; the reciprocal is rcp.approx plus one Newton step without a range branch
+// (rcp_warp2: RN(1/w) wherever an image-sized scene puts w, a stated value elsewhere); the divisions
+// of the running mean are a reciprocal-multiply with one FMA correction.  Each is checked over every
+// float against its definition (pm_debug_check_arith), and every packed instruction rounds each
+// element like its scalar counterpart, so the FP32 oracle's scalar algorithm reproduces the volume
+// bit for bit.
+//
+// Bound by issue, the FMA pipe (a packed operation takes it for two cycles) and the L1 data path
+// together: 66, 64 and 72 % at 640x480x128 with 5 sources, FP32, reference mode.  So signs are
+// arranged such that no pair operand is negated on its own, a tile's reference values roll through
+// registers (three shared-memory reads per row instead of nine), and the exact division's range is
+// looked at only where a sum is tiny: 1.110 -> 1.040 ms in reference mode, 0.711 -> 0.635 in corrected
+// mode (texture sampler 0.839 -> 0.770 and 0.593 -> 0.537; FP16 form with the exact sampler 0.913 ->
+// 0.832 and 0.661 -> 0.498, with the texture sampler at 752x480x128 0.807 -> 0.810, bound by its
+// fetches, and 0.536 -> 0.450).
 #include <cstring>
 
 #include "cost_device.cuh"

@@ -23,8 +23,8 @@ constexpr int NPIX = TXU * TY;
 // small integers, exact in FP16): fewer shared bytes per CTA leave more of the SM's L1 to the
 // texture cache, which the texture samplers' speed depends on.
 template <bool HC> struct SmemL {
-    static constexpr size_t REF = 0;                                              // float2 [TY+2][32]
-    static constexpr size_t ACC = REF + sizeof(float2) * (TY + 2) * 32;           // float [NPIX][SP]
+    static constexpr size_t REF = 0;                                              // float [TY+2][32]
+    static constexpr size_t ACC = REF + sizeof(float) * (TY + 2) * 32;           // float [NPIX][SP]
     static constexpr size_t CNT = ACC + sizeof(float) * NPIX * SP;                // float or half [NPIX][SP]
     static constexpr size_t BYTES = CNT + (HC ? sizeof(__half) : sizeof(float)) * NPIX * SP;
 };
@@ -47,6 +47,9 @@ template <bool HALF> __device__ __forceinline__ float load_cost(const void* base
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 // a - b as fma(b, -1, a): the product is exact, so this is RN(a - b) without a negation
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.0f, -1.0f), a); }
+
+// r - s at both planes
+__device__ __forceinline__ float2 diff2(float r, float2 s) { return sub2(f2(r, r), s); }
 
 __device__ __forceinline__ float2 shfl_up2(float2 v) {
     return f2(__shfl_up_sync(kFull, v.x, 1), __shfl_up_sync(kFull, v.y, 1));
@@ -263,7 +266,7 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
     constexpr bool PM = HALF;           // packed-pair warp coordinates (see the source loop)
     using SM = SmemL<HC>;
     using CntT = typename std::conditional<HC, __half, float>::type;
-    float2* const refp = reinterpret_cast<float2*>(smem_raw + SM::REF);
+    float* const refp = reinterpret_cast<float*>(smem_raw + SM::REF);
     float* const accs = reinterpret_cast<float*>(smem_raw + SM::ACC);
     CntT* const cnts = reinterpret_cast<CntT*>(smem_raw + SM::CNT);
 
@@ -272,13 +275,12 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
     const int x0 = bx * TXU, y0 = by * TY, d0 = bz * PCB;
     const int x = x0 - 1 + lane;                              // this lane's column
     const bool out_col = lane >= 1 && lane <= TXU && x < W;   // an output column of the tile
+    const int lane_l = lane > 0 ? lane - 1 : 0, lane_r = lane < 31 ? lane + 1 : 31;
 
-    // reference tile + halo (border addressing -> 0, calc_cost.cu:230-231), each value
-    // duplicated as the packed operand of both planes
+    // reference tile + halo (border addressing -> 0, calc_cost.cu:230-231)
     for (int i = tid; i < (TY + 2) * 32; i += NT) {
         const int r = i >> 5, l = i & 31;
-        const float R = ref_at(a.ref, W, H, x0 - 1 + l, y0 - 1 + r);
-        refp[i] = f2(R, R);
+        refp[i] = ref_at(a.ref, W, H, x0 - 1 + l, y0 - 1 + r);
     }
 
     // running state of the tile's voxels, [pixel][plane] with pitch SP: from memory (the
@@ -377,6 +379,9 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
         // columns (L / R); row r (down) is computed in the iteration
         float2 Su = f2(0.0f, 0.0f), Sc = Su, Lu = Su, Lc = Su, Ru = Su, Rc = Su;
         float hxc = 0.0f;
+        // reference values of rows r-2, r-1 and r at the left, own and right column: rolling rows, so that a row
+        // costs three shared-memory reads
+        float rl[3] = {0.0f, 0.0f, 0.0f}, rm[3] = {0.0f, 0.0f, 0.0f}, rr[3] = {0.0f, 0.0f, 0.0f};
         const float fx = (float)x, fy0 = (float)(y0 - 1);
 #pragma unroll   // unrolled, the rolling row registers are renamed instead of copied
         for (int r = 0; r < TY + 2; ++r) {
@@ -397,12 +402,11 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
                 Sd = sample2<SAMP>(src, c, hx, hy, hz, rho);
             }
             const float2 Ld = shfl_up2(Sd), Rd_ = shfl_down2(Sd);
+            rl[2] = refp[r * 32 + lane_l];
+            rm[2] = refp[r * 32 + lane];
+            rr[2] = refp[r * 32 + lane_r];
             const int o = r - 2;   // output row y0 + o
             if (o >= 0 && out_col && y0 + o < H) {
-                const float2* rp = refp + o * 32 + lane;   // up row, this column
-                const float2 Ru_ = rp[0], Rc_ = rp[32], Rd = rp[64];
-                const float2 Rl = rp[31], Rr = rp[33];
-                const float2 Rul = rp[-1], Rru = rp[1], Rld = rp[63], Rdr = rp[65];
                 float2 d[9];
                 if constexpr (MODE == 0) {
                     // the corrupted neighbours (calc_cost.cu:49-51, 69-71) from the centre's x
@@ -418,25 +422,25 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
                         B4 = sample2<SAMP>(src, c, xr, yr, zr, rho);
                         B8 = sample2<SAMP>(src, c, xru, yru, zru, rho);
                     }
-                    d[0] = sub2(Rc_, Sc);    // 0  (:93)
-                    d[1] = sub2(Rd, Su);     // 1  warps (u, v-1), reads ref (u, v+1) (:106)
-                    d[2] = sub2(Ru_, Sd);    // 2  warps (u, v+1), reads ref (u, v-1) (:119)
-                    d[3] = sub2(Rl, Lc);     // 3  (:132)
-                    d[4] = sub2(Rr, B4);     // 4  (:145)
-                    d[5] = sub2(Rul, Lu);    // 5  (:159)
-                    d[6] = sub2(Rdr, Rd_);   // 6  (:172)
-                    d[7] = sub2(Rld, Ld);    // 7  (:185)
-                    d[8] = sub2(Rru, B8);    // 8  (:198)
+                    d[0] = diff2(rm[1], Sc);    // 0  (:93)
+                    d[1] = diff2(rm[2], Su);    // 1  warps (u, v-1), reads ref (u, v+1) (:106)
+                    d[2] = diff2(rm[0], Sd);    // 2  warps (u, v+1), reads ref (u, v-1) (:119)
+                    d[3] = diff2(rl[1], Lc);    // 3  (:132)
+                    d[4] = diff2(rr[1], B4);    // 4  (:145)
+                    d[5] = diff2(rl[0], Lu);    // 5  (:159)
+                    d[6] = diff2(rr[2], Rd_);   // 6  (:172)
+                    d[7] = diff2(rl[2], Ld);    // 7  (:185)
+                    d[8] = diff2(rr[0], B8);    // 8  (:198)
                 } else {
-                    d[0] = sub2(Rc_, Sc);
-                    d[1] = sub2(Ru_, Su);
-                    d[2] = sub2(Rd, Sd);
-                    d[3] = sub2(Rl, Lc);
-                    d[4] = sub2(Rr, Rc);
-                    d[5] = sub2(Rul, Lu);
-                    d[6] = sub2(Rdr, Rd_);
-                    d[7] = sub2(Rld, Ld);
-                    d[8] = sub2(Rru, Ru);
+                    d[0] = diff2(rm[1], Sc);
+                    d[1] = diff2(rm[0], Su);
+                    d[2] = diff2(rm[2], Sd);
+                    d[3] = diff2(rl[1], Lc);
+                    d[4] = diff2(rr[1], Rc);
+                    d[5] = diff2(rl[0], Lu);
+                    d[6] = diff2(rr[2], Rd_);
+                    d[7] = diff2(rl[2], Ld);
+                    d[8] = diff2(rr[0], Ru);
                 }
                 // the nine terms in the reference's order, both planes in one packed add each
                 float2 t2 = f2(fabsf(d[0].x), fabsf(d[0].y));
@@ -456,6 +460,9 @@ __device__ __forceinline__ void cost_tile(const CostLaunch& a, int bx, int by, i
             Lu = Lc; Lc = Ld;
             Ru = Rc; Rc = Rd_;
             hxc = hx;
+            rl[0] = rl[1]; rl[1] = rl[2];
+            rm[0] = rm[1]; rm[1] = rm[2];
+            rr[0] = rr[1]; rr[1] = rr[2];
         }
     }
 
