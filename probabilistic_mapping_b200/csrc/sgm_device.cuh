@@ -295,6 +295,7 @@ template <int PPL> __device__ __forceinline__ void add_h(float (&o)[PPL], const 
 // steps of the current batch (bit i: step k0 + i has a reference-image gradient below tau).
 template <int PPL> struct PathState {
     float L[PPL];
+    float below, above;   // the neighbour lanes' planes next to this lane's first and last (+inf at the ends)
     float mprev;
     unsigned qmask;
 };
@@ -345,13 +346,40 @@ template <int PPL, bool FULL> __device__ __forceinline__ bool pixel_invalid(cons
     return __any_sync(kFull, lane_min<PPL, FULL>(cv, incl) < 0.0f);
 }
 
-// First pixel of a path: L = C, or 0 on an invalid pixel (sgm.cu:21-43).
+// A pixel's costs as the path takes them (0 on an invalid pixel); returns whether the pixel is invalid.
 template <int PPL, bool FULL>
-__device__ __forceinline__ void path_first(PathState<PPL>& s, const float (&cv)[PPL], uint32_t incl, float (&o)[PPL]) {
+__device__ __forceinline__ bool path_costs(float (&cz)[PPL], const float (&cv)[PPL], uint32_t incl) {
     const bool inv = pixel_invalid<PPL, FULL>(cv, incl);
 #pragma unroll
-    for (int j = 0; j < PPL; ++j) s.L[j] = o[j] = inv ? 0.0f : cv[j];
+    for (int j = 0; j < PPL; ++j) cz[j] = inv ? 0.0f : cv[j];
+    return inv;
+}
+
+// What the next step needs of a path's new values from the other lanes: started as soon as the values are there,
+// so that their latency passes behind the other end's step, the stores and the next costs.  Up to four planes per
+// lane (kAhead): with more, and with records, the registers for it cost more warps than it gives (1280x720x192 FP16
+// 1764 -> 1789 us), and there the neighbour lanes' planes are fetched, and the costs read, where a step begins.
+template <int PPL, bool ROUTE> constexpr bool kAhead = PPL <= 4 && !ROUTE;
+template <int PPL>
+__device__ __forceinline__ void path_neighbours(PathState<PPL>& s, int lane) {
+    s.below = __shfl_up_sync(kFull, s.L[PPL - 1], 1);
+    s.above = __shfl_down_sync(kFull, s.L[0], 1);
+    if (lane == 0) s.below = inf_f();
+    if (lane == 31) s.above = inf_f();
+}
+template <int PPL, bool FULL, bool ROUTE>
+__device__ __forceinline__ void path_exchange(PathState<PPL>& s, uint32_t incl, int lane) {
+    if constexpr (kAhead<PPL, ROUTE>) path_neighbours<PPL>(s, lane);
     s.mprev = warp_min_f32(lane_min<PPL, FULL>(s.L, incl));
+}
+
+// First pixel of a path: L = C, or 0 on an invalid pixel (sgm.cu:21-43).
+template <int PPL, bool FULL, bool ROUTE>
+__device__ __forceinline__ void path_first(PathState<PPL>& s, const float (&cz)[PPL], uint32_t incl, int lane,
+                                           float (&o)[PPL]) {
+#pragma unroll
+    for (int j = 0; j < PPL; ++j) s.L[j] = o[j] = cz[j];
+    path_exchange<PPL, FULL, ROUTE>(s, incl, lane);
 }
 
 // The differentiation form's record of one step: which term of the minimum each plane took, as three
@@ -362,7 +390,6 @@ __device__ __forceinline__ void path_first(PathState<PPL>& s, const float (&cv)[
 template <int PPL> struct Route {
     static constexpr int WORDS = (3 * PPL + 1 + 3) / 4 * 4;   // whole 16-byte pieces
     uint32_t w[WORDS];
-    bool inv;   // the pixel has a plane that was never measured
 };
 // Where a pass with records puts them: path r's record of a pixel is record r * N + pixel; and the invalid
 // flag of every pixel (written by pair 0).  8 * N < 2^32.  Path r's values go to volume
@@ -383,28 +410,22 @@ template <int PPL> __device__ __forceinline__ void store_route(uint32_t* p, cons
 // One pixel step of a path (sgm.cu:57-108): L(p, d) = C(p, d) + min(L(p-r, d), L(p-r, d+-1) + P1,
 // min_k L(p-r, k) + P2) - min_k L(p-r, k), P1/P2 scaled by q1/q2 when the flag q says the
 // reference image's path gradient is below tau; a plane never measured makes the pixel invalid:
-// its cost counts as 0 and the path's output there is COST_INF = 0.  o receives the output.
+// its cost counts as 0 (cz) and the path's output there is COST_INF = 0.  o receives the output.
 // ROUTE: rt receives the step's record; equal terms resolve to the same plane, then to a neighbour (the
 // lower one first), then to the minimum.
 template <int PPL, bool FULL, bool ROUTE = false>
-__device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s, const float (&cv)[PPL], bool q,
-                                          float p1q, float p2q, uint32_t incl, int lane, float (&o)[PPL],
+__device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s, const float (&cz)[PPL], bool inv,
+                                          bool q, float p1q, float p2q, uint32_t incl, int lane, float (&o)[PPL],
                                           Route<PPL>* rt = nullptr) {
-    const bool inv = pixel_invalid<PPL, FULL>(cv, incl);
     const float P1 = q ? p1q : a.p1, P2 = q ? p2q : a.p2;
     const float mP2 = __fadd_rn(s.mprev, P2);
-    float lm = __shfl_up_sync(kFull, s.L[PPL - 1], 1);
-    float lp = __shfl_down_sync(kFull, s.L[0], 1);
-    if (lane == 0) lm = inf_f();
-    if (lane == 31) lp = inf_f();
+    if constexpr (!kAhead<PPL, ROUTE>) path_neighbours<PPL>(s, lane);
+    const float lm = s.below, lp = s.above;
     // min(L[d], minL + P2, L[d-1] + P1, L[d+1] + P1) (sgm.cu:85-92); min(a+P1, b+P1) is
     // min(a, b) + P1 exactly because rounding is monotonic
-    float nb[PPL], cz[PPL], vv[PPL];
+    float nb[PPL], vv[PPL];
 #pragma unroll
-    for (int j = 0; j < PPL; ++j) {
-        nb[j] = fminf(j == 0 ? lm : s.L[j - 1], j == PPL - 1 ? lp : s.L[j + 1]);
-        cz[j] = inv ? 0.0f : cv[j];
-    }
+    for (int j = 0; j < PPL; ++j) nb[j] = fminf(j == 0 ? lm : s.L[j - 1], j == PPL - 1 ? lp : s.L[j + 1]);
     add_planes<PPL>(nb, nb, P1);
 #pragma unroll
     for (int j = 0; j < PPL; ++j) vv[j] = min3f(s.L[j], mP2, nb[j]);
@@ -420,13 +441,12 @@ __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s,
         rt->w[3 * PPL] = __reduce_min_sync(kFull, at);
 #pragma unroll
         for (int i = 3 * PPL + 1; i < Route<PPL>::WORDS; ++i) rt->w[i] = 0u;
-        rt->inv = inv;
     }
     add_planes<PPL>(vv, cz, vv);               // C + val
     add_planes<PPL>(s.L, vv, -s.mprev);        // - minL (:98); the negation is exact
 #pragma unroll
     for (int j = 0; j < PPL; ++j) o[j] = inv ? 0.0f : s.L[j];
-    s.mprev = warp_min_f32(lane_min<PPL, FULL>(s.L, incl));
+    path_exchange<PPL, FULL, ROUTE>(s, incl, lane);
 }
 
 // Reference intensity of step k of a chain starting at pixel p0 (0 past its end).
@@ -554,15 +574,27 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
             store_route<PPL>(ro->codes + (size_t)((unsigned)path * (unsigned)npix + (unsigned)pix) * Route<PPL>::WORDS, r);
     };
 
+    // the costs of the coming step, read and tested one step ahead (kAhead)
+    constexpr bool AHEAD = kAhead<PPL, ROUTE>;
+    float czf[PPL], czb[PPL];
+    bool invf, invb;
+    auto slices = [&](const unsigned char* sb, float (&cf)[PPL], float (&cb)[PPL]) {
+        load_slice<PPL, HALF>(cf, sb + lane * CB);
+        load_slice<PPL, HALF>(cb, sb + CHAIN_B + lane * CB);
+    };
+
     // step 0: the first pixel of both paths
-    cp_async_wait<PF - 1>();
+    cp_async_wait<PF - 2>();
     {
         float cf[PPL], cb[PPL], of[PPL], ob[PPL];
-        load_slice<PPL, HALF>(cf, wbase + lane * CB);
-        load_slice<PPL, HALF>(cb, wbase + CHAIN_B + lane * CB);
-        if constexpr (ROUTE) rinv = pixel_invalid<PPL, FULL>(cf, incl) ? 1u : 0u;
-        path_first<PPL, FULL>(fs, cf, incl, of);
-        path_first<PPL, FULL>(bs, cb, incl, ob);
+        [[maybe_unused]] float nf[PPL], nb[PPL];
+        slices(wbase, cf, cb);
+        if constexpr (AHEAD) slices(wbase + STAGE_B, nf, nb);   // (past a scanline of one pixel: not used)
+        invf = path_costs<PPL, FULL>(czf, cf, incl);
+        path_costs<PPL, FULL>(czb, cb, incl);
+        if constexpr (ROUTE) rinv = invf ? 1u : 0u;
+        path_first<PPL, FULL, ROUTE>(fs, czf, incl, lane, of);
+        path_first<PPL, FULL, ROUTE>(bs, czb, incl, lane, ob);
         if constexpr (ROUTE) {
             if (n == 1 && slot == 0) flush_invalid(0);
         }
@@ -575,8 +607,13 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         }
         if (PF < n) issue(wbase, PF);
         cp_async_commit();
+        if constexpr (AHEAD) {
+            invf = path_costs<PPL, FULL>(czf, nf, incl);
+            invb = path_costs<PPL, FULL>(czb, nb, incl);
+        }
     }
-    int st = PF > 1 ? 1 : 0;
+    static_assert(PF > 2, "the ring holds the step after next");
+    int st = 1;
 
     // steps 1 .. n-1: the first visits (stores), the meeting pixel of an odd chain, then the
     // second visits (reductions)
@@ -591,30 +628,37 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
             fs.qmask = penalty_flags(If, Ifn, a.ref, pf0, step, k, n, lane, a.tau, lastf, npix);
             bs.qmask = penalty_flags(Ib, Ibn, a.ref, pb0, -step, k, n, lane, a.tau, lastb, npix);
         }
-        cp_async_wait<PF - 1>();
-        unsigned char* sb = wbase + st * STAGE_B;
-        float cf[PPL], cb[PPL];
-        load_slice<PPL, HALF>(cf, sb + lane * CB);
-        load_slice<PPL, HALF>(cb, sb + CHAIN_B + lane * CB);
+        cp_async_wait<AHEAD ? PF - 2 : PF - 1>();
+        const int nst = st + 1 == PF ? 0 : st + 1;
+        float nf[PPL], nb[PPL];
+        slices(wbase + (AHEAD ? nst : st) * STAGE_B, nf, nb);
+        if constexpr (!AHEAD) {
+            invf = path_costs<PPL, FULL>(czf, nf, incl);
+            invb = path_costs<PPL, FULL>(czb, nb, incl);
+        }
         const int bit = k & 31;
         if constexpr (ROUTE) {
             Route<PPL> r;
-            path_step<PPL, FULL, true>(a, fs, cf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of, &r);
+            path_step<PPL, FULL, true>(a, fs, czf, invf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of, &r);
             put_route(slot, pf, r);
             if (slot == 0) {
-                rinv = (bit == 0 ? 0u : rinv) | (r.inv ? 1u << bit : 0u);
+                rinv = (bit == 0 ? 0u : rinv) | (invf ? 1u << bit : 0u);
                 if (bit == 31 || k == n - 1) flush_invalid(k);
             }
-            path_step<PPL, FULL, true>(a, bs, cb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob, &r);
+            path_step<PPL, FULL, true>(a, bs, czb, invb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob, &r);
             put_route(slot + 1, pb, r);
         } else {
-            path_step<PPL, FULL>(a, fs, cf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of);
-            path_step<PPL, FULL>(a, bs, cb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob);
+            path_step<PPL, FULL>(a, fs, czf, invf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of);
+            path_step<PPL, FULL>(a, bs, czb, invb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob);
         }
-        // refill this stage (consumed above) with step k + PF
-        if (k + PF < n) issue(sb, k + PF);
+        // refill this step's stage (its costs are in registers) with step k + PF
+        if (k + PF < n) issue(wbase + st * STAGE_B, k + PF);
         cp_async_commit();
-        st = (st + 1 == PF) ? 0 : st + 1;
+        if constexpr (AHEAD) {
+            invf = path_costs<PPL, FULL>(czf, nf, incl);
+            invb = path_costs<PPL, FULL>(czb, nb, incl);
+        }
+        st = nst;
     };
     const int half = n >> 1;   // steps k < half are first visits of both ends
 #pragma unroll 1
