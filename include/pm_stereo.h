@@ -337,6 +337,12 @@ PM_API pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs
 /* Gradients of the last forward's loss: grad_srcs (device, num_sources*W*H, overwritten) and
  * grad_pose (host, 6 per source: omega then upsilon). */
 PM_API pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void* stream);
+/* The same without waiting for the stream: loss (one double) and grad_pose are device memory, written when
+ * `stream` gets there. */
+PM_API pm_status pm_diff_forward_async(pm_diff* d, const float* ref, const float* srcs, const double K[9],
+                                       const double* R, const double* t, const float* rho_gt, float* rho_hat,
+                                       double* loss, void* stream);
+PM_API pm_status pm_diff_backward_async(pm_diff* d, float* grad_srcs, double* grad_pose, void* stream);
 PM_API const char* pm_diff_last_error(const pm_diff* d);
 
 /* ---------------------------------------------------------------------------------------

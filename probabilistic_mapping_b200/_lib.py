@@ -143,6 +143,8 @@ SIGNATURES = {
     "pm_diff_memory": (_I, [_VP, _P(_SZ)]),
     "pm_diff_forward": (_I, [_VP, _VP, _VP, _D, _D, _D, _VP, _VP, _D, _VP]),
     "pm_diff_backward": (_I, [_VP, _VP, _D, _VP]),
+    "pm_diff_forward_async": (_I, [_VP, _VP, _VP, _D, _D, _D, _VP, _VP, _VP, _VP]),
+    "pm_diff_backward_async": (_I, [_VP, _VP, _VP, _VP]),
     "pm_diff_last_error": (ctypes.c_char_p, [_VP]),
     "pm_pyr_down_u8": (_I, [_I, _I, _VP, _SZ, _VP, _SZ, _VP]),
     "pm_depth_up2": (_I, [_I, _I, _VP, _SZ, _VP, _SZ, _VP]),

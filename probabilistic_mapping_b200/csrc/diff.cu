@@ -213,7 +213,8 @@ struct SoftArgs {
     const uint8_t* invalid;
     float* rho_hat;           // optional
     float* gS;                // adjoint of the sum, without the 1 / count of the loss's mean
-    double* sums;             // loss sum, count
+    double* sums;             // loss sum, count, and the number of finished blocks (cleared before the launch)
+    double* loss;             // their quotient, written by the last block (optional)
     int N, D;
     float rho0, drho, T;
 };
@@ -279,6 +280,14 @@ __global__ void __launch_bounds__(256) soft_kernel(const SoftArgs a) {
         if (count) {
             atomicAdd(a.sums, loss);
             atomicAdd(a.sums + 1, (double)count);
+        }
+        if (a.loss) {
+            __threadfence();
+            if (atomicAdd(reinterpret_cast<unsigned*>(a.sums + 2), 1u) == gridDim.x - 1) {
+                __threadfence();
+                const volatile double* sums = a.sums;
+                *a.loss = sums[1] > 0.0 ? sums[0] / sums[1] : 0.0;
+            }
         }
     }
 }
@@ -603,7 +612,7 @@ struct pm_diff {
     bool wide = false;        // a volume for each term of the paths' sum (7) instead of 3
     float* vol = nullptr;     // forward: the paths' values; backward: the pairs' adjoints
     uint32_t* codes = nullptr;   // 8 paths' records, N each
-    double* sums = nullptr;   // [loss sum, valid count]
+    double* sums = nullptr;   // [loss sum, valid count, finished blocks]
     double* gP = nullptr;     // S x 6
     // inputs of the last forward
     const float* ref = nullptr;
@@ -702,7 +711,7 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     const int ppl = c->num_planes / 32;
     const size_t words = ppl == 1 ? Route<1>::WORDS : ppl == 2 ? Route<2>::WORDS : ppl == 4 ? Route<4>::WORDS : Route<8>::WORDS;
     alloc((void**)&d->codes, 8 * d->N * 4 * words);
-    alloc((void**)&d->sums, 2 * sizeof(double));
+    alloc((void**)&d->sums, 3 * sizeof(double));
     alloc((void**)&d->gP, 6 * sizeof(double) * c->num_sources);
     ok = ok && init_quad_slots(d->quads, d->N, c->num_sources, 0) == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
     if (!ok) {
@@ -729,17 +738,16 @@ pm_status pm_diff_memory(const pm_diff* d, size_t* bytes) {
     return PM_OK;
 }
 
-pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const double K[9], const double* R,
-                          const double* t, const float* rho_gt, float* rho_hat, double* loss, void* stream) {
-    if (!d || !ref || !srcs || !K || !R || !t || !rho_gt || !loss) return PM_ERR_INVALID_ARGUMENT;
+// The forward's launches; loss: device memory (optional).
+static pm_status run_forward(pm_diff* d, const float* ref, const float* srcs, const double K[9], const double* R,
+                      const double* t, const float* rho_gt, float* rho_hat, double* loss, cudaStream_t st) {
+    if (!d || !ref || !srcs || !K || !R || !t || !rho_gt) return PM_ERR_INVALID_ARGUMENT;
     if (!finite_n(K, 9) || K[1] != 0.0 || K[3] != 0.0 || K[6] != 0.0 || K[7] != 0.0 || K[8] != 1.0 || K[0] == 0.0 ||
         K[4] == 0.0)
         return dfail(d, PM_ERR_INVALID_ARGUMENT, "K must be [[fx, 0, cx], [0, fy, cy], [0, 0, 1]]");
     const pm_diff_config& c = d->cfg;
     const int S = c.num_sources, W = c.width, H = c.height, D = c.num_planes;
     if (!finite_n(R, 9 * S) || !finite_n(t, 3 * S)) return dfail(d, PM_ERR_INVALID_ARGUMENT, "poses must be finite");
-    DGuard g(c.device);
-    cudaStream_t st = (cudaStream_t)stream;
     d->ref = ref;
     // H1 = K R K^-1, H2 = K t for each source-from-reference pose
     const double Ki[9] = {1.0 / K[0], 0.0, -K[2] / K[0], 0.0, 1.0 / K[4], -K[5] / K[4], 0.0, 0.0, 1.0};
@@ -809,33 +817,29 @@ pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const
     SoftArgs sa;
     std::memset(&sa, 0, sizeof sa);
     sa.vol = d->vol;
-    PD_CK(d, cudaMemsetAsync(d->sums, 0, 2 * sizeof(double), st));
+    PD_CK(d, cudaMemsetAsync(d->sums, 0, 3 * sizeof(double), st));
     sa.rho_gt = rho_gt;
     sa.invalid = d->invalid;
     sa.rho_hat = rho_hat;
     sa.gS = d->C;
     sa.sums = d->sums;
+    sa.loss = loss;
     sa.N = (int)d->N;
     sa.D = D;
     sa.rho0 = c.rho0;
     sa.drho = c.rho_step;
     sa.T = c.temperature;
     PD_CK(d, launch_soft(sa, d->wide ? 7 : 3, st));
-    double h[2];
-    PD_CK(d, cudaMemcpyAsync(h, d->sums, sizeof h, cudaMemcpyDeviceToHost, st));
-    PD_CK(d, cudaStreamSynchronize(st));
-    *loss = h[1] > 0 ? h[0] / h[1] : 0.0;
     d->have_forward = true;
     return PM_OK;
 }
 
-pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void* stream) {
+// The backward's launches; grad_pose: device memory, 6 doubles per source.
+static pm_status run_backward(pm_diff* d, float* grad_srcs, double* grad_pose, cudaStream_t st) {
     if (!d || !grad_srcs || !grad_pose) return PM_ERR_INVALID_ARGUMENT;
     if (!d->have_forward) return dfail(d, PM_ERR_BAD_STATE, "backward before forward");
     const pm_diff_config& c = d->cfg;
     const int S = c.num_sources, D = c.num_planes;
-    DGuard g(c.device);
-    cudaStream_t st = (cudaStream_t)stream;
     AdjArgs aa;
     std::memset(&aa, 0, sizeof aa);
     aa.gS = d->C;
@@ -854,7 +858,7 @@ pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void
         PD_CK(d, launch_adj(aa, 0x2u, st));
     }
     PD_CK(d, cudaMemsetAsync(grad_srcs, 0, 4 * d->N * S, st));
-    PD_CK(d, cudaMemsetAsync(d->gP, 0, 6 * sizeof(double) * S, st));
+    PD_CK(d, cudaMemsetAsync(grad_pose, 0, 6 * sizeof(double) * S, st));
     CostBwdArgs A;
     std::memset(&A, 0, sizeof A);
     A.ref = d->ref;
@@ -876,11 +880,47 @@ pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void
     A.rho0 = c.rho0;
     A.drho = c.rho_step;
     A.gI = grad_srcs;
-    A.gP = d->gP;
+    A.gP = grad_pose;
     PD_CK(d, launch_cost_bwd(A, st));
-    PD_CK(d, cudaMemcpyAsync(grad_pose, d->gP, 6 * sizeof(double) * S, cudaMemcpyDeviceToHost, st));
+    return PM_OK;
+}
+
+pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs, const double K[9], const double* R,
+                          const double* t, const float* rho_gt, float* rho_hat, double* loss, void* stream) {
+    if (!d || !loss) return PM_ERR_INVALID_ARGUMENT;
+    DGuard g(d->cfg.device);
+    cudaStream_t st = (cudaStream_t)stream;
+    const pm_status r = run_forward(d, ref, srcs, K, R, t, rho_gt, rho_hat, nullptr, st);
+    if (r != PM_OK) return r;
+    double h[2];
+    PD_CK(d, cudaMemcpyAsync(h, d->sums, sizeof h, cudaMemcpyDeviceToHost, st));
+    PD_CK(d, cudaStreamSynchronize(st));
+    *loss = h[1] > 0 ? h[0] / h[1] : 0.0;
+    return PM_OK;
+}
+
+pm_status pm_diff_forward_async(pm_diff* d, const float* ref, const float* srcs, const double K[9], const double* R,
+                                const double* t, const float* rho_gt, float* rho_hat, double* loss, void* stream) {
+    if (!d || !loss) return PM_ERR_INVALID_ARGUMENT;
+    DGuard g(d->cfg.device);
+    return run_forward(d, ref, srcs, K, R, t, rho_gt, rho_hat, loss, (cudaStream_t)stream);
+}
+
+pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void* stream) {
+    if (!d || !grad_pose) return PM_ERR_INVALID_ARGUMENT;
+    DGuard g(d->cfg.device);
+    cudaStream_t st = (cudaStream_t)stream;
+    const pm_status r = run_backward(d, grad_srcs, d->gP, st);
+    if (r != PM_OK) return r;
+    PD_CK(d, cudaMemcpyAsync(grad_pose, d->gP, 6 * sizeof(double) * d->cfg.num_sources, cudaMemcpyDeviceToHost, st));
     PD_CK(d, cudaStreamSynchronize(st));
     return PM_OK;
+}
+
+pm_status pm_diff_backward_async(pm_diff* d, float* grad_srcs, double* grad_pose, void* stream) {
+    if (!d) return PM_ERR_INVALID_ARGUMENT;
+    DGuard g(d->cfg.device);
+    return run_backward(d, grad_srcs, grad_pose, (cudaStream_t)stream);
 }
 
 const char* pm_diff_last_error(const pm_diff* d) { return d ? d->err.c_str() : "null handle"; }

@@ -76,9 +76,7 @@ class DepthLossEngine:
         self._check(self.lib.pm_diff_memory(self.h, ctypes.byref(b)), "pm_diff_memory")
         return b.value
 
-    def forward(self, ref, srcs, K, R, t, rho_gt):
-        """ref (H, W), srcs (S, H, W), rho_gt (H, W): float32 CUDA tensors; K 3x3, R (S, 3, 3),
-        t (S, 3) host arrays.  Returns (loss, rho_hat)."""
+    def _forward(self, ref, srcs, K, R, t, rho_gt, entry, loss):
         import torch
         for x in (ref, srcs, rho_gt):
             assert x.is_cuda and x.dtype == torch.float32 and x.is_contiguous()
@@ -86,14 +84,27 @@ class DepthLossEngine:
         k, kp = _dp(K)
         r, rp = _dp(R)
         tt, tp = _dp(t)
-        loss = ctypes.c_double()
         stream = torch.cuda.current_stream().cuda_stream
-        self._check(self.lib.pm_diff_forward(self.h, ctypes.c_void_p(ref.data_ptr()), ctypes.c_void_p(srcs.data_ptr()),
-                                             kp, rp, tp, ctypes.c_void_p(rho_gt.data_ptr()),
-                                             ctypes.c_void_p(rho_hat.data_ptr()), ctypes.byref(loss),
-                                             ctypes.c_void_p(stream)), "pm_diff_forward")
+        self._check(entry(self.h, ctypes.c_void_p(ref.data_ptr()), ctypes.c_void_p(srcs.data_ptr()), kp, rp, tp,
+                          ctypes.c_void_p(rho_gt.data_ptr()), ctypes.c_void_p(rho_hat.data_ptr()), loss,
+                          ctypes.c_void_p(stream)), "pm_diff_forward")
         self._keep = (ref, srcs, rho_gt)   # the backward reads them
+        return rho_hat
+
+    def forward(self, ref, srcs, K, R, t, rho_gt):
+        """ref (H, W), srcs (S, H, W), rho_gt (H, W): float32 CUDA tensors; K 3x3, R (S, 3, 3),
+        t (S, 3) host arrays.  Returns (loss, rho_hat)."""
+        loss = ctypes.c_double()
+        rho_hat = self._forward(ref, srcs, K, R, t, rho_gt, self.lib.pm_diff_forward, ctypes.byref(loss))
         return loss.value, rho_hat
+
+    def forward_async(self, ref, srcs, K, R, t, rho_gt):
+        """forward without waiting for the GPU: the loss comes back as a float64 CUDA scalar."""
+        import torch
+        loss = torch.empty((), dtype=torch.float64, device=srcs.device)
+        rho_hat = self._forward(ref, srcs, K, R, t, rho_gt, self.lib.pm_diff_forward_async,
+                                ctypes.c_void_p(loss.data_ptr()))
+        return loss, rho_hat
 
     def backward(self):
         """Gradients of the last forward's loss: (source images, CUDA tensor (S, H, W); poses,
@@ -106,6 +117,16 @@ class DepthLossEngine:
                                               gp.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
                                               ctypes.c_void_p(stream)), "pm_diff_backward")
         return g, gp.reshape(self.S, 6)
+
+    def backward_async(self):
+        """backward without waiting for the GPU: the pose gradient comes back as a float64 CUDA tensor."""
+        import torch
+        g = torch.empty((self.S, self.H, self.W), dtype=torch.float32, device="cuda")
+        gp = torch.empty((self.S, 6), dtype=torch.float64, device="cuda")
+        stream = torch.cuda.current_stream().cuda_stream
+        self._check(self.lib.pm_diff_backward_async(self.h, ctypes.c_void_p(g.data_ptr()), ctypes.c_void_p(gp.data_ptr()),
+                                                    ctypes.c_void_p(stream)), "pm_diff_backward")
+        return g, gp
 
 
 def _autograd_function():
@@ -120,18 +141,19 @@ def _autograd_function():
         @staticmethod
         def forward(ctx, srcs, xi, engine, ref, K, R0, t0, rho_gt):
             x = xi.detach().cpu().double().numpy()
-            R = np.stack([perturb_pose(R0[s], t0[s], x[s])[0] for s in range(len(R0))])
-            t = np.stack([perturb_pose(R0[s], t0[s], x[s])[1] for s in range(len(R0))])
-            loss, _ = engine.forward(ref, srcs.detach().contiguous(), K, R, t, rho_gt)
+            poses = [perturb_pose(R0[s], t0[s], x[s]) for s in range(len(R0))]
+            # nothing here waits for the GPU: the host prepares the backward while the forward runs
+            loss, _ = engine.forward_async(ref, srcs.detach().contiguous(), K, np.stack([R for R, _ in poses]),
+                                           np.stack([t for _, t in poses]), rho_gt)
             ctx.engine = engine
             ctx.xi_dtype, ctx.xi_device = xi.dtype, xi.device
-            return torch.tensor(loss, dtype=torch.float64, device=srcs.device)
+            return loss
 
         @staticmethod
         def backward(ctx, grad):
-            g_src, g_pose = ctx.engine.backward()
-            gs = g_src * grad.to(g_src.device, g_src.dtype)
-            gp = torch.from_numpy(g_pose).to(ctx.xi_device, ctx.xi_dtype) * grad.to(ctx.xi_device, ctx.xi_dtype)
+            g_src, g_pose = ctx.engine.backward_async()
+            gs = g_src.mul_(grad.to(g_src.device, g_src.dtype))
+            gp = g_pose.to(ctx.xi_device, ctx.xi_dtype) * grad.to(ctx.xi_device, ctx.xi_dtype)
             return gs, gp, None, None, None, None, None, None
 
     return DepthLoss

@@ -46,3 +46,36 @@ def test_gradients_at_tile_edges(W, H, D, S, store):
     assert loss == pytest.approx(loss64, rel=1e-3)
     assert np.linalg.norm(gs - gs64) < 0.05 * np.linalg.norm(gs64)
     assert np.linalg.norm(gp - gp64) < 0.02 * np.linalg.norm(gp64)
+
+
+@pytest.mark.parametrize("W,H,D,S,store,side", [(61, 40, 32, 1, False, False), (130, 90, 64, 2, True, True)])
+def test_async_calls_give_the_same(W, H, D, S, store, side):
+    """forward_async / backward_async leave on the device what forward / backward return, on the default stream
+    and on another one, also when the next forward is queued before they are read."""
+    fs = [scene.make_frameset(W, H, 0.8125 * W, S, seed=s) for s in (3, 4)]
+    rho0, drho = scene.plane_range(D)
+    e = DepthLossEngine(W, H, D, S, store_paths=store, rho0=rho0, rho_step=drho, temperature=0.05)
+    cu = lambda a: torch.from_numpy(np.ascontiguousarray(np.float32(a))).cuda()  # noqa: E731
+    args = []
+    for f in fs:
+        R = np.stack([f.R_srcs[s].T @ f.R_ref for s in range(S)])
+        t = np.stack([f.R_srcs[s].T @ (f.T_ref - f.T_srcs[s]) for s in range(S)])
+        args.append((cu(f.ref / 255.0), cu(f.srcs / 255.0), f.K, R, t, cu(1.0 / f.gt_depth)))
+    want = []
+    for a in args:
+        loss, rho = e.forward(*a)
+        want.append((loss, rho, *e.backward()))
+    torch.cuda.synchronize()
+    got = []
+    stream = torch.cuda.Stream() if side else torch.cuda.current_stream()
+    with torch.cuda.stream(stream):
+        for a in args:
+            loss, rho = e.forward_async(*a)
+            got.append((loss, rho, *e.backward_async()))
+    torch.cuda.synchronize()
+    for (l0, r0, g0, p0), (l1, r1, g1, p1) in zip(want, got):
+        assert l1.is_cuda and l1.dtype == torch.float64 and l1.item() == l0
+        assert torch.equal(r0, r1)
+        np.testing.assert_allclose(g1.cpu().numpy(), g0.cpu().numpy(), rtol=1e-4, atol=1e-9)
+        np.testing.assert_allclose(p1.cpu().numpy(), p0, rtol=1e-4, atol=1e-9)
+    e.close()
