@@ -193,7 +193,9 @@ cudaError_t launch_with_priority(void (*kern)(Args...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// every plane takes part in the minima (D a power of two, or the exact minimum)
+// PPL planes per lane: whether some planes may be left out of the minima (the tree of a D that is no power of two)
+constexpr bool partial(int ppl) { return (ppl & (ppl - 1)) != 0; }
+// every plane takes part in the minima (D a power of two, or the exact minimum); else those of tree_mask do
 bool all_planes(const PlaneOrder& o, int ppl) {
     for (int l = 0; l < 32; ++l)
         if (o.incl[l] != (1u << ppl) - 1u) return false;
@@ -203,14 +205,15 @@ bool all_planes(const PlaneOrder& o, int ppl) {
 template <int PPL, bool HALF, int NW>
 cudaError_t launch_pairs_nw(const SgmLaunch& a, unsigned mask, cudaStream_t s) {
     const size_t smem = (size_t)NW * PF * Ring<PPL, HALF>::STAGE_B;
-    const bool full = all_planes(a.order, PPL);
+    const bool full = !partial(PPL) || all_planes(a.order, PPL);
+    constexpr bool P = !partial(PPL);   // then only the first of each two below is needed
     void (*kern)(SgmLaunch, PairSet);
     if constexpr (HALF && PPL % 2 == 0) {
-        if (a.part_half) kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, true> : sgm_pair_kernel<PPL, HALF, NW, false, true>;
-        else kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, false> : sgm_pair_kernel<PPL, HALF, NW, false, false>;
+        if (a.part_half) kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, true> : sgm_pair_kernel<PPL, HALF, NW, P, true>;
+        else kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, false> : sgm_pair_kernel<PPL, HALF, NW, P, false>;
     } else {
         if (a.part_half) return cudaErrorInvalidValue;   // FP16 pair volumes come with FP16 cost volumes
-        kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, false> : sgm_pair_kernel<PPL, HALF, NW, false, false>;
+        kern = full ? sgm_pair_kernel<PPL, HALF, NW, true, false> : sgm_pair_kernel<PPL, HALF, NW, P, false>;
     }
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -250,8 +253,8 @@ cudaError_t launch_groups_t(const SgmLaunch& a, int mode, cudaStream_t s) {
     const long most = (long)sm_count() * 8;
     void (*kern)(SgmLaunch);
     if (mode == kCombineArgmin) kern = combine_group_kernel<PPL, kCombineArgmin, NP, HIN, true>;
-    else if (all_planes(a.order, PPL)) kern = combine_group_kernel<PPL, kCombineFilter, NP, HIN, true>;
-    else kern = combine_group_kernel<PPL, kCombineFilter, NP, HIN, false>;
+    else if (!partial(PPL) || all_planes(a.order, PPL)) kern = combine_group_kernel<PPL, kCombineFilter, NP, HIN, true>;
+    else kern = combine_group_kernel<PPL, kCombineFilter, NP, HIN, !partial(PPL)>;
     return launch_with_priority(kern, dim3((unsigned)(need < most ? need : most)), dim3(32 * kGroupWarps), 0, s, a.priority, a);
 }
 

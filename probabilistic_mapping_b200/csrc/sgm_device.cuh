@@ -322,34 +322,48 @@ template <int PPL> __device__ __forceinline__ void add_planes(float (&o)[PPL], c
     if constexpr (PPL % 2) o[PPL - 1] = __fadd_rn(a[PPL - 1], b);
 }
 
+// The planes of a lane that take part in the reduction tree of sgm.cu:24-31 (bit j: plane j), for 32 * ppl planes:
+// the tree halves down to ppl classes of planes modulo ppl, which are the same for every lane, and then drops some
+// of them where ppl is no power of two.  A constant of the kernel, so a dropped plane costs nothing (masks read per
+// lane cost a test and a select per plane: the stage at 1280x720x192 3277 -> 3240 us, 333x251x96 148 -> 145).
+constexpr unsigned tree_mask(int ppl) {
+    unsigned slot[8] = {};
+    for (int d = 0; d < ppl; ++d) slot[d] = 1u << d;
+    for (int i = ppl >> 1; i > 0; i >>= 1)
+        for (int d = 0; d < i; ++d)
+            if (d + i < ppl) {
+                slot[d] |= slot[d + i];
+                slot[d + i] = 0;
+            }
+    return slot[0];
+}
+
 // Smallest of the lane's planes that take part in the minimum (all of them when FULL).
-template <int PPL, bool FULL> __device__ __forceinline__ float lane_min(const float (&v)[PPL], uint32_t incl) {
-    if constexpr (FULL) {
-        float m = v[0];
-        int j = 1;
+template <int PPL, bool FULL> __device__ __forceinline__ float lane_min(const float (&v)[PPL]) {
+    constexpr unsigned MASK = FULL ? (1u << PPL) - 1u : tree_mask(PPL);
+    static_assert(MASK & 1u, "plane 0 always takes part");
+    float m = v[0], one = 0.0f;
+    bool have = false;   // the odd one of two planes for a three-input minimum (all constants)
 #pragma unroll
-        for (; j + 1 < PPL; j += 2) m = min3f(m, v[j], v[j + 1]);
-        if (j < PPL) m = fminf(m, v[j]);
-        return m;
-    } else {
-        float m = inf_f();
-#pragma unroll
-        for (int j = 0; j < PPL; ++j)
-            if ((incl >> j) & 1u) m = fminf(m, v[j]);
-        return m;
+    for (int j = 1; j < PPL; ++j) {
+        if (!((MASK >> j) & 1u)) continue;
+        if (have) m = min3f(m, one, v[j]);
+        one = v[j];
+        have = !have;
     }
+    return have ? fminf(m, one) : m;
 }
 
 // Whether the pixel has a plane that was never measured (cost < 0): the path treats its cost as 0
 // and outputs COST_INF = 0 there (sgm.cu:33-38, 67-71, 101-104).
-template <int PPL, bool FULL> __device__ __forceinline__ bool pixel_invalid(const float (&cv)[PPL], uint32_t incl) {
-    return __any_sync(kFull, lane_min<PPL, FULL>(cv, incl) < 0.0f);
+template <int PPL, bool FULL> __device__ __forceinline__ bool pixel_invalid(const float (&cv)[PPL]) {
+    return __any_sync(kFull, lane_min<PPL, FULL>(cv) < 0.0f);
 }
 
 // A pixel's costs as the path takes them (0 on an invalid pixel); returns whether the pixel is invalid.
 template <int PPL, bool FULL>
-__device__ __forceinline__ bool path_costs(float (&cz)[PPL], const float (&cv)[PPL], uint32_t incl) {
-    const bool inv = pixel_invalid<PPL, FULL>(cv, incl);
+__device__ __forceinline__ bool path_costs(float (&cz)[PPL], const float (&cv)[PPL]) {
+    const bool inv = pixel_invalid<PPL, FULL>(cv);
 #pragma unroll
     for (int j = 0; j < PPL; ++j) cz[j] = inv ? 0.0f : cv[j];
     return inv;
@@ -368,18 +382,18 @@ __device__ __forceinline__ void path_neighbours(PathState<PPL>& s, int lane) {
     if (lane == 31) s.above = inf_f();
 }
 template <int PPL, bool FULL, bool ROUTE>
-__device__ __forceinline__ void path_exchange(PathState<PPL>& s, uint32_t incl, int lane) {
+__device__ __forceinline__ void path_exchange(PathState<PPL>& s, int lane) {
     if constexpr (kAhead<PPL, ROUTE>) path_neighbours<PPL>(s, lane);
-    s.mprev = warp_min_f32(lane_min<PPL, FULL>(s.L, incl));
+    s.mprev = warp_min_f32(lane_min<PPL, FULL>(s.L));
 }
 
 // First pixel of a path: L = C, or 0 on an invalid pixel (sgm.cu:21-43).
 template <int PPL, bool FULL, bool ROUTE>
-__device__ __forceinline__ void path_first(PathState<PPL>& s, const float (&cz)[PPL], uint32_t incl, int lane,
+__device__ __forceinline__ void path_first(PathState<PPL>& s, const float (&cz)[PPL], int lane,
                                            float (&o)[PPL]) {
 #pragma unroll
     for (int j = 0; j < PPL; ++j) s.L[j] = o[j] = cz[j];
-    path_exchange<PPL, FULL, ROUTE>(s, incl, lane);
+    path_exchange<PPL, FULL, ROUTE>(s, lane);
 }
 
 // The differentiation form's record of one step: which term of the minimum each plane took, as three
@@ -415,7 +429,7 @@ template <int PPL> __device__ __forceinline__ void store_route(uint32_t* p, cons
 // lower one first), then to the minimum.
 template <int PPL, bool FULL, bool ROUTE = false>
 __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s, const float (&cz)[PPL], bool inv,
-                                          bool q, float p1q, float p2q, uint32_t incl, int lane, float (&o)[PPL],
+                                          bool q, float p1q, float p2q, int lane, float (&o)[PPL],
                                           Route<PPL>* rt = nullptr) {
     const float P1 = q ? p1q : a.p1, P2 = q ? p2q : a.p2;
     const float mP2 = __fadd_rn(s.mprev, P2);
@@ -446,7 +460,7 @@ __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s,
     add_planes<PPL>(s.L, vv, -s.mprev);        // - minL (:98); the negation is exact
 #pragma unroll
     for (int j = 0; j < PPL; ++j) o[j] = inv ? 0.0f : s.L[j];
-    path_exchange<PPL, FULL, ROUTE>(s, incl, lane);
+    path_exchange<PPL, FULL, ROUTE>(s, lane);
 }
 
 // Reference intensity of step k of a chain starting at pixel p0 (0 past its end).
@@ -552,8 +566,6 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         cp_async_commit();
     }
 
-    uint32_t incl = kFull;
-    if constexpr (!FULL) incl = a.order.incl[lane];
     const float p1q = __fmul_rn(a.p1, a.q1), p2q = __fmul_rn(a.p2, a.q2);
     PathState<PPL> fs, bs;
     float lastf = 0.0f, lastb = 0.0f;
@@ -590,11 +602,11 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         [[maybe_unused]] float nf[PPL], nb[PPL];
         slices(wbase, cf, cb);
         if constexpr (AHEAD) slices(wbase + STAGE_B, nf, nb);   // (past a scanline of one pixel: not used)
-        invf = path_costs<PPL, FULL>(czf, cf, incl);
-        path_costs<PPL, FULL>(czb, cb, incl);
+        invf = path_costs<PPL, FULL>(czf, cf);
+        path_costs<PPL, FULL>(czb, cb);
         if constexpr (ROUTE) rinv = invf ? 1u : 0u;
-        path_first<PPL, FULL, ROUTE>(fs, czf, incl, lane, of);
-        path_first<PPL, FULL, ROUTE>(bs, czb, incl, lane, ob);
+        path_first<PPL, FULL, ROUTE>(fs, czf, lane, of);
+        path_first<PPL, FULL, ROUTE>(bs, czb, lane, ob);
         if constexpr (ROUTE) {
             if (n == 1 && slot == 0) flush_invalid(0);
         }
@@ -608,8 +620,8 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         if (PF < n) issue(wbase, PF);
         cp_async_commit();
         if constexpr (AHEAD) {
-            invf = path_costs<PPL, FULL>(czf, nf, incl);
-            invb = path_costs<PPL, FULL>(czb, nb, incl);
+            invf = path_costs<PPL, FULL>(czf, nf);
+            invb = path_costs<PPL, FULL>(czb, nb);
         }
     }
     static_assert(PF > 2, "the ring holds the step after next");
@@ -633,30 +645,30 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
         float nf[PPL], nb[PPL];
         slices(wbase + (AHEAD ? nst : st) * STAGE_B, nf, nb);
         if constexpr (!AHEAD) {
-            invf = path_costs<PPL, FULL>(czf, nf, incl);
-            invb = path_costs<PPL, FULL>(czb, nb, incl);
+            invf = path_costs<PPL, FULL>(czf, nf);
+            invb = path_costs<PPL, FULL>(czb, nb);
         }
         const int bit = k & 31;
         if constexpr (ROUTE) {
             Route<PPL> r;
-            path_step<PPL, FULL, true>(a, fs, czf, invf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of, &r);
+            path_step<PPL, FULL, true>(a, fs, czf, invf, (fs.qmask >> bit) & 1u, p1q, p2q, lane, of, &r);
             put_route(slot, pf, r);
             if (slot == 0) {
                 rinv = (bit == 0 ? 0u : rinv) | (invf ? 1u << bit : 0u);
                 if (bit == 31 || k == n - 1) flush_invalid(k);
             }
-            path_step<PPL, FULL, true>(a, bs, czb, invb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob, &r);
+            path_step<PPL, FULL, true>(a, bs, czb, invb, (bs.qmask >> bit) & 1u, p1q, p2q, lane, ob, &r);
             put_route(slot + 1, pb, r);
         } else {
-            path_step<PPL, FULL>(a, fs, czf, invf, (fs.qmask >> bit) & 1u, p1q, p2q, incl, lane, of);
-            path_step<PPL, FULL>(a, bs, czb, invb, (bs.qmask >> bit) & 1u, p1q, p2q, incl, lane, ob);
+            path_step<PPL, FULL>(a, fs, czf, invf, (fs.qmask >> bit) & 1u, p1q, p2q, lane, of);
+            path_step<PPL, FULL>(a, bs, czb, invb, (bs.qmask >> bit) & 1u, p1q, p2q, lane, ob);
         }
         // refill this step's stage (its costs are in registers) with step k + PF
         if (k + PF < n) issue(wbase + st * STAGE_B, k + PF);
         cp_async_commit();
         if constexpr (AHEAD) {
-            invf = path_costs<PPL, FULL>(czf, nf, incl);
-            invb = path_costs<PPL, FULL>(czb, nb, incl);
+            invf = path_costs<PPL, FULL>(czf, nf);
+            invb = path_costs<PPL, FULL>(czb, nb);
         }
         st = nst;
     };
