@@ -871,6 +871,32 @@ pm_status pm_stage_calc_cost(const pm_config* cfg, const float* ref, const float
     size_t pitch = 0;
     bool ok = true;
     int done = 0;
+    // A volume that starts from initReference is free until its first tile is stored, so its first rows serve as the
+    // quads of the sources: the other rows are computed from them, and then these rows from the float images.  The
+    // quads take a load where four float taps and their addresses go: 640x480x64 with 5 sources 882 -> 669 us, of
+    // which the 160 rows that hold the quads take some 300 (corrected mode 402 -> 374).  Where the rest is small the two more launches cost more.
+    const int rows = (H + kCostTileRows - 1) / kCostTileRows;
+    if (!tex && !cnt && nsrc > 0 && (reinterpret_cast<uintptr_t>(cost) & 15) == 0) {
+        const size_t quads = quad_stride(N) * nsrc, tile = (size_t)W * kCostTileRows * cfg->num_planes / 4;   // in float4
+        const size_t used = (quads + tile - 1) / tile;   // tile rows
+        const double rest = used < (size_t)rows ? (double)(H - (int)used * kCostTileRows) * W * cfg->num_planes * nsrc : 0.0;
+        if (rest >= (cfg->cost_mode == PM_COST_REFERENCE ? 4e6 : 16e6)) {
+            a.srcq = reinterpret_cast<const float4*>(cost);
+            a.nsrc = nsrc;
+            for (int s = 0; s < nsrc; ++s)
+                for (int i = 0; i < 12; ++i) a.hom[s][i] = homs[12 * s + i];
+            a.tile_y0 = (int)used;
+            a.tile_rows = rows - (int)used;
+            a.invalid = nullptr;   // below, once the volume is complete
+            if (launch_to_quad_f(W, H, nsrc, srcs, reinterpret_cast<float4*>(cost), st) != cudaSuccess ||
+                launch_cost(a, st) != cudaSuccess)
+                return PM_ERR_CUDA;
+            a.srcq = nullptr;
+            a.tile_y0 = 0;
+            a.tile_rows = (int)used;
+            a.invalid = invalid;
+        }
+    }
     do {
         const int n = std::min(nsrc - done, kMaxSources);
         a.srcs = srcs + N * done;

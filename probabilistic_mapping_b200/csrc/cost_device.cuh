@@ -12,7 +12,7 @@ namespace {
 
 
 constexpr int TXU = 30;                  // output columns per tile (lanes 1..30)
-constexpr int TY = 8;                    // output rows per tile
+constexpr int TY = kCostTileRows;        // output rows per tile
 constexpr int WARPS = 8;                 // one plane pair per warp
 constexpr int PCB = 2 * WARPS;           // planes per CTA
 constexpr int NT = 32 * WARPS;

@@ -552,16 +552,6 @@ cudaError_t launch_cost_bwd(const CostBwdArgs& A, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-__global__ void to_quad_f_kernel(int W, int H, const float* __restrict__ img, float4* __restrict__ q) {
-    const int y = blockIdx.y;
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < W; x += gridDim.x * blockDim.x) {
-        const float* r0 = img + (size_t)y * W;
-        const bool hx = x + 1 < W, hy = y + 1 < H;
-        q[(size_t)y * W + x] = make_float4(r0[x], hy ? r0[x + W] : 0.0f, hx ? r0[x + 1] : 0.0f,
-                                           (hx && hy) ? r0[x + W + 1] : 0.0f);
-    }
-}
-
 template <int PPL> cudaError_t launch_fwd_t(const SgmLaunch& a, const RouteOut& ro, unsigned mask, cudaStream_t s) {
     const PairSet ps = make_pair_set(mask, a.W, a.H, kPairWarps);
     const size_t smem = (size_t)kPairWarps * PF * Ring<PPL, false>::STAGE_B;
@@ -713,7 +703,6 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     alloc((void**)&d->codes, 8 * d->N * 4 * words);
     alloc((void**)&d->sums, 3 * sizeof(double));
     alloc((void**)&d->gP, 6 * sizeof(double) * c->num_sources);
-    ok = ok && init_quad_slots(d->quads, d->N, c->num_sources, 0) == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         free_diff(d);
@@ -764,10 +753,7 @@ static pm_status run_forward(pm_diff* d, const float* ref, const float* srcs, co
     d->cam[1] = (float)K[4];
     d->cam[2] = (float)K[2];
     d->cam[3] = (float)K[5];
-    const dim3 qg((W + 255) / 256, H);
-    for (int s = 0; s < S; ++s)
-        to_quad_f_kernel<<<qg, 256, 0, st>>>(W, H, srcs + (size_t)s * d->N, d->quads + s * quad_stride(d->N));
-    PD_CK(d, cudaGetLastError());
+    PD_CK(d, launch_to_quad_f(W, H, S, srcs, d->quads, st));
     CostLaunch a;
     std::memset(&a, 0, sizeof a);
     a.ref = ref;

@@ -44,6 +44,7 @@ enum BoundsSite {
 };
 
 // ---- plane-sweep cost volume (calc_cost.cu) ----------------------------------------------
+constexpr int kCostTileRows = 8;
 struct CostLaunch {
     const float* ref;      // W*H scaled reference image
     const float* srcs;     // nsrc consecutive W*H scaled source images (used when srcq is null)
@@ -73,6 +74,9 @@ struct CostLaunch {
     float* cnt;            // running count (incremental mode) or nullptr
     uint8_t* invalid;      // W*H, 1 where a plane was never measured (optional)
     int incremental;       // start from (cost, cnt) in memory instead of (-1, 0)
+    // rows of the volume to compute, in tiles of kCostTileRows: [tile_y0, tile_y0 + tile_rows), tile_rows 0: all.  The
+    // FP16 rebase and the invalid flags cover the whole volume.
+    int tile_y0, tile_rows;
     cudaEvent_t kernel_done = nullptr;   // recorded right after the cost kernel (before the rebase)
 };
 // An integer M in [2^23, 1.5 * 2^23] whose bits(M) * (W + 1), modulo 2^32, plus W*H stays below 2^32.
@@ -153,6 +157,8 @@ cudaError_t launch_to_float_h(int W, int H, const uint8_t* src, size_t src_pitch
 // outside the image (the border addressing of the reference textures, calc_cost.cu:230-237).
 cudaError_t launch_to_quad(int W, int H, const uint8_t* src, size_t src_pitch, float4* dst,
                            float scale, cudaStream_t s);
+// nsrc consecutive W*H float images -> nsrc quad slots (quad_stride(W*H) apart), NaN quads included.
+cudaError_t launch_to_quad_f(int W, int H, int nsrc, const float* src, float4* dst, cudaStream_t s);
 // A pitched W x H source image (FP16 texels, or FP32 texels when f32) and its texture object:
 // linear filtering, zero border, unnormalised coordinates (the reference's texture setup,
 // calc_cost.cu:226-237).

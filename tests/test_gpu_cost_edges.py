@@ -70,3 +70,29 @@ def test_floor_bias():
     got, homs = cost_of(W, H, D, ref, [src], [(R, np.array([0.05, -0.03, 0.01]))], K, 0.04, 1.0, 1)
     want, _ = oracle.calc_cost(p, ref, src[None], homs, "f32")
     assert (bits(got) == bits(want)).all()
+
+
+@pytest.mark.parametrize("W,H,D,S,mode", [(203, 151, 64, 3, 0), (97, 263, 96, 5, 0), (401, 305, 32, 7, 0), (203, 57, 64, 3, 0),
+                                          (333, 251, 64, 5, 1), (401, 305, 32, 9, 0)])
+def test_stage_cost_through_the_volume(pm_lib, W, H, D, S, mode):
+    """pm_stage_calc_cost keeps the sources' quads in the first rows of the volume where the other rows are worth it
+    (all but the fourth case, which is too small, and the last, whose quads would take every row)."""
+    import ctypes
+    from test_gpu_stages import config, upload_images, vp
+    fs, poses = setup(W, H, S, 11)
+    p = oracle.Params(W=W, H=H, D=D, rho0=0.05, drho=0.03, intensity_scale=1.0, cost_mode=mode, num_paths=4)
+    homs = np.stack([oracle.compose_homography(fs.K, np.eye(3), np.zeros(3), R, T) for R, T in poses]).astype(np.float32)
+    want, _ = oracle.calc_cost(p, fs.ref, fs.srcs, homs, "f32")
+    rf, sf = upload_images(pm_lib, fs, 1.0)
+    buf = torch.full((W * H * D + 64,), 7.0, dtype=torch.float32, device="cuda")
+    inv = torch.full((H, W), 9, dtype=torch.uint8, device="cuda")
+    cfg = config(p)
+    hp = np.ascontiguousarray(homs).ctypes.data_as(ctypes.POINTER(ctypes.c_float))
+    for guard in (0, 1):   # 16-byte aligned, and not
+        cost = ctypes.c_void_p(buf.data_ptr() + 4 * guard)
+        assert pm_lib.pm_stage_calc_cost(ctypes.byref(cfg), vp(rf), vp(sf), S, hp, cost, None, vp(inv), None) == 0
+        torch.cuda.synchronize()
+        got = buf[guard:guard + W * H * D].cpu().numpy().reshape(H, W, D)
+        assert (bits(got) == bits(want)).all()
+        assert (inv.cpu().numpy() == (want < 0).any(-1)).all()
+        assert (buf[guard + W * H * D:] == 7.0).all()
