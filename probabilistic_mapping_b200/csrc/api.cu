@@ -307,7 +307,25 @@ pm_status evaluate_cost(pm_mapper* h, bool into_state) {
     return PM_OK;
 }
 
-pm_status run_sgm_filter(pm_mapper* h) {
+// A caller's W x H float map that the kernels can write themselves: plain memory of the mapper's own device, floats on
+// their boundaries.  (Other devices', managed and host memory take a copy.)
+bool kernels_can_write(const pm_mapper* h, const float* p, size_t pitch) {
+    cudaPointerAttributes at;
+    if (!p || (reinterpret_cast<uintptr_t>(p) | pitch) % sizeof(float) || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == h->cfg.device;
+}
+
+// The output pitch in bytes (0: packed), or 0 when it is too small.
+size_t out_pitch(const pm_mapper* h, size_t pitch) {
+    const size_t row = sizeof(float) * (size_t)h->cfg.width;
+    return pitch == 0 ? row : pitch < row ? 0 : pitch;
+}
+
+// direct: the winner-take-all depth also goes there, with a byte pitch (optional).
+pm_status run_sgm_filter(pm_mapper* h, float* direct = nullptr, size_t direct_pitch = 0) {
     const pm_config& c = h->cfg;
     SgmLaunch a;
     fill_sgm_launch(c, h->order, a);
@@ -320,6 +338,8 @@ pm_status run_sgm_filter(pm_mapper* h) {
     a.part_half = a.cost_half && !h->store_sgm;
     a.depth = h->d_depth;
     a.depth_pitch = sizeof(float) * (size_t)c.width;
+    a.depth2 = direct;
+    a.depth2_pitch = direct_pitch;
     a.index = h->d_idx;
     a.wta_class = h->stats ? h->d_wta_class : nullptr;
     PM_CK(h, launch_sgm(a, kCombineFilter, h->stream));
@@ -567,10 +587,12 @@ pm_status pm_output(pm_mapper* h, float* depth, size_t pitch) {
     mark(h, 0);
     st = evaluate_cost(h, false);
     mark_done(h, 0);
-    if (st == PM_OK) st = run_sgm_filter(h);
+    const size_t p = out_pitch(h, pitch);
+    const bool direct = p && kernels_can_write(h, depth, p);
+    if (st == PM_OK) st = run_sgm_filter(h, direct ? depth : nullptr, p);
     mark_done(h, 1);
     mark(h, 3);
-    if (st == PM_OK) st = copy_out(h, depth, pitch, h->d_depth);
+    if (st == PM_OK && !direct) st = copy_out(h, depth, pitch, h->d_depth);
     mark_done(h, 3);
     return st;
 }
@@ -634,6 +656,14 @@ pm_status pm_output_fusion(pm_mapper* h, float* depth, size_t depth_pitch, float
     if (st == PM_OK) st = run_sgm_filter(h);
     mark_done(h, 1);
     if (st != PM_OK) return st;
+    // what the update kernel writes for the caller itself (not the zeros of the first keyframe)
+    FuseOut out{};
+    out.depth_pitch = out_pitch(h, depth_pitch);
+    out.variance_pitch = out_pitch(h, var_pitch);
+    if (!h->first_fusion && out.depth_pitch && (!variance || out.variance_pitch)) {
+        if (kernels_can_write(h, depth, out.depth_pitch)) out.depth = depth;
+        if (variance && kernels_can_write(h, variance, out.variance_pitch)) out.variance = variance;
+    }
     if (h->first_fusion) {   // stereo_mapper.cpp:128-146
         h->first_fusion = false;
         std::memcpy(h->R_prev, R, sizeof h->R_prev);
@@ -658,6 +688,7 @@ pm_status pm_output_fusion(pm_mapper* h, float* depth, size_t depth_pitch, float
         }
         f.table = reinterpret_cast<uint32_t*>(h->d_table);
         f.variance = h->d_var;
+        f.out = out;
         f.mask = h->d_cmask;
         f.orig_mu = h->d_corig;
         f.head = h->d_chead;
@@ -684,6 +715,7 @@ pm_status pm_output_fusion(pm_mapper* h, float* depth, size_t depth_pitch, float
         f.ztable = h->d_ztable;
         f.table = h->d_table;
         f.variance = h->d_var;
+        f.out = out;
         f.stats = h->stats ? h->d_stats : nullptr;
         PM_CK(h, launch_fuse_gpu(f, h->stream));
         std::memcpy(h->R_prev, R, sizeof h->R_prev);
@@ -692,8 +724,8 @@ pm_status pm_output_fusion(pm_mapper* h, float* depth, size_t depth_pitch, float
     }
     mark_done(h, 2);
     mark(h, 3);
-    st = copy_out(h, depth, depth_pitch, h->d_fused);
-    if (st == PM_OK && variance) st = copy_out(h, variance, var_pitch, h->d_var);
+    if (!out.depth) st = copy_out(h, depth, depth_pitch, h->d_fused);
+    if (st == PM_OK && variance && !out.variance) st = copy_out(h, variance, var_pitch, h->d_var);
     mark_done(h, 3);
     return st;
 }

@@ -189,7 +189,9 @@ __device__ __forceinline__ int2 update_pixel(const FuseLaunch& a, const FuseView
     v.cur[0][e] = ca;
     if (write_all) { v.cur[1][e] = cb; v.cur[2][e] = cm; v.cur[3][e] = cs; }
     a.depth[e] = out_d;
-    if (a.variance) a.variance[e] = write_all ? cs : v.cur[3][e];
+    const float var = write_all || !(a.variance || a.out.variance) ? cs : v.cur[3][e];
+    if (a.variance) a.variance[e] = var;
+    fuse_out(a.out, x, y, out_d, var);
     return make_int2(t == 0 ? 0 : direct ? 1 : 2, ucls);
 }
 

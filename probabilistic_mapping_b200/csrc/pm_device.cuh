@@ -53,6 +53,15 @@ __device__ __forceinline__ void tally_block(unsigned* g, int c0, int c1 = -1, in
     if (threadIdx.x < N && s[threadIdx.x]) atomicAdd(g + threadIdx.x, s[threadIdx.x]);
 }
 
+// element (x, y) of a map with a byte pitch
+__device__ __forceinline__ float& pitched(float* p, size_t pitch, int x, int y) {
+    return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + (size_t)y * pitch)[x];
+}
+__device__ __forceinline__ void fuse_out(const FuseOut& o, int x, int y, float depth, float variance) {
+    if (o.depth) pitched(o.depth, o.depth_pitch, x, y) = depth;
+    if (o.variance) pitched(o.variance, o.variance_pitch, x, y) = variance;
+}
+
 // Homography of one source frame as kernel arguments (the 12 floats of ad_calc_cost,
 // calc_cost.cu:212-219).
 struct Hom {

@@ -113,6 +113,8 @@ struct SgmLaunch {
     FilterParams fp;
     float* depth;          // W*H with byte pitch depth_pitch (fused filter only)
     size_t depth_pitch;
+    float* depth2;         // the depth a second time, with its own byte pitch (optional)
+    size_t depth2_pitch;
     int32_t* index;        // W*H (optional)
     PlaneOrder order;
     int pair_warps;        // scanlines per block of the path-pair kernel: 2, 4 or 8 (0: by the image)
@@ -167,6 +169,14 @@ cudaError_t launch_convert(int W, int H, const float* in, float* out, int flag, 
                            cudaStream_t s);
 
 // ---- depth fusion (depth_fusion.cu) --------------------------------------------------------
+// Where a caller in device memory takes the fused depth and its variance, with byte pitches (each optional):
+// written beside the library's own maps by the kernel that has the values, instead of copied afterwards.
+struct FuseOut {
+    float* depth;
+    size_t depth_pitch;
+    float* variance;
+    size_t variance_pitch;
+};
 struct FuseLaunch {
     int W, H;
     float pose[12];        // R_p2c row-major, t_p2c
@@ -178,6 +188,7 @@ struct FuseLaunch {
     unsigned long long* ztable;  // W*H scratch z-buffer
     int32_t* table;        // W*H filled propagation table (optional)
     float* variance;       // W*H sigma^2 of the current state (optional)
+    FuseOut out;           // a second copy of both
     // Batched form (values that change every step, read from device memory so that a captured
     // graph stays valid): params_dev = pose[12], cam[4]; flags_dev = {first, pre_index}; the
     // state sets are state[pre_index] (previous) and state[pre_index ^ 1] (current).  On the first
@@ -199,6 +210,7 @@ struct FuseCpuLaunch {
     float* cur[4];         // state of the current keyframe
     uint32_t* table;       // W*H filled propagation table, packed (y << 16) | x (optional)
     float* variance;       // W*H sigma^2 of the current state (optional)
+    FuseOut out;           // a second copy of both
     // scratch, W*H each
     uint8_t* mask;
     float* orig_mu;

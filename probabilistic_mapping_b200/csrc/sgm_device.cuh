@@ -806,6 +806,10 @@ __device__ __forceinline__ void combine_pixels(const SgmLaunch& a, long first, l
                     dp = reinterpret_cast<float*>(reinterpret_cast<char*>(a.depth) + (size_t)y * a.depth_pitch) + x;
                 }
                 *dp = depth;
+                if (a.depth2) {
+                    const unsigned up = (unsigned)pix, uw = (unsigned)a.W, y = up / uw;
+                    pitched(a.depth2, a.depth2_pitch, (int)(up - y * uw), (int)y) = depth;
+                }
                 if (a.index) a.index[pix] = idx;
                 if (a.wta_class) a.wta_class[pix] = (uint8_t)cls;
             }
@@ -1023,6 +1027,10 @@ __device__ __forceinline__ void combine_groups(const SgmLaunch& a, const void* c
                 dp = reinterpret_cast<float*>(reinterpret_cast<char*>(a.depth) + (size_t)y * a.depth_pitch) + x;
             }
             *dp = depth;
+            if (a.depth2) {
+                const unsigned up = (unsigned)pix, uw = (unsigned)a.W, y = up / uw;
+                pitched(a.depth2, a.depth2_pitch, (int)(up - y * uw), (int)y) = depth;
+            }
             if (a.index) a.index[pix] = idx;
             if (a.wta_class) a.wta_class[pix] = (uint8_t)cls;
         }
