@@ -46,7 +46,7 @@ namespace {
 template <int MODE, bool HALF, int SAMP, bool INC>
 __global__ void __launch_bounds__(NT, (HALF && SAMP == kTex && !INC) ? 4 : 3) cost_kernel(const CostLaunch a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    cost_tile<MODE, HALF, SAMP, INC>(a, blockIdx.x, blockIdx.y + a.tile_y0, blockIdx.z, smem_raw);
+    cost_tile<MODE, HALF, SAMP, INC>(a, blockIdx.x, blockIdx.z + a.tile_y0, blockIdx.y, smem_raw);
 }
 
 template <int PPL>
@@ -113,7 +113,12 @@ cudaError_t init_quad_slots(float4* q, size_t npix, int slots, cudaStream_t s) {
 cudaError_t launch_cost(const CostLaunch& a, cudaStream_t s) {
     if (a.nsrc > kMaxSources || a.D % PCB || a.W < 1 || a.H < 1) return cudaErrorInvalidValue;
     if (a.cost_half && (!a.offset || !a.block_offset || (a.D / 32) % 2)) return cudaErrorInvalidValue;
-    const dim3 grid((a.W + TXU - 1) / TXU, a.tile_rows ? a.tile_rows : (a.H + TY - 1) / TY, a.D / PCB);
+    // A row of tiles, all its planes, the next row: the rows of the sources that a row of tiles reads stay in the L2
+    // cache for all its planes.  With the planes outermost the sources were read again for every 16 planes, from
+    // memory where they and the volume's stores do not fit the cache together: 1280x720, 192 planes, 4 sources, FP32
+    // texture 2861 -> 2688 us, exact 3717 -> 3611, FP16 texture 2757 -> 2527 (256 planes, 2 sources, corrected 1388 ->
+    // 1232, 64 planes FP32 texture 962 -> 926); up to 640x480 the same within 1 %.
+    const dim3 grid((a.W + TXU - 1) / TXU, a.D / PCB, a.tile_rows ? a.tile_rows : (a.H + TY - 1) / TY);
     cudaError_t e;
     if (a.mode == 0) e = a.cost_half ? launch_q<0, true>(a, grid, s) : launch_q<0, false>(a, grid, s);
     else e = a.cost_half ? launch_q<1, true>(a, grid, s) : launch_q<1, false>(a, grid, s);
