@@ -34,9 +34,10 @@ __device__ inline float warp_sum(float v) {
 
 // ---- forward paths ------------------------------------------------------------------------
 // The product's pair recurrences (sgm_pair_block), which also leave the records that the adjoint
-// routes by: 3 to 4 bits per voxel and path, where the path states themselves would take 32.  Bound by memory like the product's: two reads of the costs, a store and a
-// reduction per pair, 20 bytes per voxel and pair, and 0.5 for the records.  All eight paths at 640x480x128:
-// 0.94 ms (one path after the other, each adding to the sum and storing its states: 5.0 ms).
+// routes by: 3 to 4 bits per voxel and path, where the path states themselves would take 32.  Bound by memory like the
+// product's: two reads of the costs, a store and a reduction per pair (two stores where each path has its own
+// volume), 16 to 20 bytes per voxel and pair, and 1 for the records.  All eight paths at 640x480x128:
+// 0.60 ms (one path after the other, each adding to the sum and storing its states: 5.0 ms).
 constexpr int kPairWarps = 1;   // scanlines per block: small blocks spread an image's scanlines over the SMs
 
 template <int PPL>
@@ -92,8 +93,8 @@ __device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[
 // A pair's adjoints: path 2p's from the far end of the scanline, path 2p + 1's from its start, both
 // by one warp, as sgm_pair_block walks the forward: two independent recurrences in flight, gS and the
 // records streamed PF steps ahead, the first visit of a pixel stores and the second adds.  Bound by
-// memory: two reads of gS, a store and a reduction, 20 bytes per voxel and pair (0.55 ms for all eight paths at
-// 640x480x128, 5.8 TB/s; path by path from the stored states 6.4 ms).
+// memory: two reads of gS, a store and a reduction, 20 bytes per voxel and pair (0.57 ms for all eight paths at
+// 640x480x128, 5.5 TB/s; path by path from the stored states 6.4 ms).
 template <int PPL, int NW>
 __device__ __forceinline__ void adjoint_pair_block(const AdjArgs& a, int pair, int bx, unsigned char* ring) {
     constexpr int SLICE_B = 128 * PPL, REC_B = 4 * Route<PPL>::WORDS;
@@ -221,7 +222,7 @@ struct SoftArgs {
 
 // The sum of the volumes, the soft-argmin over it, the loss's terms and its adjoint, one warp per pixel.  The
 // paths are added in their order, so that the loss's signs do not depend on the layout of the volumes.  Bound by
-// memory: NV reads and a write per voxel (0.17 ms at 640x480x128 with 4 volumes).  The loss is summed in double
+// memory: NV reads and a write per voxel (0.27 ms at 640x480x128 with 7 volumes: 4.7 TB/s).  The loss is summed in double
 // precision per warp, block and grid.
 template <int PPL, int NV>
 __global__ void __launch_bounds__(256) soft_kernel(const SoftArgs a) {
@@ -326,8 +327,8 @@ struct CostBwdArgs {
 //   * the pose terms stay in registers over a tile's rows, then one double atomic per CTA and component.
 // The samples repeat the cost kernel's operations (homography FMAs, reciprocal, exact bilinear), so that
 // the signs are the forward's.  Bound by issue (about 100 instructions per sample and plane pair); with one
-// thread per voxel, 27 samples per source and nine scatters it was bound by its atomics: 29.5 -> 0.78 ms at
-// 640x480x128 with 3 sources, 5.14 -> 0.088 ms at 320x240x64 with 2.
+// thread per voxel, 27 samples per source and nine scatters it was bound by its atomics: 29.5 -> 0.79 ms at
+// 640x480x128 with 3 sources, 5.14 -> 0.094 ms at 320x240x64 with 2.
 constexpr int BQX = 28;                  // positions per row of a tile
 constexpr int BWARPS = 8;                // plane pairs per CTA
 constexpr int BPL = 2 * BWARPS;          // planes per CTA
@@ -352,7 +353,7 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
     __shared__ float ps[BWARPS][6 * kMaxDiffSources];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int W = A.W, H = A.H, D = A.D;
-    const int x0 = blockIdx.x * BQX - 1, y0 = blockIdx.y * R - 1, d0 = blockIdx.z * BPL;   // first position q
+    const int x0 = blockIdx.x * BQX - 1, y0 = blockIdx.z * R - 1, d0 = blockIdx.y * BPL;   // first position q
     const int x = x0 - 2 + lane;
 
     for (int e = tid; e < PX * PY * (BPL / 4); e += 32 * BWARPS) {
@@ -543,12 +544,14 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
 }
 
 // 16 rows per tile halve the share of the two-row rings against 8; images whose grid of 16-row tiles does not
-// give every SM several CTAs take 8 rows.
+// give every SM several CTAs take 8 rows.  A row of tiles takes all its planes before the next row, so that the rows
+// of the quads that it samples and scatters into stay in the caches: 847 -> 788 us at 640x480x128 with 3 sources against
+// the planes outermost.
 cudaError_t launch_cost_bwd(const CostBwdArgs& A, cudaStream_t s) {
     const int gx = (A.W + 2 + BQX - 1) / BQX, gz = A.D / BPL;
     const long tall = (long)gx * ((A.H + 2 + 15) / 16) * gz;
-    if (tall >= 148 * 6) cost_bwd_kernel<16><<<dim3(gx, (A.H + 2 + 15) / 16, gz), 32 * BWARPS, 0, s>>>(A);
-    else cost_bwd_kernel<8><<<dim3(gx, (A.H + 2 + 7) / 8, gz), 32 * BWARPS, 0, s>>>(A);
+    if (tall >= 148 * 6) cost_bwd_kernel<16><<<dim3(gx, gz, (A.H + 2 + 15) / 16), 32 * BWARPS, 0, s>>>(A);
+    else cost_bwd_kernel<8><<<dim3(gx, gz, (A.H + 2 + 7) / 8), 32 * BWARPS, 0, s>>>(A);
     return cudaGetLastError();
 }
 
