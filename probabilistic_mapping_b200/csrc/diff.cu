@@ -222,10 +222,12 @@ struct SoftArgs {
 
 // The sum of the volumes, the soft-argmin over it, the loss's terms and its adjoint, one warp per pixel.  The
 // paths are added in their order, so that the loss's signs do not depend on the layout of the volumes.  Bound by
-// memory: NV reads and a write per voxel (0.27 ms at 640x480x128 with 7 volumes: 4.7 TB/s).  The loss is summed in double
-// precision per warp, block and grid.
+// memory: NV reads and a write per voxel (0.20 ms at 640x480x128 with 7 volumes: 6.2 TB/s).  Six blocks per SM where
+// the volumes' planes leave the registers for it, and several waves of them: 268 -> 201 us against four that the
+// compiler's choice let in and a grid of six per SM, 320x240x64 with 3 volumes 31.9 -> 25.1.  The loss is summed in
+// double precision per warp, block and grid.
 template <int PPL, int NV>
-__global__ void __launch_bounds__(256) soft_kernel(const SoftArgs a) {
+__global__ void __launch_bounds__(256, PPL <= 4 ? 6 : 1) soft_kernel(const SoftArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long nw = (long)gridDim.x * 8;
     double loss = 0.0;
@@ -568,7 +570,7 @@ template <int PPL> cudaError_t launch_adj_t(const AdjArgs& a, unsigned mask, cud
     return cudaGetLastError();
 }
 template <int PPL> cudaError_t launch_soft_t(const SoftArgs& a, int nv, cudaStream_t s) {
-    const int blocks = std::min((a.N + 7) / 8, 148 * 6);
+    const int blocks = std::min((a.N + 7) / 8, 148 * 16);
     if (nv == 7) soft_kernel<PPL, 7><<<blocks, 256, 0, s>>>(a);
     else soft_kernel<PPL, 3><<<blocks, 256, 0, s>>>(a);
     return cudaGetLastError();
