@@ -807,8 +807,10 @@ def main():
     sgm_alg_gbs = b_sgm_alg / ((sgm_ms + fuse_ms) / 1000.0) / 1e9 if sgm_ms > 0 else None
     map_s = 1.0 / (value / world)   # seconds per map per GPU
     # to_float (reference) + one conversion per source, cost (+ the FP16 volume's rebase), one
-    # kernel per opposite-path pair, combine + winner-take-all, fusion transform + update
-    launches_per_map = 1 + S + 1 + (1 if e == 2 else 0) + PATHS // 2 + 1 + 2
+    # kernel for the opposite-path pairs (one per pair in the serial schedule), combine + winner-take-all,
+    # fusion transform + update
+    pair_launches = PATHS // 2 if tuning and tuning[1] else 1
+    launches_per_map = 1 + S + 1 + (1 if e == 2 else 0) + pair_launches + 1 + 2
     mixed = None
     if args.form == "batched" and not args.no_mixed:
         best_m, res_m, t_plain_m, _, _, _ = mixed_measure(args, rank, world)
@@ -850,7 +852,7 @@ def main():
                                                   else "cost_kernel_fp16" if e == 2 else None)),
             # the SGM stage against the bytes this implementation moves, and the SGM + winner-take-
             # all + fusion stages against their share of the path-grouped lower bound B_alg
-            "roofline_sgm": {"bound": "hbm", "kernel": "sgm_pair_kernel x 4 + combine_kernel (winner-take-all)",
+            "roofline_sgm": {"bound": "hbm", "kernel": "sgm_pair_kernel (4 path pairs) + combine_group_kernel (winner-take-all)",
                              "achieved": sgm_gbs, "peak": peak_hbm, "unit": "GB/s",
                              "frac": (sgm_gbs / peak_hbm) if sgm_gbs else None,
                              "implementation_bytes_per_map": sgm_bytes, "ms": sgm_ms, "peak_kind": peak_kind,
