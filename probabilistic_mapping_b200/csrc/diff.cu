@@ -329,8 +329,8 @@ struct CostBwdArgs {
 //   * the pose terms stay in registers over a tile's rows, then one double atomic per CTA and component.
 // The samples repeat the cost kernel's operations (homography FMAs, reciprocal, exact bilinear), so that
 // the signs are the forward's.  Bound by issue (about 100 instructions per sample and plane pair); with one
-// thread per voxel, 27 samples per source and nine scatters it was bound by its atomics: 29.5 -> 0.79 ms at
-// 640x480x128 with 3 sources, 5.14 -> 0.094 ms at 320x240x64 with 2.
+// thread per voxel, 27 samples per source and nine scatters it was bound by its atomics: 29.5 -> 0.81 ms at
+// 640x480x128 with 3 sources, 5.14 -> 0.096 ms at 320x240x64 with 2.
 constexpr int BQX = 28;                  // positions per row of a tile
 constexpr int BWARPS = 8;                // plane pairs per CTA
 constexpr int BPL = 2 * BWARPS;          // planes per CTA
@@ -342,8 +342,9 @@ struct Pending {
     float l, r;
 };
 
-__device__ __forceinline__ void red_add(float* p, float v) {
-    if (v != 0.0f) atomicAdd(p, v);
+// Adds v to element idx + k of an image of npix pixels: the address p + idx, which a sample's two taps share, plus k.
+__device__ __forceinline__ void red_add(float* p, unsigned idx, unsigned k, [[maybe_unused]] long long npix, float v) {
+    if (v != 0.0f && PM_IN_BOUNDS((long long)idx + k, npix, kSiteDiffGrad)) atomicAdd(p + idx + k, v);
 }
 
 template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(const CostBwdArgs A) {
@@ -450,15 +451,17 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
     __syncwarp();
 
     const bool in_q = lane >= 2 && lane < 2 + BQX;
+    const float fW1 = (float)(W - 1), fH1 = (float)(H - 1);
     const float rfx = 1.0f / A.fx, rfy = 1.0f / A.fy;
     for (int s = 0; s < A.S; ++s) {
         const float4* const quads = A.quads + s * quad_stride((size_t)W * H);
         float* const gi = A.gI + (size_t)s * W * H;
         float gp[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         Pending pend[2] = {{0u, 0.0f, 0.0f}, {0u, 0.0f, 0.0f}};
-        auto flush = [&](Pending& q) {
-            red_add(gi + q.idx, q.l);
-            red_add(gi + q.idx + 1, q.r);
+        const long long npix = (long long)W * H;
+        auto flush = [&](const Pending& q) {
+            red_add(gi, q.idx, 0, npix, q.l);
+            red_add(gi, q.idx, 1, npix, q.r);
         };
         float2 ha = make_float2(0.0f, 0.0f), hb = ha;   // row sums of the two rows above
         for (int r = 0; r < PY; ++r) {
@@ -499,9 +502,11 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
                 const float c = diff > 0.0f ? -bj : diff < 0.0f ? bj : 0.0f;
                 if (c == 0.0f) continue;
                 const float a1 = 1.0f - a, b1 = 1.0f - b;
-                // taps; the right and lower ones are 0 on the image's last column and row, where a or b is 0
-                const float ct = c * b1, cb = c * b;
-                float tl = ct * a1, tr = ct * a;
+                // taps; the image's last column has no right ones and its last row no lower ones (a or b is 0 there,
+                // but their product with an infinite or NaN adjoint is not)
+                const bool right = uj < fW1, lower = vj < fH1;
+                const float ct = c * b1, cb = lower ? c * b : 0.0f;
+                float tl = ct * a1, tr = right ? ct * a : 0.0f;
                 Pending& q = pend[j];
                 if (q.idx == idx) {
                     tl += q.l;
@@ -509,11 +514,11 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
                 } else {
                     flush(q);
                 }
-                red_add(gi + idx, tl);
-                red_add(gi + idx + 1, tr);
+                red_add(gi, idx, 0, npix, tl);
+                red_add(gi, idx, 1, npix, tr);
                 q.idx = idx + (unsigned)W;
                 q.l = cb * a1;
-                q.r = cb * a;
+                q.r = right ? cb * a : 0.0f;
                 // pose: P = w (U, V, 1); dP = omega x P + rho upsilon; g = dL/dP * w
                 const float dIdu = __fmaf_rn(b, dx1, b1 * dx0);
                 const float dIdv = __fmaf_rn(a, t.w - t.z, a1 * (t.y - t.x));
