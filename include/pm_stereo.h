@@ -338,7 +338,9 @@ PM_API pm_status pm_diff_forward(pm_diff* d, const float* ref, const float* srcs
  * grad_pose (host, 6 per source: omega then upsilon). */
 PM_API pm_status pm_diff_backward(pm_diff* d, float* grad_srcs, double* grad_pose, void* stream);
 /* The same without waiting for the stream: loss (one double) and grad_pose are device memory, written when
- * `stream` gets there. */
+ * `stream` gets there.  All calls on a handle run in their order, also when their streams differ (captured ones in
+ * the order in which their graph is launched); the buffers of a call must stay valid until `stream` has passed it, and
+ * ref until it has passed the backward, which reads it again. */
 PM_API pm_status pm_diff_forward_async(pm_diff* d, const float* ref, const float* srcs, const double K[9],
                                        const double* R, const double* t, const float* rho_gt, float* rho_hat,
                                        double* loss, void* stream);

@@ -619,6 +619,7 @@ struct pm_diff {
     float hom[kMaxSources][12]{};
     float cam[4]{};
     bool have_forward = false;
+    cudaEvent_t done = nullptr;   // the last call's work: the next one waits for it, on whichever stream
     size_t bytes = 0;
     std::string err;
 };
@@ -649,7 +650,33 @@ struct DGuard {
     }
 };
 
+// Orders a call's launches after those of the calls before it, which share the workspaces but not necessarily the
+// stream; under capture as nodes of the graph, so that the order holds where it is replayed.
+class InOrder {
+    pm_diff* d;
+    cudaStream_t st;
+    bool capturing = false, ended = false;
+
+public:
+    InOrder(pm_diff* d_, cudaStream_t st_) : d(d_), st(st_) {}
+    cudaError_t begin() {
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+        const cudaError_t e = cudaStreamIsCapturing(st, &c);
+        if (e != cudaSuccess) return e;
+        capturing = c == cudaStreamCaptureStatusActive;
+        return cudaStreamWaitEvent(st, d->done, capturing ? cudaEventWaitExternal : cudaEventWaitDefault);
+    }
+    cudaError_t end() {
+        ended = true;
+        return cudaEventRecordWithFlags(d->done, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault);
+    }
+    ~InOrder() {   // a call that failed on the way
+        if (!ended && end() != cudaSuccess) cudaGetLastError();
+    }
+};
+
 void free_diff(pm_diff* d) {
+    if (d->done) cudaEventDestroy(d->done);
     cudaFree(d->quads);
     cudaFree(d->C);
     cudaFree(d->invalid);
@@ -713,6 +740,7 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     alloc((void**)&d->codes, 8 * d->N * 4 * words);
     alloc((void**)&d->sums, 3 * sizeof(double));
     alloc((void**)&d->gP, 6 * sizeof(double) * c->num_sources);
+    ok = ok && cudaEventCreateWithFlags(&d->done, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         free_diff(d);
@@ -747,6 +775,8 @@ static pm_status run_forward(pm_diff* d, const float* ref, const float* srcs, co
     const pm_diff_config& c = d->cfg;
     const int S = c.num_sources, W = c.width, H = c.height, D = c.num_planes;
     if (!finite_n(R, 9 * S) || !finite_n(t, 3 * S)) return dfail(d, PM_ERR_INVALID_ARGUMENT, "poses must be finite");
+    InOrder order(d, st);
+    PD_CK(d, order.begin());
     d->ref = ref;
     // H1 = K R K^-1, H2 = K t for each source-from-reference pose
     const double Ki[9] = {1.0 / K[0], 0.0, -K[2] / K[0], 0.0, 1.0 / K[4], -K[5] / K[4], 0.0, 0.0, 1.0};
@@ -826,6 +856,7 @@ static pm_status run_forward(pm_diff* d, const float* ref, const float* srcs, co
     sa.drho = c.rho_step;
     sa.T = c.temperature;
     PD_CK(d, launch_soft(sa, d->wide ? 7 : 3, st));
+    PD_CK(d, order.end());
     d->have_forward = true;
     return PM_OK;
 }
@@ -834,6 +865,8 @@ static pm_status run_forward(pm_diff* d, const float* ref, const float* srcs, co
 static pm_status run_backward(pm_diff* d, float* grad_srcs, double* grad_pose, cudaStream_t st) {
     if (!d || !grad_srcs || !grad_pose) return PM_ERR_INVALID_ARGUMENT;
     if (!d->have_forward) return dfail(d, PM_ERR_BAD_STATE, "backward before forward");
+    InOrder order(d, st);
+    PD_CK(d, order.begin());
     const pm_diff_config& c = d->cfg;
     const int S = c.num_sources, D = c.num_planes;
     AdjArgs aa;
@@ -878,6 +911,7 @@ static pm_status run_backward(pm_diff* d, float* grad_srcs, double* grad_pose, c
     A.gI = grad_srcs;
     A.gP = grad_pose;
     PD_CK(d, launch_cost_bwd(A, st));
+    PD_CK(d, order.end());
     return PM_OK;
 }
 

@@ -84,11 +84,13 @@ class DepthLossEngine:
         k, kp = _dp(K)
         r, rp = _dp(R)
         tt, tp = _dp(t)
-        stream = torch.cuda.current_stream().cuda_stream
+        stream = torch.cuda.current_stream()
+        for x in (ref, srcs, rho_gt):   # it may not have read them yet when they are let go of
+            x.record_stream(stream)
         self._check(entry(self.h, ctypes.c_void_p(ref.data_ptr()), ctypes.c_void_p(srcs.data_ptr()), kp, rp, tp,
                           ctypes.c_void_p(rho_gt.data_ptr()), ctypes.c_void_p(rho_hat.data_ptr()), loss,
-                          ctypes.c_void_p(stream)), "pm_diff_forward")
-        self._keep = (ref, srcs, rho_gt)   # the backward reads them
+                          ctypes.c_void_p(stream.cuda_stream)), "pm_diff_forward")
+        self._keep = (ref, srcs, rho_gt)   # the backward reads ref; a captured forward reads all
         return rho_hat
 
     def forward(self, ref, srcs, K, R, t, rho_gt):
@@ -123,9 +125,11 @@ class DepthLossEngine:
         import torch
         g = torch.empty((self.S, self.H, self.W), dtype=torch.float32, device="cuda")
         gp = torch.empty((self.S, 6), dtype=torch.float64, device="cuda")
-        stream = torch.cuda.current_stream().cuda_stream
+        stream = torch.cuda.current_stream()
+        if self._keep:
+            self._keep[0].record_stream(stream)   # ref, which the backward reads
         self._check(self.lib.pm_diff_backward_async(self.h, ctypes.c_void_p(g.data_ptr()), ctypes.c_void_p(gp.data_ptr()),
-                                                    ctypes.c_void_p(stream)), "pm_diff_backward")
+                                                    ctypes.c_void_p(stream.cuda_stream)), "pm_diff_backward")
         return g, gp
 
 
