@@ -156,7 +156,7 @@ def _autograd_function():
         @staticmethod
         def backward(ctx, grad):
             g_src, g_pose = ctx.engine.backward_async()
-            gs = g_src.mul_(grad.to(g_src.device, g_src.dtype))
+            gs = g_src * grad.to(g_src.device, g_src.dtype)   # not in place: grad may be a batch (is_grads_batched)
             gp = g_pose.to(ctx.xi_device, ctx.xi_dtype) * grad.to(ctx.xi_device, ctx.xi_dtype)
             return gs, gp, None, None, None, None, None, None
 
