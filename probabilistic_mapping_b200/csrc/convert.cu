@@ -43,17 +43,19 @@ __global__ void __launch_bounds__(256) to_quad_kernel(int W, int H, const uint8_
     }
 }
 
-// Float images (blockIdx.z: the image), each quad slot closed by its quad of NaN.
+// Float images (blockIdx.z: the image), each quad slot closed by its quad of NaN.  Rows in strides of the grid: an
+// image may have more of them than a grid.
 __global__ void __launch_bounds__(256) to_quad_f_kernel(int W, int H, const float* __restrict__ src, float4* __restrict__ dst) {
-    const int y = blockIdx.y;
     const size_t npix = (size_t)W * H;
-    const float* r0 = src + blockIdx.z * npix + (size_t)y * W;
     float4* const q = dst + blockIdx.z * quad_stride(npix);
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < W; x += gridDim.x * blockDim.x) {
-        const bool hx = x + 1 < W, hy = y + 1 < H;
-        q[(size_t)y * W + x] = make_float4(r0[x], hy ? r0[x + W] : 0.0f, hx ? r0[x + 1] : 0.0f, (hx && hy) ? r0[x + W + 1] : 0.0f);
+    for (int y = blockIdx.y; y < H; y += gridDim.y) {
+        const float* r0 = src + blockIdx.z * npix + (size_t)y * W;
+        for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < W; x += gridDim.x * blockDim.x) {
+            const bool hx = x + 1 < W, hy = y + 1 < H;
+            q[(size_t)y * W + x] = make_float4(r0[x], hy ? r0[x + W] : 0.0f, hx ? r0[x + 1] : 0.0f, (hx && hy) ? r0[x + W + 1] : 0.0f);
+        }
     }
-    if (y == 0 && blockIdx.x == 0 && threadIdx.x == 0) q[npix] = make_float4(nan_f(), nan_f(), nan_f(), nan_f());
+    if (blockIdx.y == 0 && blockIdx.x == 0 && threadIdx.x == 0) q[npix] = make_float4(nan_f(), nan_f(), nan_f(), nan_f());
 }
 
 __global__ void __launch_bounds__(256) to_half_kernel(int W, int H, const uint8_t* __restrict__ src, size_t pitch,
@@ -128,7 +130,7 @@ cudaError_t launch_to_quad(int W, int H, const uint8_t* src, size_t src_pitch, f
 }
 
 cudaError_t launch_to_quad_f(int W, int H, int nsrc, const float* src, float4* dst, cudaStream_t s) {
-    const dim3 grid((W + 255) / 256, H, nsrc);
+    const dim3 grid((W + 255) / 256, H < 65535 ? H : 65535, nsrc);
     to_quad_f_kernel<<<grid, 256, 0, s>>>(W, H, src, dst);
     return cudaGetLastError();
 }
