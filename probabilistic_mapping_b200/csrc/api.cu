@@ -324,6 +324,14 @@ size_t out_pitch(const pm_mapper* h, size_t pitch) {
     return pitch == 0 ? row : pitch < row ? 0 : pitch;
 }
 
+// Whether two W x H float maps with these byte pitches share memory (or lie between each other's rows): written by one
+// kernel, what they share would have no order.
+bool maps_meet(const pm_mapper* h, const float* a, size_t pitch_a, const float* b, size_t pitch_b) {
+    const uintptr_t pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
+    const size_t row = sizeof(float) * (size_t)h->cfg.width, rows = (size_t)h->cfg.height - 1;
+    return pa < pb + rows * pitch_b + row && pb < pa + rows * pitch_a + row;
+}
+
 // direct: the winner-take-all depth also goes there, with a byte pitch (optional).
 pm_status run_sgm_filter(pm_mapper* h, float* direct = nullptr, size_t direct_pitch = 0) {
     const pm_config& c = h->cfg;
@@ -656,11 +664,13 @@ pm_status pm_output_fusion(pm_mapper* h, float* depth, size_t depth_pitch, float
     if (st == PM_OK) st = run_sgm_filter(h);
     mark_done(h, 1);
     if (st != PM_OK) return st;
-    // what the update kernel writes for the caller itself (not the zeros of the first keyframe)
+    // what the update kernel writes for the caller itself (not the zeros of the first keyframe, and not two maps in the
+    // same memory, where the variance is copied after the depth)
     FuseOut out{};
     out.depth_pitch = out_pitch(h, depth_pitch);
     out.variance_pitch = out_pitch(h, var_pitch);
-    if (!h->first_fusion && out.depth_pitch && (!variance || out.variance_pitch)) {
+    if (!h->first_fusion && out.depth_pitch && (!variance || out.variance_pitch) &&
+        !(variance && maps_meet(h, depth, out.depth_pitch, variance, out.variance_pitch))) {
         if (kernels_can_write(h, depth, out.depth_pitch)) out.depth = depth;
         if (variance && kernels_can_write(h, variance, out.variance_pitch)) out.variance = variance;
     }
