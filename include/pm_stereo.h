@@ -237,6 +237,9 @@ PM_API pm_status pm_debug_check_arith(uint64_t out[4], void* stream);
  * index and extent of the first one.  Synchronises the device; reset = 1 clears the record.
  * The product library returns PM_ERR_UNSUPPORTED (and zeros). */
 PM_API pm_status pm_debug_bounds(uint64_t out[4], int reset);
+/* The same library's sites: bit s of out[0] is set where site s has made a test since the last
+ * reset, bit s of out[1] where the library has a site s. */
+PM_API pm_status pm_debug_bounds_sites(uint64_t out[2], int reset);
 PM_API const char* pm_last_error(const pm_mapper* h);
 PM_API const char* pm_status_string(pm_status s);
 

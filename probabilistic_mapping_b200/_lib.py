@@ -106,6 +106,7 @@ SIGNATURES = {
     "pm_synchronize": (_I, [_VP]),
     "pm_debug_check_arith": (_I, [_P(ctypes.c_uint64), _VP]),
     "pm_debug_bounds": (_I, [_P(ctypes.c_uint64), _I]),
+    "pm_debug_bounds_sites": (_I, [_P(ctypes.c_uint64), _I]),
     "pm_last_error": (ctypes.c_char_p, [_VP]),
     "pm_status_string": (ctypes.c_char_p, [_I]),
     "pm_stage_to_float": (_I, [_I, _I, _VP, _SZ, _VP, _F, _VP]),

@@ -142,7 +142,9 @@ __device__ __forceinline__ float2 sample2_core(const Src<SAMP>& src, const WarpC
             const unsigned dx0 = in0 && __float_as_uint(tu.x) < lastx ? 1u : 0u, dx1 = in1 && __float_as_uint(tu.y) < lastx ? 1u : 0u;
             const unsigned dy0 = in0 && __float_as_uint(tv.x) < lasty ? (unsigned)src.W : 0u;
             const unsigned dy1 = in1 && __float_as_uint(tv.y) < lasty ? (unsigned)src.W : 0u;
-            auto at = [&](unsigned i) { return __ldg(reinterpret_cast<const float*>(src.base + (size_t)i * 4)); };
+            auto at = [&](unsigned i) {
+                return PM_IN_BOUNDS(i - src.off, nq, kSiteCostTap) ? __ldg(reinterpret_cast<const float*>(src.base + (size_t)i * 4)) : 0.0f;
+            };
             lo0 = f2(at(i0), at(i0 + dy0)); hi0 = f2(at(i0 + dx0), at(i0 + dy0 + dx0));
             lo1 = f2(at(i1), at(i1 + dy1)); hi1 = f2(at(i1 + dx1), at(i1 + dy1 + dx1));
         } else {

@@ -12,6 +12,7 @@ namespace pm {
 
 #ifdef PM_BOUNDS_CHECK
 __device__ unsigned long long g_bounds_log[4];
+__device__ unsigned g_bounds_seen[kBoundsSites];
 __device__ bool bounds_fail(int site, long long idx, long long n) {
     if (atomicAdd(&g_bounds_log[0], 1ull) == 0) {
         g_bounds_log[1] = (unsigned long long)site;
@@ -105,5 +106,25 @@ extern "C" pm_status pm_debug_bounds(uint64_t out[4], int reset) {
     (void)reset;
     for (int k = 0; k < 4; ++k) out[k] = 0;
     return PM_ERR_UNSUPPORTED;   // the product library has no checks
+#endif
+}
+
+extern "C" pm_status pm_debug_bounds_sites(uint64_t out[2], int reset) {
+    if (!out) return PM_ERR_INVALID_ARGUMENT;
+    out[0] = out[1] = 0;
+#ifdef PM_BOUNDS_CHECK
+    unsigned seen[pm::kBoundsSites] = {};
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpyFromSymbol(seen, pm::g_bounds_seen, sizeof seen) != cudaSuccess)
+        return PM_ERR_CUDA;
+    for (int s = 1; s < pm::kBoundsSites; ++s) {
+        out[0] |= (uint64_t)(seen[s] ? 1 : 0) << s;
+        out[1] |= (uint64_t)1 << s;
+        seen[s] = 0;
+    }
+    if (reset && cudaMemcpyToSymbol(pm::g_bounds_seen, seen, sizeof seen) != cudaSuccess) return PM_ERR_CUDA;
+    return PM_OK;
+#else
+    (void)reset;
+    return PM_ERR_UNSUPPORTED;
 #endif
 }

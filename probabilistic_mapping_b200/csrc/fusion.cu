@@ -191,7 +191,7 @@ __device__ __forceinline__ int2 update_pixel(const FuseLaunch& a, const FuseView
     a.depth[e] = out_d;
     const float var = write_all || !(a.variance || a.out.variance) ? cs : v.cur[3][e];
     if (a.variance) a.variance[e] = var;
-    fuse_out(a.out, x, y, out_d, var);
+    fuse_out(a.out, a.W, a.H, x, y, out_d, var);
     return make_int2(t == 0 ? 0 : direct ? 1 : 2, ucls);
 }
 

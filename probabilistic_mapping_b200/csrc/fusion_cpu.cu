@@ -181,7 +181,7 @@ __device__ __forceinline__ int3 cpu_update_pixel(const FuseCpuLaunch& a, int x, 
     if ((double)res < 0.1) res = 0.0f;
     a.result[i] = res;
     if (a.variance) a.variance[i] = cs;
-    fuse_out(a.out, x, y, res, cs);
+    fuse_out(a.out, a.W, a.H, x, y, res, cs);
     return make_int3(t == 0 ? 0 : 1, t != 0 && !direct ? 2 : -1, 3 + ucls);
 }
 

@@ -21,14 +21,17 @@ constexpr unsigned kFull = 0xffffffffu;
 // that every kernel shares one record).  In it each checked global access first tests its element
 // index against the buffer's extent; a failing index is not accessed.  Every failure is counted,
 // and the first failure's site (BoundsSite), index and extent are kept (pm_debug_bounds), so a
-// wrong index shows up as a record instead of a fault.  In the product library the test is the
-// constant true and compiles away.
+// wrong index shows up as a record instead of a fault; the sites that made a test are kept too
+// (pm_debug_bounds_sites).  In the product library the test is the constant true and compiles away.
 #ifdef PM_BOUNDS_CHECK
 extern __device__ unsigned long long g_bounds_log[4];   // failures, first site, its index, its extent
+extern __device__ unsigned g_bounds_seen[kBoundsSites];  // 1: the site has been reached
 __device__ bool bounds_fail(int site, long long idx, long long n);
-#define PM_IN_BOUNDS(idx, n, site)                                                        \
-    (((unsigned long long)(long long)(idx) < (unsigned long long)(long long)(n)) ||       \
-     ::pm::bounds_fail((site), (long long)(idx), (long long)(n)))
+__device__ __forceinline__ bool bounds_test(int site, long long idx, long long n) {
+    if (!g_bounds_seen[site]) g_bounds_seen[site] = 1u;
+    return (unsigned long long)idx < (unsigned long long)n || bounds_fail(site, idx, n);
+}
+#define PM_IN_BOUNDS(idx, n, site) ::pm::bounds_test((site), (long long)(idx), (long long)(n))
 #else
 #define PM_IN_BOUNDS(idx, n, site) true
 #endif
@@ -57,9 +60,10 @@ __device__ __forceinline__ void tally_block(unsigned* g, int c0, int c1 = -1, in
 __device__ __forceinline__ float& pitched(float* p, size_t pitch, int x, int y) {
     return reinterpret_cast<float*>(reinterpret_cast<char*>(p) + (size_t)y * pitch)[x];
 }
-__device__ __forceinline__ void fuse_out(const FuseOut& o, int x, int y, float depth, float variance) {
-    if (o.depth) pitched(o.depth, o.depth_pitch, x, y) = depth;
-    if (o.variance) pitched(o.variance, o.variance_pitch, x, y) = variance;
+__device__ __forceinline__ void fuse_out(const FuseOut& o, int W, int H, int x, int y, float depth, float variance) {
+    auto inside = [&]() { return PM_IN_BOUNDS(x, W, kSiteFuseOut) && PM_IN_BOUNDS(y, H, kSiteFuseOut); };
+    if (o.depth && inside()) pitched(o.depth, o.depth_pitch, x, y) = depth;
+    if (o.variance && inside()) pitched(o.variance, o.variance_pitch, x, y) = variance;
 }
 
 // Homography of one source frame as kernel arguments (the 12 floats of ad_calc_cost,

@@ -40,7 +40,12 @@ enum BoundsSite {
     kSiteCpuGather,        // CPU-variant fusion: a neighbour or predecessor cell
     kSiteClassCount,       // pm_stats class counting
     kSiteDiffRoute,        // differentiation form: a step's record, plane index or invalid flag
-    kSiteDiffGrad,         // differentiation form: a voxel of an adjoint volume or a source quad
+    kSiteDiffGrad,         // differentiation form: a voxel of an adjoint volume, a source quad or a tap's gradient
+    kSiteCostTap,          // cost kernel: a tap of a float image
+    kSiteCombineSum,       // four-pixel combine: the sum's slice
+    kSiteDepthOut,         // combine kernel: the depth in a caller's map
+    kSiteFuseOut,          // fusion: the depth or variance in a caller's map
+    kBoundsSites
 };
 
 // ---- plane-sweep cost volume (calc_cost.cu) ----------------------------------------------

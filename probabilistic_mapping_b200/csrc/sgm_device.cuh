@@ -703,6 +703,12 @@ __device__ __forceinline__ void sgm_pair_block(const SgmLaunch& a, int dx, int d
     cp_async_wait<0>();
 }
 
+// The depth of pixel (x, y) in the caller's map.
+__device__ __forceinline__ void depth_out(const SgmLaunch& a, int x, int y, float depth) {
+    if (PM_IN_BOUNDS(x, a.W, kSiteDepthOut) && PM_IN_BOUNDS(y, a.H, kSiteDepthOut))
+        pitched(a.depth2, a.depth2_pitch, x, y) = depth;
+}
+
 // Sum of the NP pair volumes (each P_2p + P_2p+1) in the order (P0 + P1) + (P2 + P3)
 // [+ ((P4 + P5) + (P6 + P7))], then the winner-take-all filter (MODE kCombineFilter), the debug
 // argmin (kCombineArgmin) or only a store of the sum (kCombineStore).  One warp per pixel: the
@@ -808,7 +814,7 @@ __device__ __forceinline__ void combine_pixels(const SgmLaunch& a, long first, l
                 *dp = depth;
                 if (a.depth2) {
                     const unsigned up = (unsigned)pix, uw = (unsigned)a.W, y = up / uw;
-                    pitched(a.depth2, a.depth2_pitch, (int)(up - y * uw), (int)y) = depth;
+                    depth_out(a, (int)(up - y * uw), (int)y, depth);
                 }
                 if (a.index) a.index[pix] = idx;
                 if (a.wta_class) a.wta_class[pix] = (uint8_t)cls;
@@ -948,7 +954,8 @@ __device__ __forceinline__ void combine_groups(const SgmLaunch& a, const void* c
         if (a.total && live)
 #pragma unroll
             for (int c = 0; c < NV; c += 4)
-                *reinterpret_cast<float4*>(a.total + (size_t)pix * D + plane(c)) = make_float4(s[c], s[c + 1], s[c + 2], s[c + 3]);
+                if (PM_RANGE_IN_BOUNDS(pix * D + plane(c), 4, (long long)npix * D, kSiteCombineSum))
+                    *reinterpret_cast<float4*>(a.total + (size_t)pix * D + plane(c)) = make_float4(s[c], s[c + 1], s[c + 2], s[c + 3]);
 
         float depth;
         int idx, cls = kWtaDepth;
@@ -1029,7 +1036,7 @@ __device__ __forceinline__ void combine_groups(const SgmLaunch& a, const void* c
             *dp = depth;
             if (a.depth2) {
                 const unsigned up = (unsigned)pix, uw = (unsigned)a.W, y = up / uw;
-                pitched(a.depth2, a.depth2_pitch, (int)(up - y * uw), (int)y) = depth;
+                depth_out(a, (int)(up - y * uw), (int)y, depth);
             }
             if (a.index) a.index[pix] = idx;
             if (a.wta_class) a.wta_class[pix] = (uint8_t)cls;
