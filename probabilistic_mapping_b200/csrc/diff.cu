@@ -557,7 +557,7 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
 cudaError_t launch_cost_bwd(const CostBwdArgs& A, cudaStream_t s) {
     const int gx = (A.W + 2 + BQX - 1) / BQX, gz = A.D / BPL;
     const long tall = (long)gx * ((A.H + 2 + 15) / 16) * gz;
-    if (tall >= 148 * 6) cost_bwd_kernel<16><<<dim3(gx, gz, (A.H + 2 + 15) / 16), 32 * BWARPS, 0, s>>>(A);
+    if (tall >= sm_count() * 6) cost_bwd_kernel<16><<<dim3(gx, gz, (A.H + 2 + 15) / 16), 32 * BWARPS, 0, s>>>(A);
     else cost_bwd_kernel<8><<<dim3(gx, gz, (A.H + 2 + 7) / 8), 32 * BWARPS, 0, s>>>(A);
     return cudaGetLastError();
 }
@@ -575,7 +575,7 @@ template <int PPL> cudaError_t launch_adj_t(const AdjArgs& a, unsigned mask, cud
     return cudaGetLastError();
 }
 template <int PPL> cudaError_t launch_soft_t(const SoftArgs& a, int nv, cudaStream_t s) {
-    const int blocks = std::min((a.N + 7) / 8, 148 * 16);
+    const int blocks = std::min((a.N + 7) / 8, sm_count() * 16);
     if (nv == 7) soft_kernel<PPL, 7><<<blocks, 256, 0, s>>>(a);
     else soft_kernel<PPL, 3><<<blocks, 256, 0, s>>>(a);
     return cudaGetLastError();
@@ -834,7 +834,7 @@ static pm_status run_forward(pm_diff* d, const float* ref, const float* srcs, co
         for (int i = 0; i < 3; ++i) {
             if (i) {
                 float4* const v = reinterpret_cast<float4*>(d->vol);
-                fold_kernel<<<148 * 8, 256, 0, st>>>(v, v + d->V / 4, v + d->V / 2, d->V / 4);
+                fold_kernel<<<sm_count() * 8, 256, 0, st>>>(v, v + d->V / 4, v + d->V / 2, d->V / 4);
                 PD_CK(d, cudaGetLastError());
             }
             PD_CK(d, launch_fwd(g0, ro, pairs[i], st));

@@ -48,6 +48,9 @@ enum BoundsSite {
     kBoundsSites
 };
 
+// SMs of the current device, which the launch rules and grids that count blocks per SM ask for.
+int sm_count();
+
 // ---- plane-sweep cost volume (calc_cost.cu) ----------------------------------------------
 constexpr int kCostTileRows = 8;
 struct CostLaunch {

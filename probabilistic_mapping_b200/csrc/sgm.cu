@@ -37,6 +37,13 @@
 
 namespace pm {
 
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
+
 void plane_order(int D, int compat, PlaneOrder& out) {
     // Merge order of `for (i = D>>1; i > 0; i >>= 1) if (d < i && d + i < D ...)`:
     // slot d keeps its element on ties, so the winner among equal values is the first in
@@ -236,14 +243,7 @@ cudaError_t launch_pairs(const SgmLaunch& a, unsigned mask, cudaStream_t s) {
         case 8: return launch_pairs_nw<PPL, HALF, 8>(a, mask, s);
         default: break;
     }
-    return few_chains(mask, a.W, a.H) ? launch_pairs_nw<PPL, HALF, 1>(a, mask, s) : launch_pairs_nw<PPL, HALF, 4>(a, mask, s);
-}
-
-int sm_count() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
+    return few_chains(mask, a.W, a.H, sm_count()) ? launch_pairs_nw<PPL, HALF, 1>(a, mask, s) : launch_pairs_nw<PPL, HALF, 4>(a, mask, s);
 }
 
 // The four-pixel kernel over np pair volumes a.part[0 .. np) (np = 1: one volume, the sum).

@@ -51,9 +51,9 @@ inline PairSet make_pair_set(unsigned mask, int W, int H, int nw) {
     return s;
 }
 // Fewer than twelve scanlines per SM: one per block, else four neighbouring ones.
-inline bool few_chains(unsigned mask, int W, int H) {
+inline bool few_chains(unsigned mask, int W, int H, int sms) {
     const PairSet s = make_pair_set(mask, W, H, 1);
-    return s.start[s.n] < 148 * 12;
+    return s.start[s.n] < sms * 12;
 }
 // The pair of block bx; bx becomes the block's index within it.
 __device__ __forceinline__ int pair_of_block(const PairSet& s, int& bx) {
