@@ -322,7 +322,8 @@ typedef struct pm_diff_config {
     float temperature;   /* soft-argmin temperature in cost units */
     float p1, p2, tau_so, q1, q2;
     int store_paths;     /* 1: seven path volumes, all paths at once; 0: less memory, three volumes and
-                            the path pairs in three launches (same results) */
+                            the path pairs in three launches (same results; up to 2^20 voxels the seven
+                            are taken either way) */
     int device;
 } pm_diff_config;
 PM_API void pm_diff_config_default(pm_diff_config* c, int width, int height, int num_planes, int num_sources);

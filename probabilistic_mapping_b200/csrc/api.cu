@@ -916,7 +916,10 @@ pm_status pm_stage_calc_cost(const pm_config* cfg, const float* ref, const float
     // A volume that starts from initReference is free until its first tile is stored, so its first rows serve as the
     // quads of the sources: the other rows are computed from them, and then these rows from the float images.  The
     // quads take a load where four float taps and their addresses go: 640x480x64 with 5 sources 882 -> 669 us, of
-    // which the 160 rows that hold the quads take some 300 (corrected mode 402 -> 374).  Where the rest is small the two more launches cost more.
+    // which the 160 rows that hold the quads take some 300 (corrected mode 402 -> 374).  The two more launches and the
+    // split cost 10 to 18 us, so the rest has to be large (millions of voxels x sources; us from rows against quads):
+    // reference mode 2.1 42 / 52, 3.6 70 / 70, 4.5 70 / 68, 8.1 109 / 113, 8.5 105 / 97, 12 146 / 128, 164 1802 / 1206;
+    // corrected mode, half as long per voxel, 12 78 / 84, 16 115 / 115, 24 141 / 134, 164 816 / 710.
     const int rows = (H + kCostTileRows - 1) / kCostTileRows;
     if (!tex && !cnt && nsrc > 0 && (reinterpret_cast<uintptr_t>(cost) & 15) == 0) {
         const size_t quads = quad_stride(N) * nsrc, tile = (size_t)W * kCostTileRows * cfg->num_planes / 4;   // in float4

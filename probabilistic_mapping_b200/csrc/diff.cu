@@ -731,8 +731,10 @@ pm_status pm_diff_create(const pm_diff_config* c, pm_diff** out) {
     alloc((void**)&d->quads, 16 * quad_stride(d->N) * c->num_sources);
     alloc((void**)&d->C, 4 * d->V);
     alloc((void**)&d->invalid, d->N);
-    // store_paths, and volumes of up to 4 MB, whose steps are bound by the recurrences' latency: 7 volumes
-    // and all paths at once; else 3 and the pairs in three launches
+    // 7 volumes and all paths at once, or 3 and the pairs in three launches: a choice of memory.  The 7 are faster at
+    // every size (forward and backward, replayed as graphs: 0.2 M voxels 146 -> 97 us, 1.04 M 239 -> 158, 4.9 M 581 ->
+    // 405, 39 M 3042 -> 2550, 59 M 3965 -> 3517), so volumes of up to 4 MB, where they add at most 17 MB, always take
+    // them, and larger ones (4.9 M voxels: 179 MB against 101) where store_paths asks for it.
     d->wide = c->store_paths || d->V <= ((size_t)1 << 20);
     alloc((void**)&d->vol, 4 * d->V * (d->wide ? 7 : 3));
     const int ppl = c->num_planes / 32;
