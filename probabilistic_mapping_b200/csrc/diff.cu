@@ -62,7 +62,8 @@ struct AdjArgs {
 // One adjoint recurrence along a scanline: lambda = gS + mu; the planes' lambda go to the
 // predecessor's planes that the forward's minima took (the same, the lower or the upper one), and the
 // plane of the predecessor's minimum receives the lambda that took the minimum, less all of them for
-// the subtracted minimum: together the negative sum over the planes that did not take it.
+// the subtracted minimum: together the negative sum over the planes that did not take it.  A lambda that took it and
+// is not finite leaves a NaN there, as in the two sums.
 template <int PPL>
 __device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[PPL],
                                              const uint32_t (&w)[Route<PPL>::WORDS], int lane, float (&lam)[PPL]) {
@@ -75,7 +76,7 @@ __device__ __forceinline__ void adjoint_step(const float (&g)[PPL], float (&mu)[
         mu[j] = (same & bit) ? lam[j] : 0.0f;
         lo[j] = (~same & side & lower & bit) ? lam[j] : 0.0f;
         hi[j] = (~same & side & ~lower & bit) ? lam[j] : 0.0f;
-        direct += ((same | side) & bit) ? lam[j] : 0.0f;
+        direct = __fmaf_rn(lam[j], ((same | side) & bit) ? 1.0f : 0.0f, direct);   // NaN where a lam is not finite
     }
     float fromU = __shfl_down_sync(kFull, lo[0], 1);        // lane + 1's first plane -> my last
     float fromL = __shfl_up_sync(kFull, hi[PPL - 1], 1);    // lane - 1's last plane -> my first
@@ -499,7 +500,7 @@ template <int R> __global__ void __launch_bounds__(32 * BWARPS) cost_bwd_kernel(
                 const float dx0 = __fsub_rn(t.z, t.x), dx1 = __fsub_rn(t.w, t.y);
                 const float top = __fmaf_rn(a, dx0, t.x), bot = __fmaf_rn(a, dx1, t.y);
                 const float diff = __fsub_rn(ref, __fmaf_rn(b, __fsub_rn(bot, top), top));
-                const float c = diff > 0.0f ? -bj : diff < 0.0f ? bj : 0.0f;
+                const float c = diff > 0.0f ? -bj : diff < 0.0f ? bj : 0.0f * bj;   // sign 0: a NaN or infinite adjoint stays
                 if (c == 0.0f) continue;
                 const float a1 = 1.0f - a, b1 = 1.0f - b;
                 // taps; the image's last column has no right ones and its last row no lower ones (a or b is 0 there,

@@ -426,7 +426,8 @@ template <int PPL> __device__ __forceinline__ void store_route(uint32_t* p, cons
 // reference image's path gradient is below tau; a plane never measured makes the pixel invalid:
 // its cost counts as 0 (cz) and the path's output there is COST_INF = 0.  o receives the output.
 // ROUTE: rt receives the step's record; equal terms resolve to the same plane, then to a neighbour (the
-// lower one first), then to the minimum.
+// lower one first), then to the minimum; and an invalid pixel's output is the path's value, as a NaN must show in the
+// sum there too (the loss leaves the pixel out).
 template <int PPL, bool FULL, bool ROUTE = false>
 __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s, const float (&cz)[PPL], bool inv,
                                           bool q, float p1q, float p2q, int lane, float (&o)[PPL],
@@ -459,7 +460,7 @@ __device__ __forceinline__ void path_step(const SgmLaunch& a, PathState<PPL>& s,
     add_planes<PPL>(vv, cz, vv);               // C + val
     add_planes<PPL>(s.L, vv, -s.mprev);        // - minL (:98); the negation is exact
 #pragma unroll
-    for (int j = 0; j < PPL; ++j) o[j] = inv ? 0.0f : s.L[j];
+    for (int j = 0; j < PPL; ++j) o[j] = !ROUTE && inv ? 0.0f : s.L[j];
     path_exchange<PPL, FULL, ROUTE>(s, lane);
 }
 
